@@ -87,6 +87,28 @@ __device__ __forceinline__ double legendre(int l, double mu) {
     }
 }
 
+// ---- column sums of per-block partials ----------------------------------------------
+// Sum of src[0], src[stride], ..., src[(n - 1) stride] for the column of threadIdx.x, by a block
+// of SUM_COLS x SUM_ROWS threads in a fixed order; valid on the threads with threadIdx.y == 0.
+// One thread per column, a serial chain of n loads, took 7 - 30 us for the few hundred partials of
+// a reduction (and 110 us for the thousands of a Fisher shell); 16 threads per column take 2 - 4 us.
+constexpr int SUM_COLS = 32, SUM_ROWS = 16;
+__device__ __forceinline__ double block_column_sum(const double *src, int64_t stride, int n, bool live) {
+    __shared__ double part[SUM_ROWS][SUM_COLS + 1];
+    double s = 0.0;
+    if (live) {
+#pragma unroll 4
+        for (int k = threadIdx.y; k < n; k += SUM_ROWS) s += src[(int64_t)k * stride];
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+#pragma unroll
+        for (int k = 1; k < SUM_ROWS; ++k) s += part[k][threadIdx.x];
+    }
+    return s;
+}
+
 template <typename T> struct cplx;
 template <> struct cplx<float> { using type = float2; };
 template <> struct cplx<double> { using type = double2; };

@@ -387,14 +387,20 @@ static bool lanes_plan(const Grid &G, int n_rows, int nk, int n_ell, LanesLaunch
 
 __global__ void binred_finalize(const double *partials, int n_blocks, int per_row, int n_rows, double scale,
                                 double *out, int accumulate) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_rows * per_row) return;
-    int row = t / per_row, j = t - row * per_row;
-    const double *src = partials + (int64_t)row * n_blocks * per_row + j;
-    double s = 0.0;
-    for (int blk = 0; blk < n_blocks; ++blk) s += src[(int64_t)blk * per_row];
+    const int t = blockIdx.x * SUM_COLS + threadIdx.x;
+    const bool live = t < n_rows * per_row;
+    const int row = live ? t / per_row : 0, j = t - row * per_row;
+    double s = block_column_sum(partials + (int64_t)row * n_blocks * per_row + j, per_row, n_blocks, live);
+    if (threadIdx.y != 0 || !live) return;
     s *= scale;
     out[t] = accumulate ? out[t] + s : s;
+}
+
+static void launch_binred_finalize(const double *partials, int n_blocks, int per_row, int n_rows, double scale,
+                                   double *out, int accumulate, cudaStream_t s) {
+    const int total = n_rows * per_row;
+    binred_finalize<<<(total + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(partials, n_blocks, per_row,
+                                                                                          n_rows, scale, out, accumulate);
 }
 
 }  // namespace pb
@@ -491,9 +497,7 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
 #undef PB_BL_NE
 #undef PB_BL_LAUNCH
         PB_LAUNCH_CHECK("pb_bin_reduce(lanes)");
-        const int per = nk * n_ell;
-        const int total = per * n_rows;
-        binred_finalize<<<(total + 255) / 256, 256, 0, s>>>(partials, LL.gx, per, n_rows, scale, out, accumulate);
+        launch_binred_finalize(partials, LL.gx, nk * n_ell, n_rows, scale, out, accumulate, s);
         PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
         return PB_OK;
     }
@@ -526,8 +530,7 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
         }
 #undef PB_RR_LAUNCH
         PB_LAUNCH_CHECK("pb_bin_reduce(rows)");
-        const int total = per * n_rows;
-        binred_finalize<<<(total + 255) / 256, 256, 0, s>>>(partials, nb, per, n_rows, scale, out, accumulate);
+        launch_binred_finalize(partials, nb, per, n_rows, scale, out, accumulate, s);
         PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
         return PB_OK;
     }
@@ -548,9 +551,7 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
     }
 #undef PB_RED_LAUNCH
     PB_LAUNCH_CHECK("pb_bin_reduce");
-    int per_row = nk * n_ell;
-    int total = per_row * n_rows;
-    binred_finalize<<<(total + 255) / 256, 256, 0, s>>>(partials, nb, per_row, n_rows, scale, out, accumulate);
+    launch_binred_finalize(partials, nb, nk * n_ell, n_rows, scale, out, accumulate, s);
     PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
     return PB_OK;
 }
@@ -620,11 +621,11 @@ struct ShellRowOut {
 
 __global__ void shell_rows_finalize(const double *partials, int n_chunks, int n_rows, int n_cols, double scale,
                                     double *out, int64_t out_stride, ShellRowOut o) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_rows * n_cols) return;
-    int r = t / n_cols, j = t - r * n_cols;
-    double s = 0.0;
-    for (int c = 0; c < n_chunks; ++c) s += partials[((int64_t)c * n_rows + r) * n_cols + j];
+    const int t = blockIdx.x * SUM_COLS + threadIdx.x;
+    const int total = n_rows * n_cols;
+    const double s = block_column_sum(partials + t, total, n_chunks, t < total);
+    if (threadIdx.y != 0 || t >= total) return;
+    const int r = t / n_cols, j = t - r * n_cols;
     out[(int64_t)o.orow[r] * out_stride + j] = s * scale;
 }
 }  // namespace pb
@@ -679,8 +680,8 @@ extern "C" int pb_shell_rows(const pb_grid_t *g, int precision, const void *F, i
         return fail(PB_ERR_INVALID, "bad precision");
     PB_LAUNCH_CHECK("pb_shell_rows");
     int total = n_rows * n_cols;
-    shell_rows_finalize<<<(total + 255) / 256, 256, 0, s>>>(partials, (int)n_chunks, n_rows, n_cols, scale, out,
-                                                           out_stride, orow);
+    shell_rows_finalize<<<(total + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(
+        partials, (int)n_chunks, n_rows, n_cols, scale, out, out_stride, orow);
     PB_LAUNCH_CHECK("pb_shell_rows(finalize)");
     return PB_OK;
 }
@@ -811,9 +812,7 @@ extern "C" int pb_bin_reduce_noalloc(const pb_grid_t *g, int precision, int mode
                                                                              row_stride, p, partials);
     }
     PB_LAUNCH_CHECK("pb_bin_reduce_noalloc");
-    int per_row = nk * n_ell;
-    int total = per_row * n_rows;
-    binred_finalize<<<(total + 255) / 256, 256, 0, s>>>(partials, nb, per_row, n_rows, scale, out, accumulate);
+    launch_binred_finalize(partials, nb, nk * n_ell, n_rows, scale, out, accumulate, s);
     PB_LAUNCH_CHECK("pb_bin_reduce_noalloc(finalize)");
     return PB_OK;
 }

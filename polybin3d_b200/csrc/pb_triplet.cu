@@ -240,11 +240,9 @@ __global__ void __launch_bounds__(SIMT_THREADS, sizeof(T) == 4 ? 3 : 1) triplet_
 }
 
 __global__ void triplet_finalize(const double *partials, int n_parts, int n_trip, double scale, double *out) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_trip) return;
-    double s = 0.0;
-    for (int c = 0; c < n_parts; ++c) s += partials[(int64_t)c * n_trip + t];
-    out[t] = s * scale;
+    const int t = blockIdx.x * SUM_COLS + threadIdx.x;
+    const double s = block_column_sum(partials + t, n_trip, n_parts, t < n_trip);
+    if (threadIdx.y == 0 && t < n_trip) out[t] = s * scale;
 }
 
 int simt_geometry(int64_t n_vox, int n_items, int *grid_x, int *grid_y, int *group_p) {
@@ -297,7 +295,7 @@ int launch_triplet_simt(int precision, const void *A, int n_a, const void *B, in
             items_dev, n_items, gp, partials, n_trip, vec);
     }
     PB_LAUNCH_CHECK("pb_triplet_contract(simt)");
-    triplet_finalize<<<(n_trip + 255) / 256, 256, 0, s>>>(partials, gx, n_trip, scale, out);
+    triplet_finalize<<<(n_trip + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(partials, gx, n_trip, scale, out);
     PB_LAUNCH_CHECK("pb_triplet_contract(finalize)");
     return PB_OK;
 }
