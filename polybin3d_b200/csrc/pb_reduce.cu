@@ -1,6 +1,8 @@
 // k-bin x Legendre reductions over half spectra (the power-spectrum binning pass) and
 // the per-shell Fisher-row contraction.  FP64 accumulation, deterministic two-pass sums.
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 #include "pb_common.cuh"
@@ -358,6 +360,222 @@ __global__ void __launch_bounds__(256) binred_lanes_kernel(Grid g, const typenam
     }
 }
 
+// ------------------------------------------------------------------------------------
+// Few rows (a field's own spectrum): the folded reduction.
+//
+// The mode-tile kernel spends its time on the geometry (FP64 sqrt, division, bin search and
+// Legendre polynomials per mode), not on the spectrum.  Here
+//  * the four modes (+-kx, +-ky, kz) share one evaluation: their |x|^2 are summed first;
+//  * bins are found from s = |k|^2 against thresholds t_b, the smallest doubles with
+//    sqrt(t_b) >= edge_b (sqrt is monotone and correctly rounded on both sides, so membership
+//    is bit for bit that of |k|), and s grows along a lane's walk over ky, so the search is
+//    one comparison with the next threshold;
+//  * the Legendre products are polynomials in mu^2 = kz^2 / s: a lane sums f mu^(2m) and the
+//    block turns its moments into the requested products.
+// A unit is 32 consecutive kz of a kx plane (coalesced reads) times a run of ky that one warp
+// walks; each lane keeps the sums of its current bin in registers and adds them to its own slot
+// of the warp's shared-memory window [bin - first bin of the unit][moment][lane] when the bin
+// changes; the window is summed over the lanes into the warp's totals after the unit.  No
+// atomics, a fixed order.  The window holds the bins that a unit can meet (a bound from the
+// bin widths), so that 16 warps fit on an SM; with all 40 bins' slots only 6 did (483 us).
+// Measured on a B200, one FP32 spectrum of 512^3, 40 bins, l = 0, 2, 4: 222 us against 2450 us
+// for the mode-tile kernel (256^3 FP32: 42 against 310 us; 128^3 FP64: below 20 against 50 us).
+// ------------------------------------------------------------------------------------
+constexpr int FOLD_MAX_M = 5;           // mu^0 .. mu^8
+constexpr int FOLD_SMEM = 100 * 1024;   // accumulators per block, two blocks per SM
+
+struct FoldParams {
+    double t[PB_RED_MAX_BINS + 1];                  // thresholds on |k|^2
+    double coef[PB_RED_MAX_ELLS][FOLD_MAX_M];       // L_la L_lb as a polynomial in mu^2
+    int32_t nk, n_ell;
+    int32_t jseg, n_jseg, n_lchunk;                 // ky steps per unit, units per (kx, kz chunk)
+    int32_t wb;                                     // bins of a unit's window
+};
+
+template <typename T, int MODE>
+__device__ __forceinline__ double fold_value(const typename cplx<T>::type *a, const typename cplx<T>::type *b,
+                                             const T *w, int64_t idx) {
+    if (MODE == PB_RED_ABS2) {
+        const typename cplx<T>::type v = a[idx];
+        return (double)v.x * (double)v.x + (double)v.y * (double)v.y;
+    }
+    if (MODE == PB_RED_CROSS) {
+        const typename cplx<T>::type u = a[idx], v = b[idx];
+        return (double)u.x * (double)v.x + (double)u.y * (double)v.y;
+    }
+    const double v = w ? (double)w[idx] : 1.0;
+    return v * v;
+}
+
+template <typename T, int MODE, int NM>
+__global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typename cplx<T>::type *a,
+                                                            const typename cplx<T>::type *b, const T *w,
+                                                            int64_t row_stride, const __grid_constant__ FoldParams p,
+                                                            double *partials) {
+    constexpr int U = sizeof(T) == 4 ? 4 : 2;  // ky steps whose values are in flight together
+    extern __shared__ __align__(16) double fold_smem[];  // [warp][window bin][moment][32], [warp][bin][moment]
+    __shared__ double t[PB_RED_MAX_BINS + 2];
+    const int nk = p.nk, nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = nk * NM, wper = p.wb * NM;
+    double *const win = fold_smem + (size_t)warp * wper * 32;
+    double *const totals = fold_smem + (size_t)nw * wper * 32;
+    double *const tot = totals + (size_t)warp * per;
+    for (int i = threadIdx.x; i < nw * (wper * 32 + per); i += blockDim.x) fold_smem[i] = 0.0;
+    for (int i = threadIdx.x; i <= nk; i += blockDim.x) t[i] = p.t[i];
+    if (threadIdx.x == 0) t[nk + 1] = __longlong_as_double(0x7ff0000000000000LL);
+    __syncthreads();
+    const int row = blockIdx.y;
+    if (MODE == PB_RED_ABS2) a += (int64_t)row * row_stride;
+    if (MODE == PB_RED_CROSS) b += (int64_t)row * row_stride;
+    const int h0 = g.n0 >> 1, h1 = g.n1 >> 1;       // frequency f >= 0 sits at f < n / 2, f < 0 at f + n
+    const int m0 = g.n0 - h0, m1 = g.n1 - h1;       // largest |f| of each axis
+    const int64_t units = (int64_t)(m0 + 1) * p.n_lchunk * p.n_jseg;
+    const double t_lo = p.t[0], t_hi = p.t[nk];
+    for (int64_t u = (int64_t)blockIdx.x * nw + warp; u < units; u += (int64_t)gridDim.x * nw) {
+        const int js = (int)(u % p.n_jseg);
+        const int64_t r = u / p.n_jseg;
+        const int l0 = (int)(r % p.n_lchunk) * 32, l = l0 + lane, fi = (int)(r / p.n_lchunk);
+        const bool live = l < g.nh2, hp = fi < h0, hm = fi >= 1;
+        const int64_t op = (int64_t)(hp ? fi : 0) * g.n1 * g.nh2 + l, om = (int64_t)(hm ? g.n0 - fi : 0) * g.n1 * g.nh2 + l;
+        const double kx = __dmul_rn((double)fi, g.kf0), kz = __dmul_rn((double)l, g.kf2);
+        const double kx2 = __dmul_rn(kx, kx), kz2 = __dmul_rn(kz, kz);
+        const double deg = l > 0 ? 2.0 : 1.0;
+        const int jb = js * p.jseg, j1 = min(jb + p.jseg, m1 + 1);
+        // the unit's first bin: the one of its smallest |k|^2 (or the first edge still ahead)
+        int base;
+        {
+            const double ky = __dmul_rn((double)jb, g.kf1), kzb = __dmul_rn((double)l0, g.kf2);
+            const double sb = __dadd_rn(__dadd_rn(kx2, __dmul_rn(ky, ky)), __dmul_rn(kzb, kzb));
+            if (sb >= t_hi) continue;
+            base = 0;
+            while (t[base + 1] <= sb) ++base;
+        }
+        int bin = base - 1;      // current bin (base - 1: none yet); t[bin + 1] is the next threshold
+        double next = t[base], acc[NM];
+#pragma unroll
+        for (int m = 0; m < NM; ++m) acc[m] = 0.0;
+        for (int j0 = jb; j0 < j1; j0 += U) {
+            double s[U], f[U];
+            bool any = false;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int fj = j0 + q;
+                const double ky = __dmul_rn((double)fj, g.kf1);
+                s[q] = __dadd_rn(__dadd_rn(kx2, __dmul_rn(ky, ky)), kz2);
+                const bool in = live && fj < j1 && s[q] < t_hi;
+                any = any || in;
+                f[q] = 0.0;
+                if (in && s[q] >= t_lo) {
+                    // the up to four mirrored modes; the loads of the U steps are independent
+                    const int jp = fj * g.nh2, jm = (g.n1 - fj) * g.nh2;
+                    if (fj < h1) {
+                        if (hp) f[q] += fold_value<T, MODE>(a, b, w, op + jp);
+                        if (hm) f[q] += fold_value<T, MODE>(a, b, w, om + jp);
+                    }
+                    if (fj >= 1) {
+                        if (hp) f[q] += fold_value<T, MODE>(a, b, w, op + jm);
+                        if (hm) f[q] += fold_value<T, MODE>(a, b, w, om + jm);
+                    }
+                }
+            }
+            if (!__any_sync(0xffffffffu, any)) break;  // s only grows from here
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                if (s[q] >= next) {
+                    if (bin >= base) {
+#pragma unroll
+                        for (int m = 0; m < NM; ++m) win[((bin - base) * NM + m) * 32 + lane] += acc[m];
+                    }
+#pragma unroll
+                    for (int m = 0; m < NM; ++m) acc[m] = 0.0;
+                    do {
+                        ++bin;
+                        next = t[bin + 1];
+                    } while (s[q] >= next);
+                    // past the last edge, or a mode beyond the run: nothing more is added
+                    if (bin >= nk || j0 + q >= j1) {
+                        bin = base - 1;
+                        next = t[nk + 1];
+                    }
+                }
+                double x = f[q] * deg;
+                acc[0] += x;
+                if (NM > 1) {
+                    const double mu2 = s[q] > 0.0 ? kz2 / s[q] : 0.0;
+#pragma unroll
+                    for (int m = 1; m < NM; ++m) {
+                        x *= mu2;
+                        acc[m] += x;
+                    }
+                }
+            }
+        }
+        if (bin >= base) {
+#pragma unroll
+            for (int m = 0; m < NM; ++m) win[((bin - base) * NM + m) * 32 + lane] += acc[m];
+        }
+        __syncwarp();
+        // a lane sums one (bin, moment) over the 32 slots (rotated: no bank conflicts), clearing them
+        const int rows = min(p.wb, nk - base) * NM;
+        for (int q = lane; q < rows; q += 32) {
+            double x = 0.0;
+#pragma unroll 16
+            for (int k = 0; k < 32; ++k) x += win[q * 32 + ((lane + k) & 31)];
+#pragma unroll 16
+            for (int k = 0; k < 32; ++k) win[q * 32 + ((lane + k) & 31)] = 0.0;
+            tot[base * NM + q] += x;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < per; i += blockDim.x) {
+        double x = totals[i];
+        for (int k = 1; k < nw; ++k) x += totals[(size_t)k * per + i];
+        totals[i] = x;
+    }
+    __syncthreads();
+    double *dst = partials + ((int64_t)row * gridDim.x + blockIdx.x) * (p.n_ell * nk);
+    for (int i = threadIdx.x; i < p.n_ell * nk; i += blockDim.x) {
+        const int e = i / nk, bn = i - e * nk;
+        double x = 0.0;
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+            if (p.coef[e][m] != 0.0) x += p.coef[e][m] * totals[bn * NM + m];
+        dst[i] = x;
+    }
+}
+
+// smallest double t >= 0 with sqrt(t) >= e
+static double sqrt_threshold(double e) {
+    if (!(e > 0.0)) return 0.0;
+    double t = e * e;
+    while (t > 0.0 && std::sqrt(t) >= e) t = std::nextafter(t, 0.0);
+    while (std::sqrt(t) < e) t = std::nextafter(t, HUGE_VAL);
+    return t;
+}
+
+// Fills the fold parameters when the folded kernel takes this reduction: the global line of
+// sight (mu of the four mirrored modes agrees) and even Legendre products; false otherwise.
+static bool fold_plan(const Grid &G, const RedParams &r, FoldParams *p, int *n_moments) {
+    if (G.los) return false;
+    static const double leg[5][3] = {{1.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {-0.5, 1.5, 0.0}, {0.0, 0.0, 0.0},
+                                     {0.375, -3.75, 4.375}};
+    memset(p, 0, sizeof(*p));
+    int top = 0;
+    for (int e = 0; e < r.n_ell; ++e) {
+        const int la = r.la[e], lb = r.lb[e];
+        if ((la | lb) & 1) return false;
+        for (int i = 0; i <= la / 2; ++i)
+            for (int j = 0; j <= lb / 2; ++j) p->coef[e][i + j] += leg[la][i] * leg[lb][j];
+        top = std::max(top, (la + lb) / 2);
+    }
+    for (int i = 0; i <= r.nk; ++i) p->t[i] = sqrt_threshold(r.edges[i]);
+    p->nk = r.nk;
+    p->n_ell = r.n_ell;
+    *n_moments = top + 1;
+    return true;
+}
+
 struct LanesLaunch {
     int nw, gx;
     size_t smem;
@@ -401,6 +619,69 @@ static void launch_binred_finalize(const double *partials, int n_blocks, int per
     const int total = n_rows * per_row;
     binred_finalize<<<(total + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(partials, n_blocks, per_row,
                                                                                           n_rows, scale, out, accumulate);
+}
+
+template <typename T, int MODE, int NM>
+static cudaError_t fold_launch(const Grid &G, const void *a, const void *b, int n_rows, int64_t row_stride,
+                               const FoldParams &p, int nb, int nw, double *partials, cudaStream_t s) {
+    const size_t smem = (size_t)nw * (p.wb * 32 + p.nk) * NM * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(binred_fold_kernel<T, MODE, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    binred_fold_kernel<T, MODE, NM><<<dim3(nb, n_rows), 32 * nw, smem, s>>>(
+        G, (const typename cplx<T>::type *)a, (const typename cplx<T>::type *)b, (const T *)a, row_stride, p, partials);
+    return cudaSuccess;
+}
+
+// bins that an interval of |k| of length D can meet
+static int bins_within(const double *edges, int nk, double D) {
+    int most = 1;
+    for (int i = 0, j = 0; i < nk; ++i) {
+        // an interval that ends in bin j (edge j below its end) and starts in bin i
+        while (j + 1 < nk && edges[j + 1] - edges[i + 1] <= D) ++j;
+        most = std::max(most, j - i + 1);
+    }
+    return most;
+}
+
+// one folded reduction on nb blocks per row; false when its accumulators do not fit
+static bool launch_fold(const Grid &G, int precision, int mode, const void *a, const void *b, int n_rows,
+                        int64_t row_stride, const double *edges, FoldParams p, int nm, int nb, double *partials,
+                        cudaStream_t s) {
+    const int m0 = G.n0 - G.n0 / 2, m1 = G.n1 - G.n1 / 2;
+    p.n_lchunk = (G.nh2 + 31) / 32;
+    // ky steps of a unit: 32, shorter while eight warps' windows do not fit or a warp gets fewer
+    // than eight units (their work differs: 5 units of 64 steps a warp took 294 us at 512^3, 222 us now)
+    int nw = 0;
+    for (p.jseg = 32;; p.jseg /= 2) {
+        const double dy = (p.jseg + 1) * G.kf1, dz = 32 * G.kf2;
+        p.wb = std::min(p.nk, 1 + bins_within(edges, p.nk, std::sqrt(dy * dy + dz * dz)));
+        nw = (int)std::min<size_t>(8, FOLD_SMEM / ((size_t)(p.wb * 32 + p.nk) * nm * sizeof(double)));
+        const int64_t units = (int64_t)(m0 + 1) * p.n_lchunk * ((m1 + p.jseg) / p.jseg);
+        if (p.jseg == 8 || (nw == 8 && units >= (int64_t)8 * nb * nw)) break;
+    }
+    if (nw < 1) return false;
+    p.n_jseg = (m1 + p.jseg) / p.jseg;  // m1 + 1 frequencies |f| = 0 .. m1
+    cudaError_t e = cudaSuccess;
+#define PB_FOLD_M(T, MODE, M) \
+    case M: e = fold_launch<T, MODE, M>(G, a, b, n_rows, row_stride, p, nb, nw, partials, s); break;
+#define PB_FOLD(T, MODE)                                                                                          \
+    switch (nm) {                                                                                                 \
+        PB_FOLD_M(T, MODE, 1) PB_FOLD_M(T, MODE, 2) PB_FOLD_M(T, MODE, 3) PB_FOLD_M(T, MODE, 4)                    \
+        PB_FOLD_M(T, MODE, 5)                                                                                     \
+    }
+    if (precision == PB_F32) {
+        if (mode == PB_RED_ABS2) PB_FOLD(float, PB_RED_ABS2)
+        else if (mode == PB_RED_CROSS) PB_FOLD(float, PB_RED_CROSS)
+        else PB_FOLD(float, PB_RED_REAL2)
+    } else {
+        if (mode == PB_RED_ABS2) PB_FOLD(double, PB_RED_ABS2)
+        else if (mode == PB_RED_CROSS) PB_FOLD(double, PB_RED_CROSS)
+        else PB_FOLD(double, PB_RED_REAL2)
+    }
+#undef PB_FOLD
+#undef PB_FOLD_M
+    return e == cudaSuccess;
 }
 
 }  // namespace pb
@@ -504,6 +785,18 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
     if (!workspace || workspace_bytes < need)
         return fail(PB_ERR_WORKSPACE, "pb_bin_reduce: workspace too small (need " + std::to_string(need) + " bytes)");
     double *partials = (double *)workspace;
+    // the folded kernel wherever its symmetry holds: at 128^3 FP64 CROSS, l = 0, 2, 4, it takes
+    // 37 / 71 / 141 us for 4 / 8 / 15 rows against 87 / 129 / 216 us for the mode-tile kernel (from
+    // 16 rows the lane-per-row kernel above takes over)
+    FoldParams fp;
+    int nm = 0;
+    if (tuning().red_method != 2 && fold_plan(G, p, &fp, &nm) &&
+        launch_fold(G, precision, mode, a, b, n_rows, row_stride, p.edges, fp, nm, nb, partials, s)) {
+        PB_LAUNCH_CHECK("pb_bin_reduce(fold)");
+        launch_binred_finalize(partials, nb, nk * n_ell, n_rows, scale, out, accumulate, s);
+        PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
+        return PB_OK;
+    }
     if (mode != PB_RED_REAL2) {
         // spectra: mode geometry once per tile for a group of rows (binred_rows_kernel)
         const int per = nk * n_ell;
