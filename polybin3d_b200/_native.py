@@ -84,6 +84,10 @@ SIGNATURES = {
     "pb_pair_products": ([_I, _I64, _P, _P, _P, _P, _P, _I, _D, _P, _P], _I),
     "pb_shell_rows_workspace_size": ([_I64, _I, _I, ctypes.POINTER(_SZ)], _I),
     "pb_shell_rows": ([_GP, _I, _P, _I, _P, _I, _P, _I64, _P, _P, _I, _D, _P, _I64, _P, _SZ, _P], _I),
+    "pb_masked_rows_table": ([_GP, _P, ctypes.POINTER(_SZ)], _I),
+    "pb_masked_rows_workspace_size": ([_GP, _D, _I, ctypes.POINTER(_SZ)], _I),
+    "pb_masked_rows": ([_GP, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _D, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _SZ, _P],
+                       _I),
 }
 
 
@@ -564,4 +568,59 @@ class BilinearPlan:
         check(load().pb_bilinear_maps(precision_of(G.dtype), G[0].numel(), ptr(G), self.n_g, ptr(self.table),
                                       self.n_table, self.n_out, ptr(out), stream_ptr()), "pb_bilinear_maps")
         _count(1)
+        return out
+
+
+# workspace of pb_masked_rows: up to 32 maps in flight, fewer above this
+MASKED_WS_BYTES = 1 << 30
+
+
+class MaskedRows:
+    """pb_masked_rows for one mask: its non-zero rows and the transform tables, on the device.
+    Raises NotImplementedError when the grid's dimensions are not supported."""
+
+    def __init__(self, grid, mask):
+        lib = load()
+        self.grid, self.mask = grid, mask
+        nbytes = ctypes.c_size_t()
+        check(lib.pb_masked_rows_table(ctypes.byref(grid), None, ctypes.byref(nbytes)), "pb_masked_rows_table")
+        table = np.zeros(nbytes.value // 8, dtype=np.float64)
+        check(lib.pb_masked_rows_table(ctypes.byref(grid), hptr(table), ctypes.byref(nbytes)), "pb_masked_rows_table")
+        n0, n1 = int(grid.n[0]), int(grid.n[1])
+        act = (mask != 0).any(2).cpu().numpy()
+        x, y = np.nonzero(act)                       # ordered by x, then y
+        rank = (np.cumsum(act, axis=1) - 1)[x, y]    # position among the rows of the same x
+        last = rank + 1 == act.sum(1)[x]
+        first, alone = rank % 2 == 0, (rank % 2 == 0) & last
+        row = (x * n1 + y).astype(np.int32)
+        nxt, prv = np.roll(y, -1), np.roll(y, 1)
+        code = np.full((n0, n1), -1, dtype=np.int32)
+        code[x, y] = np.where(alone, 4 * y, np.where(first, 4 * nxt + 1, 4 * prv + 2))
+        pairs = np.stack([row[first], np.where(alone, -1, np.roll(row, -1))[first]], axis=1)
+        on = act.any(1)
+        dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=mask.device)
+        self.pairs, self.code, self.xs, self.x_on = dev(pairs), dev(code), dev(np.nonzero(on)[0]), dev(on)
+        self.table = torch.as_tensor(table, device=mask.device)
+
+    def run(self, src, maps, k_out, out, ws, src_stride=None):
+        """out[m] = rfftn(mask * c2r(F_m)) on |k| < k_out (other modes of out are not written);
+        maps: per output a list of (src_idx, lo, hi, ell, scale) legs, the same count for all."""
+        lib = load()
+        arr = np.asarray(maps, dtype=np.float64)
+        n_maps, n_legs = arr.shape[:2]
+        arr = arr.reshape(n_maps * n_legs, 5)
+        si, ell = (np.ascontiguousarray(arr[:, k].astype(np.int32)) for k in (0, 3))
+        lo, hi, sc = (np.ascontiguousarray(arr[:, k]) for k in (1, 2, 4))
+        one = ctypes.c_size_t()
+        check(lib.pb_masked_rows_workspace_size(ctypes.byref(self.grid), float(k_out), 1, ctypes.byref(one)),
+              "pb_masked_rows_workspace_size")
+        chunk = max(1, min(n_maps, 32, MASKED_WS_BYTES // one.value))
+        buf = ws.get(chunk * one.value, "masked")
+        stride = src_stride if src_stride is not None else (src[0].numel() if src.dim() == 4 else 0)
+        check(lib.pb_masked_rows(ctypes.byref(self.grid), ptr(src), stride, n_maps, n_legs, hptr(si), hptr(lo), hptr(hi),
+                                 hptr(ell), hptr(sc), float(k_out), ptr(self.mask), ptr(self.pairs),
+                                 self.pairs.shape[0], ptr(self.code), ptr(self.xs), self.xs.numel(), ptr(self.x_on),
+                                 ptr(self.table), ptr(out), ptr(buf), chunk * one.value, stream_ptr()),
+              "pb_masked_rows")
+        _count(5 * ((n_maps + chunk - 1) // chunk))
         return out

@@ -27,6 +27,7 @@ class Pointing:
         self.kind = kind
         self.mask = mask
         self._typed = {}
+        self._rows = False  # not looked at yet
         if kind == 'mask':
             return
         dev = base.device
@@ -47,6 +48,18 @@ class Pointing:
         self.inside = torch.as_tensor((zidx >= 0), device=dev)
         den = np.bincount(zidx[zidx >= 0], weights=mic[zidx >= 0], minlength=self.nz)
         self.den = torch.as_tensor(den, device=dev)
+
+    def rows(self):
+        """The band-limited chain c2r, mask, r2c of half spectra (nat.MaskedRows), or None: an
+        integral constraint, or a grid whose lengths it does not transform."""
+        if self._rows is False:
+            self._rows = None
+            if self.kind == 'mask':
+                try:
+                    self._rows = nat.MaskedRows(self.base.grid, self.mask)
+                except NotImplementedError:
+                    pass
+        return self._rows
 
     def _as(self, t, dtype):
         if t.dtype == dtype:

@@ -316,28 +316,42 @@ class PSpec:
                                    bm=None if bm is None else bm[i])
             return fish if theory is None else (fish, bm)
         rows = [(li, ki) for li in range(self.Nl) for ki in range(self.Nk)]
+        # trivial S^-1 and a varying mask: only the binned modes of each row are made
+        chain = None if (self._custom_sinv or xi is not None or self.const_mask) else self._pointing().rows()
+        k_out = float(max(self.k_bins[-1], theory[0][-1] if theory is not None else 0.0))
         for i in range(B):
             Q = torch.empty((self.N_bins,) + b.nhalf_shape, dtype=torch.complex128, device=b.device)
             qs = 1.0 if self._custom_sinv else (qscale if self.const_mask else invN)
-            maps = [(i, self.k_bins[ki], self.k_bins[ki + 1], 2 * li, 0, qs, 0) for (li, ki) in rows]
-            nat.spectral_filter(grid, F64, SinvP, Q, maps, src_stride=nh)
-            if self._custom_sinv:
-                for r in range(self.N_bins):
-                    Q[r] = self._dagger_custom(Q[r], False, xi)
-            elif xi is not None:
-                Q = self._cov_rows(Q, xi)
-            elif not self.const_mask:
-                qr = b.fft_c2r(Q)
+            if chain is not None:
+                chain.run(SinvP, [[(i, self.k_bins[ki], self.k_bins[ki + 1], 2 * li, qs)] for (li, ki) in rows], k_out,
+                          Q, b.ws, src_stride=nh)
                 b.n_FFTs_reverse += self.N_bins
-                self._pointing()(qr, True, out=qr)
-                Q = b.fft_r2c(qr, out=Q)
                 b.n_FFTs_forward += self.N_bins
+            else:
+                self._fisher_rows(SinvP, i, rows, qs, invN, Q, xi)
             autotune.bin_reduce(grid, F64, nat.PB_RED_CROSS, Ainv[i], Q, self.N_bins, self.k_bins,
                                 self._ells(self.Nl), scaling, fish[i], b.ws)
             if theory is not None:                                       # pspec.py:395-402
                 autotune.bin_reduce(grid, F64, nat.PB_RED_CROSS, Ainv[i], Q, self.N_bins, theory[0],
                                     self._ells(theory[1]), scaling, bm[i], b.ws)
         return fish if theory is None else (fish, bm)
+
+    def _fisher_rows(self, S, i, rows, qs, invN, Q, xi):
+        """Q <- the rows D Theta_b L_l S[i] on whole half spectra."""
+        b = self.base
+        maps = [(i, self.k_bins[ki], self.k_bins[ki + 1], 2 * li, 0, qs, 0) for (li, ki) in rows]
+        nat.spectral_filter(b.grid, nat.PB_F64, S, Q, maps, src_stride=b.nhalf)
+        if self._custom_sinv:
+            for r in range(self.N_bins):
+                Q[r] = self._dagger_custom(Q[r], False, xi)
+        elif xi is not None:
+            self._cov_rows(Q, xi)
+        elif not self.const_mask:
+            qr = b.fft_c2r(Q)
+            b.n_FFTs_reverse += self.N_bins
+            self._pointing()(qr, True, out=qr)
+            b.fft_r2c(qr, out=Q)
+            b.n_FFTs_forward += self.N_bins
 
     def _xi_grids(self, Pk_cov):
         return covariance.xi_grids(self.base, Pk_cov)
