@@ -372,6 +372,12 @@ PB_API int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_strid
                           int n_pairs, const int32_t *row_code, const int32_t *xs, int n_x,
                           const int32_t *x_on, const void *table, void *out, void *workspace,
                           size_t workspace_bytes, void *stream);
+/* out[p] = rfftn(X[i] X[j] - Z[i] Z[j]) (Z may be NULL) on the modes |k| < k_out for host (i, j)  */
+/* pairs of FP64 real maps: the products of the bispectrum's Q maps (bspec.py:579-597).  Same      */
+/* table, workspace and grid lengths as pb_masked_rows.                                           */
+PB_API int pb_product_rows(const pb_grid_t *g, const double *X, const double *Z, const int32_t *pairs,
+                           int n_pairs, double k_out, const void *table, void *out, void *workspace,
+                           size_t workspace_bytes, void *stream);
 
 #ifdef __cplusplus
 }

@@ -88,6 +88,7 @@ SIGNATURES = {
     "pb_masked_rows_workspace_size": ([_GP, _D, _I, ctypes.POINTER(_SZ)], _I),
     "pb_masked_rows": ([_GP, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _D, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _SZ, _P],
                        _I),
+    "pb_product_rows": ([_GP, _P, _P, _P, _I, _D, _P, _P, _P, _SZ, _P], _I),
 }
 
 
@@ -575,17 +576,43 @@ class BilinearPlan:
 MASKED_WS_BYTES = 1 << 30
 
 
+def transform_table(grid, device):
+    """Twiddle table of pb_masked_rows and pb_product_rows for a grid, on the device."""
+    lib = load()
+    nbytes = ctypes.c_size_t()
+    check(lib.pb_masked_rows_table(ctypes.byref(grid), None, ctypes.byref(nbytes)), "pb_masked_rows_table")
+    table = np.zeros(nbytes.value // 8, dtype=np.float64)
+    check(lib.pb_masked_rows_table(ctypes.byref(grid), hptr(table), ctypes.byref(nbytes)), "pb_masked_rows_table")
+    return torch.as_tensor(table, device=device)
+
+
+def _rows_workspace(grid, k_out, n_maps, ws):
+    """(buffer, bytes used, maps per chunk) of a chain of n_maps rows."""
+    one = ctypes.c_size_t()
+    check(load().pb_masked_rows_workspace_size(ctypes.byref(grid), float(k_out), 1, ctypes.byref(one)),
+          "pb_masked_rows_workspace_size")
+    chunk = max(1, min(n_maps, 32, MASKED_WS_BYTES // one.value))
+    return ws.get(chunk * one.value, "masked"), chunk * one.value, chunk
+
+
+def product_rows(grid, X, Z, pairs, k_out, out, table, ws):
+    """out[p] = rfftn(X[i] X[j] - Z[i] Z[j]) on |k| < k_out (other modes of out are not written);
+    X, Z: (n, n0, n1, n2) FP64 maps, Z may be None."""
+    pairs = np.ascontiguousarray(np.asarray(pairs, dtype=np.int32).reshape(-1, 2))
+    buf, nbytes, chunk = _rows_workspace(grid, k_out, len(pairs), ws)
+    check(load().pb_product_rows(ctypes.byref(grid), ptr(X), ptr(Z), hptr(pairs), len(pairs), float(k_out), ptr(table),
+                                 ptr(out), ptr(buf), nbytes, stream_ptr()), "pb_product_rows")
+    _count(3 * ((len(pairs) + chunk - 1) // chunk))
+    return out
+
+
 class MaskedRows:
     """pb_masked_rows for one mask: its non-zero rows and the transform tables, on the device.
     Raises NotImplementedError when the grid's dimensions are not supported."""
 
     def __init__(self, grid, mask):
-        lib = load()
         self.grid, self.mask = grid, mask
-        nbytes = ctypes.c_size_t()
-        check(lib.pb_masked_rows_table(ctypes.byref(grid), None, ctypes.byref(nbytes)), "pb_masked_rows_table")
-        table = np.zeros(nbytes.value // 8, dtype=np.float64)
-        check(lib.pb_masked_rows_table(ctypes.byref(grid), hptr(table), ctypes.byref(nbytes)), "pb_masked_rows_table")
+        self.table = transform_table(grid, mask.device)
         n0, n1 = int(grid.n[0]), int(grid.n[1])
         act = (mask != 0).any(2).cpu().numpy()
         x, y = np.nonzero(act)                       # ordered by x, then y
@@ -600,7 +627,6 @@ class MaskedRows:
         on = act.any(1)
         dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=mask.device)
         self.pairs, self.code, self.xs, self.x_on = dev(pairs), dev(code), dev(np.nonzero(on)[0]), dev(on)
-        self.table = torch.as_tensor(table, device=mask.device)
 
     def run(self, src, maps, k_out, out, ws, src_stride=None):
         """out[m] = rfftn(mask * c2r(F_m)) on |k| < k_out (other modes of out are not written);
@@ -611,16 +637,12 @@ class MaskedRows:
         arr = arr.reshape(n_maps * n_legs, 5)
         si, ell = (np.ascontiguousarray(arr[:, k].astype(np.int32)) for k in (0, 3))
         lo, hi, sc = (np.ascontiguousarray(arr[:, k]) for k in (1, 2, 4))
-        one = ctypes.c_size_t()
-        check(lib.pb_masked_rows_workspace_size(ctypes.byref(self.grid), float(k_out), 1, ctypes.byref(one)),
-              "pb_masked_rows_workspace_size")
-        chunk = max(1, min(n_maps, 32, MASKED_WS_BYTES // one.value))
-        buf = ws.get(chunk * one.value, "masked")
+        buf, nbytes, chunk = _rows_workspace(self.grid, k_out, n_maps, ws)
         stride = src_stride if src_stride is not None else (src[0].numel() if src.dim() == 4 else 0)
         check(lib.pb_masked_rows(ctypes.byref(self.grid), ptr(src), stride, n_maps, n_legs, hptr(si), hptr(lo), hptr(hi),
                                  hptr(ell), hptr(sc), float(k_out), ptr(self.mask), ptr(self.pairs),
                                  self.pairs.shape[0], ptr(self.code), ptr(self.xs), self.xs.numel(), ptr(self.x_on),
-                                 ptr(self.table), ptr(out), ptr(buf), chunk * one.value, stream_ptr()),
+                                 ptr(self.table), ptr(out), ptr(buf), nbytes, stream_ptr()),
               "pb_masked_rows")
         _count(5 * ((n_maps + chunk - 1) // chunk))
         return out

@@ -320,6 +320,16 @@ class PolyBin3D:
         p.exec(k, out, self.ws.get(p.ws_bytes, "fft"))
         return out
 
+    def rows_table(self):
+        """Device twiddle table of the band-limited FP64 chains on the data grid, or None when its
+        lengths are not supported."""
+        if 'rows_table' not in self._dev:
+            try:
+                self._dev['rows_table'] = nat.transform_table(self.grid, self.device)
+            except NotImplementedError:
+                self._dev['rows_table'] = None
+        return self._dev['rows_table']
+
     def to_fourier(self, _input_rmap):
         """Transform from real- to Fourier-space (numpy rfftn convention)."""
         x = self.as_device(_input_rmap) if not isinstance(_input_rmap, torch.Tensor) else _input_rmap.contiguous()

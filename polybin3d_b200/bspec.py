@@ -907,10 +907,17 @@ class BSpec:
         return G1, G2
 
     def _key_fts(self, G1, G2, keys):
-        """FT[g1_0,A g1_l,B - g2_0,A g2_l,B] for keys (A, B, l) as a batch of half spectra."""
+        """FT[g1_0,A g1_l,B - g2_0,A g2_l,B] for keys (A, B, l) as a batch of half spectra: the
+        binned modes of each (what the legs and the shells read), or whole spectra where the
+        grid's lengths have no band-limited chain."""
         b = self.base
         nks = self.Nk_squeeze
         pairs = [(A, (l // 2) * nks + B) for (A, B, l) in keys]
+        table = b.rows_table()
+        if table is not None:
+            b.n_FFTs_forward += len(keys)
+            out = torch.empty((len(keys),) + b.nhalf_shape, dtype=torch.complex128, device=b.device)
+            return nat.product_rows(b.grid, G1, G2, pairs, float(self.k_bins_squeeze[-1]), out, table, b.ws)
         prods = nat.pair_products(G1, G1, pairs, Z=G2, U=G2)
         b.n_FFTs_forward += len(keys)
         return b.fft_r2c(prods)
@@ -968,14 +975,23 @@ class BSpec:
         del G1, G2
         qs = 1.0 if self._custom_sinv else (invN if not self.const_mask else (1.0 if xi is not None else self.mask_mean))
         Q = torch.empty((self.N_bins,) + b.nhalf_shape, dtype=torch.complex128, device=b.device)
+        # trivial S^-1 and a varying mask: the legs, the mask and both transforms as one chain on the
+        # binned modes
+        chain = None if (self._custom_sinv or xi is not None or self.const_mask or local) else self._pointing().rows()
         # leg b3 carries L_l; with the local sightline that leg is applied in real space below
         leg1 = [(kpos[(r[0], r[1], 0)], ks[r[2]], ks[r[2] + 1], 0 if local else r[3], 0,
                  0.0 if (local and r[3] > 0) else qs, 0) for r in ab.tolist()]
         leg2 = [(kpos[(r[1], r[2], r[3])], ks[r[0]], ks[r[0] + 1], 0, 0, qs, 0) for r in ab.tolist()]
         leg3 = [(kpos[(r[0], r[2], r[3])], ks[r[1]], ks[r[1] + 1], 0, 0, qs, 0) for r in ab.tolist()]
-        nat.spectral_filter(b.grid, F64, FT, Q, leg1, src_stride=nh)
-        nat.spectral_filter(b.grid, F64, FT, Q, leg2, src_stride=nh, accumulate=True)
-        nat.spectral_filter(b.grid, F64, FT, Q, leg3, src_stride=nh, accumulate=True)
+        if chain is not None:
+            chain.run(FT, [[(x[0], x[1], x[2], x[3], x[5]) for x in row] for row in zip(leg1, leg2, leg3)],
+                      float(ks[-1]), Q, b.ws, src_stride=nh)
+            b.n_FFTs_reverse += self.N_bins
+            b.n_FFTs_forward += self.N_bins
+        else:
+            nat.spectral_filter(b.grid, F64, FT, Q, leg1, src_stride=nh)
+            nat.spectral_filter(b.grid, F64, FT, Q, leg2, src_stride=nh, accumulate=True)
+            nat.spectral_filter(b.grid, F64, FT, Q, leg3, src_stride=nh, accumulate=True)
         if local:
             # Q += FT[sum_m Y_lm(x) IFT(Y_lm(k) Theta_b3 FT_AB0)] for the rows of multipole l
             # (bspec.py:621-631), batched over the rows
@@ -999,7 +1015,8 @@ class BSpec:
                 idx = torch.as_tensor(rows, device=b.device)
                 Q[idx] = Q[idx] + b.fft_r2c(acc) * qs
         del FT
-        Q = self._filter_rows(Q, xi, mask_shot)
+        if chain is None:
+            Q = self._filter_rows(Q, xi, mask_shot)
         # --- rows from Q[S^-1 P a] (compute_Q 'Sinv', bspec.py:528-597)
         if self._custom_sinv:
             ws = torch.stack([a1.reshape(b.nhalf_shape), a2.reshape(b.nhalf_shape)]).to(torch.complex128)

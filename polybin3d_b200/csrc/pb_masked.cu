@@ -193,7 +193,12 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_x_kernel(const __grid_consta
 
 // ---- Y: inverse (SIGN 1) and forward (SIGN -1) transforms along y, in place ---------------
 // row_code[x n1 + y]: -1 the mask is zero on the row; partner_y * 4 + kind otherwise (kind 0: alone, 1 / 2:
-// first / second row of a packed pair)
+// first / second row of a packed pair).  NULL: every row, (y, y + 1) packed for even y; xs NULL: every x
+__device__ __forceinline__ int code_of(const int32_t *code, int y, int n1) {
+    if (code) return code[y];
+    const int o = y ^ 1;
+    return o >= n1 ? 4 * y : 4 * o + 1 + (y & 1);
+}
 template <int SIGN>
 __global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_constant__ MrParams p, const double2 *table,
                                                             const int32_t *xs, const int32_t *row_code, double2 *W) {
@@ -201,14 +206,15 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_consta
     const Grid &g = p.g;
     const MrMap &mp = p.maps[blockIdx.y];
     const int L = blockDim.x, runs = p.kz_out / L + 1;
-    const int run = blockIdx.x % runs, x = xs[blockIdx.x / runs], kz0 = run * L;
+    const int run = blockIdx.x % runs, xi = blockIdx.x / runs, x = xs ? xs[xi] : xi,
+              kz0 = run * L;
     const int kz_max = SIGN > 0 ? mp.kz_max : p.kz_out;
     if (kz0 > kz_max) return;
     double2 *tw = mr_smem, *sm = tw + p.ay.tw_len, *sm2 = sm + p.ay.n * L;
     load_table(tw, table + p.tw_y, p.ay.tw_len);
     const int line = threadIdx.x, kz = kz0 + line;
     const bool on = kz <= kz_max;
-    const int32_t *code = row_code + (int64_t)x * g.n1;
+    const int32_t *code = row_code ? row_code + (int64_t)x * g.n1 : nullptr;
     double2 *w = W + blockIdx.y * p.w_map + (int64_t)x * g.n1 * p.ldz + kz;
     const int ry = ky_radius(g, SIGN > 0 ? mp.hi2 : p.out2, kz), row = p.ldz * (int)sizeof(double2);
     auto at = [&](int e) { return e * L + line; };
@@ -218,13 +224,13 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_consta
             p.ay, threadIdx.y, blockDim.y, on, sm, sm2, tw, at,
             [&](int e) { return abs(freq_index(e, g.n1)) <= ry ? elem(w, e, row) : zero; },
             [&](int y, double2 v) {
-                if (code[y] >= 0) elem(w, y, row) = v;
+                if (code_of(code, y, g.n1) >= 0) elem(w, y, row) = v;
             });
     } else {
         fft::line_fft<double, -1>(
             p.ay, threadIdx.y, blockDim.y, on, sm, sm2, tw, at,
             [&](int y) {
-                const int c = code[y];
+                const int c = code_of(code, y, g.n1);
                 if (c < 0) return zero;
                 const double2 a = elem(w, y, row);
                 if ((c & 3) == 0) return a;
@@ -340,6 +346,48 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     if (on) fft::line_pass<double, -1, 2>(af, t, nt, twf, [&](int e) { return sm2[atf(e)]; }, stf);
 }
 
+// ---- products: forward transform along z of X_i X_j - Z_i Z_j, two rows per complex line ----------
+// block (threads per line, L pairs of rows); grid (products, row pairs / L): the products of a few
+// rows follow each other, so the maps' rows come from L2 after the first
+struct MrPairs {
+    int16_t i[MR_MAX_MAPS], j[MR_MAX_MAPS];
+};
+__global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_constant__ MrParams p,
+                                                                  const __grid_constant__ MrPairs pr,
+                                                                  const double2 *table, const double *X, const double *Z,
+                                                                  double2 *W) {
+    extern __shared__ __align__(16) double2 mr_smem[];
+    const Grid &g = p.g;
+    const Axis &ax = p.azi;
+    const int L = blockDim.y, n = ax.n, ld = fft::row_len(ax);
+    double2 *tw = mr_smem, *sm = tw + ax.tw_len + threadIdx.y * ld, *sm2 = sm + L * ld;
+    load_table(tw, table + p.tw_zi, ax.tw_len);
+    const int half = (g.n1 + 1) / 2, q = blockIdx.y * L + threadIdx.y;
+    const bool on = q < g.n0 * half;
+    const int x = on ? q / half : 0, y = on ? 2 * (q - x * half) : 0;
+    const bool two = y + 1 < g.n1;
+    const int64_t ra = (int64_t)x * g.n1 + y, oi = pr.i[blockIdx.x] * g.nreal, oj = pr.j[blockIdx.x] * g.nreal;
+    const double *xi = X + oi + ra * n, *xj = X + oj + ra * n;
+    const double *zi = Z ? Z + oi + ra * n : nullptr, *zj = Z ? Z + oj + ra * n : nullptr;
+    double2 *wa = W + blockIdx.x * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
+    fft::line_fft<double, -1>(
+        ax, threadIdx.x, blockDim.x, on, sm, sm2, tw, [&](int e) { return fft::row_at(ax, e); },
+        [&](int e) {
+            double2 v = make_double2(xi[e] * xj[e], 0.0);
+            if (Z) v.x -= zi[e] * zj[e];
+            if (two) {
+                v.y = xi[e + n] * xj[e + n];
+                if (Z) v.y -= zi[e + n] * zj[e + n];
+            }
+            return v;
+        },
+        [&](int e, double2 v) {
+            if (e <= p.kz_out) wa[e] = v;
+            const int kz = e == 0 ? 0 : n - e;
+            if (two && kz <= p.kz_out) wb[kz] = v;
+        });
+}
+
 // ---- X': forward transform along x ---------------------------------------------------------
 __global__ void __launch_bounds__(MR_THREADS, 2) mr_out_kernel(const __grid_constant__ MrParams p, const double2 *table,
                                                               const int32_t *x_on, const double2 *W, double2 *out) {
@@ -359,7 +407,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_out_kernel(const __grid_cons
     const int rx = index_radius(p.out2, (ky * g.kf1) * (ky * g.kf1) + (kz * g.kf2) * (kz * g.kf2), g.kf0);
     fft::line_fft<double, -1>(
         p.ax, threadIdx.y, blockDim.y, on, sm, sm2, tw, [&](int e) { return e * L + line; },
-        [&](int x) { return x_on[x] ? elem(w, x, wx) : make_double2(0.0, 0.0); },
+        [&](int x) { return !x_on || x_on[x] ? elem(w, x, wx) : make_double2(0.0, 0.0); },
         [&](int e, double2 v) {
             if (abs(freq_index(e, g.n0)) <= rx) elem(o, e, ox) = v;
         });
@@ -397,6 +445,49 @@ static void line_shape(const Axis &ax, int *L, int *nt, size_t *smem) {
     while (*L > 2 && bytes(*L) > (size_t)MR_SMEM) *L /= 2;
     *nt = std::max(1, std::min(ax.nb[ax.np - 1], MR_THREADS / *L));
     *smem = bytes(*L);
+}
+
+struct MrShapes {
+    int Lx, Tx, Ly, Ty, Lz, Tz;   // lines per block and threads per line of each axis
+    size_t sx, sy, sz;
+};
+
+// everything of MrParams that the grid and k_out fix, and the launch shapes
+static int mr_setup(const Grid &G, double k_out, MrParams *pp, MrShapes *sh) {
+    MrLayout lay;
+    const int st = mr_layout(G, &lay);
+    if (st) return st;
+    MrParams &p = *pp;
+    memset(&p, 0, sizeof(p));
+    p.g = G;
+    p.ldz = mr_row_stride(G, k_out);
+    p.kz_out = std::min(G.nh2 - 1, (int)std::floor(k_out / G.kf2));
+    p.out2 = k_out * k_out * (1.0 + 1e-12);
+    p.w_map = (int64_t)G.n0 * G.n1 * p.ldz;
+    p.ax = lay.ax;
+    p.ay = lay.ay;
+    p.azi = lay.azi;
+    p.azf = lay.azf;
+    p.tw_x = lay.tw_x;
+    p.tw_y = lay.tw_y;
+    p.tw_zi = lay.tw_zi;
+    p.tw_zf = lay.tw_zf;
+    line_shape(p.ax, &sh->Lx, &sh->Tx, &sh->sx);
+    line_shape(p.ay, &sh->Ly, &sh->Ty, &sh->sy);
+    // z: one butterfly of the last inverse pass per thread, pairs of rows up to 128 threads
+    const int Tz = p.azi.nb[p.azi.np - 1];
+    const int ldr = std::max(fft::row_len(p.azi), fft::row_len(p.azf));
+    auto zbytes = [&](int l) {
+        return ((size_t)p.azi.tw_len + p.azf.tw_len + (size_t)(p.azi.np == 3 ? 2 : 1) * l * ldr) * sizeof(double2);
+    };
+    int Lz = std::max(1, 128 / Tz);
+    while (Lz > 1 && zbytes(Lz) > (size_t)MR_SMEM) Lz /= 2;
+    sh->Lz = Lz;
+    sh->Tz = Tz;
+    sh->sz = zbytes(Lz);
+    if (Tz * Lz > MR_THREADS || std::max(sh->sz, std::max(sh->sx, sh->sy)) > (size_t)MR_SMEM)
+        return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: lines too long");
+    return PB_OK;
 }
 
 static double threshold_sq(double e) {  // smallest t with sqrt(t) >= e
@@ -455,56 +546,28 @@ extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_s
         return fail(PB_ERR_INVALID, "pb_masked_rows: NULL argument");
     if (n_maps < 1 || n_legs < 1 || n_legs > MR_MAX_LEGS || n_pairs < 1 || n_x < 1 || n_x > G.n0 || !(k_out > 0.0))
         return fail(PB_ERR_INVALID, "pb_masked_rows: bad sizes");
-    MrLayout lay;
-    st = mr_layout(G, &lay);
-    if (st) return st;
     MrParams p;
-    memset(&p, 0, sizeof(p));
-    p.g = G;
+    MrShapes sh;
+    st = mr_setup(G, k_out, &p, &sh);
+    if (st) return st;
     p.n_legs = n_legs;
-    p.ldz = mr_row_stride(G, k_out);
-    p.kz_out = std::min(G.nh2 - 1, (int)std::floor(k_out / G.kf2));
-    p.out2 = k_out * k_out * (1.0 + 1e-12);
     p.src_stride = src_stride;
-    p.w_map = (int64_t)G.n0 * G.n1 * p.ldz;
     p.n_x = n_x;
     p.n_pairs = n_pairs;
-    p.ax = lay.ax;
-    p.ay = lay.ay;
-    p.azi = lay.azi;
-    p.azf = lay.azf;
-    p.tw_x = lay.tw_x;
-    p.tw_y = lay.tw_y;
-    p.tw_zi = lay.tw_zi;
-    p.tw_zf = lay.tw_zf;
     for (int i = 0; i < n_maps * n_legs; ++i) {
         if (ell[i] != 0 && ell[i] != 2 && ell[i] != 4) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: even Legendre orders up to 4");
         if (ell[i] != 0 && G.los) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: Legendre weights need the global line of sight");
         if (src_idx[i] < 0) return fail(PB_ERR_INVALID, "pb_masked_rows: negative source index");
         if (!(hi[i] > 0.0) || hi[i] > k_out) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: upper edges must lie in (0, k_out]");
     }
-    int Lx, Tx, Ly, Ty;
-    size_t sx, sy;
-    line_shape(p.ax, &Lx, &Tx, &sx);
-    line_shape(p.ay, &Ly, &Ty, &sy);
-    // z: one butterfly of the last inverse pass per thread; pairs of rows per block to 128 - 256 threads
-    const int Tz = p.azi.nb[p.azi.np - 1];
-    const int ldr = std::max(fft::row_len(p.azi), fft::row_len(p.azf));
-    auto zbytes = [&](int l) {
-        return ((size_t)p.azi.tw_len + p.azf.tw_len + (size_t)(p.azi.np == 3 ? 2 : 1) * l * ldr) * sizeof(double2);
-    };
-    int Lz = std::max(1, 128 / Tz);
-    while (Lz > 1 && zbytes(Lz) > (size_t)MR_SMEM) Lz /= 2;
-    if (Tz * Lz > MR_THREADS || zbytes(Lz) > (size_t)MR_SMEM || sx > (size_t)MR_SMEM || sy > (size_t)MR_SMEM)
-        return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: lines too long");
     const size_t per = (size_t)p.w_map * sizeof(double2);
     const int chunk = (int)std::min<size_t>(MR_MAX_MAPS, workspace_bytes / per);
     if (!workspace || chunk < 1) return fail(PB_ERR_WORKSPACE, "pb_masked_rows: workspace too small");
-    PB_CUDA(cudaFuncSetAttribute(mr_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx));
-    PB_CUDA(cudaFuncSetAttribute(mr_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx));
-    PB_CUDA(cudaFuncSetAttribute(mr_y_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy));
-    PB_CUDA(cudaFuncSetAttribute(mr_y_kernel<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy));
-    PB_CUDA(cudaFuncSetAttribute(mr_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zbytes(Lz)));
+    PB_CUDA(cudaFuncSetAttribute(mr_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sx));
+    PB_CUDA(cudaFuncSetAttribute(mr_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sx));
+    PB_CUDA(cudaFuncSetAttribute(mr_y_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sy));
+    PB_CUDA(cudaFuncSetAttribute(mr_y_kernel<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sy));
+    PB_CUDA(cudaFuncSetAttribute(mr_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sz));
     cudaStream_t s = as_stream(stream);
     double2 *W = (double2 *)workspace;
     const double2 *tab = (const double2 *)table;
@@ -523,17 +586,61 @@ extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_s
             mp.lo2 = low * low;
             mp.kz_max = std::min(p.kz_out, (int)std::floor(top / G.kf2));
         }
-        const int runs_x = p.kz_out / Lx + 1, runs_y = p.kz_out / Ly + 1;
-        mr_x_kernel<<<dim3(G.n1 * runs_x, nm), dim3(Lx, Tx), sx, s>>>(p, (const double2 *)src, tab, W);
+        const int runs_x = p.kz_out / sh.Lx + 1, runs_y = p.kz_out / sh.Ly + 1;
+        mr_x_kernel<<<dim3(G.n1 * runs_x, nm), dim3(sh.Lx, sh.Tx), sh.sx, s>>>(p, (const double2 *)src, tab, W);
         PB_LAUNCH_CHECK("pb_masked_rows(x)");
-        mr_y_kernel<1><<<dim3(n_x * runs_y, nm), dim3(Ly, Ty), sy, s>>>(p, tab, xs, row_code, W);
+        mr_y_kernel<1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, row_code, W);
         PB_LAUNCH_CHECK("pb_masked_rows(y)");
-        mr_z_kernel<<<dim3((n_pairs + Lz - 1) / Lz, nm), dim3(Tz, Lz), zbytes(Lz), s>>>(p, tab, pairs, mask, W);
+        mr_z_kernel<<<dim3((n_pairs + sh.Lz - 1) / sh.Lz, nm), dim3(sh.Tz, sh.Lz), sh.sz, s>>>(p, tab, pairs, mask, W);
         PB_LAUNCH_CHECK("pb_masked_rows(z)");
-        mr_y_kernel<-1><<<dim3(n_x * runs_y, nm), dim3(Ly, Ty), sy, s>>>(p, tab, xs, row_code, W);
+        mr_y_kernel<-1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, row_code, W);
         PB_LAUNCH_CHECK("pb_masked_rows(y')");
-        mr_out_kernel<<<dim3(G.n1 * runs_x, nm), dim3(Lx, Tx), sx, s>>>(p, tab, x_on, W, (double2 *)out + (int64_t)m0 * G.nhalf);
+        mr_out_kernel<<<dim3(G.n1 * runs_x, nm), dim3(sh.Lx, sh.Tx), sh.sx, s>>>(p, tab, x_on, W,
+                                                                                 (double2 *)out + (int64_t)m0 * G.nhalf);
         PB_LAUNCH_CHECK("pb_masked_rows(x')");
+    }
+    return PB_OK;
+}
+
+extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double *Z, const int32_t *pairs, int n_pairs,
+                               double k_out, const void *table, void *out, void *workspace, size_t workspace_bytes,
+                               void *stream) {
+    Grid G;
+    int st = make_grid(g, &G);
+    if (st) return st;
+    if (!X || !pairs || !table || !out) return fail(PB_ERR_INVALID, "pb_product_rows: NULL argument");
+    if (n_pairs < 1 || !(k_out > 0.0)) return fail(PB_ERR_INVALID, "pb_product_rows: bad sizes");
+    for (int k = 0; k < 2 * n_pairs; ++k)
+        if (pairs[k] < 0 || pairs[k] > 32767) return fail(PB_ERR_INVALID, "pb_product_rows: map index out of range");
+    MrParams p;
+    MrShapes sh;
+    st = mr_setup(G, k_out, &p, &sh);
+    if (st) return st;
+    const size_t per = (size_t)p.w_map * sizeof(double2);
+    const int chunk = (int)std::min<size_t>(MR_MAX_MAPS, workspace_bytes / per);
+    if (!workspace || chunk < 1) return fail(PB_ERR_WORKSPACE, "pb_product_rows: workspace too small");
+    PB_CUDA(cudaFuncSetAttribute(mr_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sz));
+    PB_CUDA(cudaFuncSetAttribute(mr_y_kernel<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sy));
+    PB_CUDA(cudaFuncSetAttribute(mr_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.sx));
+    cudaStream_t s = as_stream(stream);
+    double2 *W = (double2 *)workspace;
+    const double2 *tab = (const double2 *)table;
+    const int rows = G.n0 * ((G.n1 + 1) / 2);
+    for (int m0 = 0; m0 < n_pairs; m0 += chunk) {
+        const int nm = std::min(chunk, n_pairs - m0);
+        MrPairs pr;
+        for (int m = 0; m < nm; ++m) {
+            pr.i[m] = (int16_t)pairs[2 * (m0 + m)];
+            pr.j[m] = (int16_t)pairs[2 * (m0 + m) + 1];
+        }
+        mr_product_kernel<<<dim3(nm, (rows + sh.Lz - 1) / sh.Lz), dim3(sh.Tz, sh.Lz), sh.sz, s>>>(p, pr, tab, X, Z, W);
+        PB_LAUNCH_CHECK("pb_product_rows(z)");
+        mr_y_kernel<-1><<<dim3(G.n0 * (p.kz_out / sh.Ly + 1), nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, nullptr,
+                                                                                                  nullptr, W);
+        PB_LAUNCH_CHECK("pb_product_rows(y)");
+        mr_out_kernel<<<dim3(G.n1 * (p.kz_out / sh.Lx + 1), nm), dim3(sh.Lx, sh.Tx), sh.sx, s>>>(
+            p, tab, nullptr, W, (double2 *)out + (int64_t)m0 * G.nhalf);
+        PB_LAUNCH_CHECK("pb_product_rows(x)");
     }
     return PB_OK;
 }

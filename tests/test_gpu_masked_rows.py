@@ -87,3 +87,25 @@ def test_unsupported_length():
     from polybin3d_b200 import _native as nat
     with pytest.raises(NotImplementedError):
         nat.MaskedRows(grid_of((34, 32, 32), (1.0, 1.0, 1.0)), torch.ones(34, 32, 32, device="cuda", dtype=torch.float64))
+
+
+@pytest.mark.parametrize("with_z", [True, False])
+@pytest.mark.parametrize("n,kf", [((16, 12, 10), (1.0, 1.0, 1.0)), ((27, 35, 22), (1.0, 0.8, 1.2)),
+                                  ((20, 13, 512), (1.0, 1.0, 0.05)), ((64, 9, 26), (1.0, 1.0, 1.0))])
+def test_product_rows(n, kf, with_z):
+    from polybin3d_b200 import _native as nat
+    rng = np.random.default_rng(5)
+    dev = torch.device("cuda")
+    X, Z = (torch.as_tensor(rng.standard_normal((4,) + n), device=dev) for _ in range(2))
+    pairs = [(int(i), int(j)) for i, j in rng.integers(0, 4, (37, 2))]
+    grid = grid_of(n, kf)
+    k, _ = modes(n, kf)
+    k_out = 0.97 * min(np.asarray(n) // 2 * np.asarray(kf))
+    want = torch.stack([torch.fft.rfftn(X[i] * X[j] - (Z[i] * Z[j] if with_z else 0)) for i, j in pairs])
+    out = torch.full_like(want, float("nan"))
+    nat.product_rows(grid, X, Z if with_z else None, pairs, k_out, out, nat.transform_table(grid, dev),
+                     nat.Workspace(dev))
+    sel = torch.as_tensor(k < k_out, device=dev)
+    got, want = out[:, sel], want[:, sel]
+    tol = 10 * np.finfo(np.float64).eps * np.log2(np.prod(n)) * float(want.abs().max())
+    assert bool(torch.isfinite(torch.view_as_real(got)).all()) and float((got - want).abs().max()) <= tol
