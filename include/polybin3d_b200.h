@@ -354,11 +354,11 @@ PB_API int pb_bin_reduce_noalloc(const pb_grid_t *g, int precision, int mode, co
 /* (PolyBin3D/pspec.py:443-456, bspec.py:600-640) as one band-limited chain.  Modes of     */
 /* out with |k| >= k_out are not written.  Parameter arrays: host, [n_maps][n_legs],       */
 /* n_legs <= 3; hi <= k_out; ell in {0, 2, 4}, ell > 0 for the z line of sight only.        */
-/* mask: device FP64 (n0, n1, n2).  Its non-zero rows r = x n1 + y, device int32:           */
-/*   pairs    [n_pairs][2]: every non-zero row once, two of the same x, or (r, -1);         */
-/*   row_code [n0 n1]: -1 for a zero row, else 4 partner_y + kind (kind 0 alone, 1 / 2        */
-/*            first / second of its pair);                                                */
-/*   xs       [n_x]: the planes x that hold a non-zero row; x_on [n0]: 1 for those, else 0. */
+/* mask: device FP64 (n0, n1, n2).  Rows (x, y) go in pairs (y even, y + 1; the last alone when   */
+/* n1 is odd); the pairs on which the mask is not zero, on the device:                            */
+/*   pairs   int32 [n_pairs]: x n1 + y of their first rows;                                       */
+/*   pair_on uint8 [n0 ceil(n1 / 2)]: 1 for those, else 0;                                        */
+/*   xs      int32 [n_x]: the planes x that hold one; x_on int32 [n0]: 1 for those, else 0.          */
 /* table: pb_masked_rows_table, copied to the device.  workspace: any multiple of            */
 /* workspace_size(.., 1), up to 32 maps; maps go through it in chunks.  The grid            */
 /* dimensions must be products of at most three factors up to 16 (of 2, 3, 5, 7, 11, 13):   */
@@ -369,7 +369,7 @@ PB_API int pb_masked_rows_workspace_size(const pb_grid_t *g, double k_out, int n
 PB_API int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_stride, int n_maps, int n_legs,
                           const int32_t *src_idx, const double *lo, const double *hi, const int32_t *ell,
                           const double *scale, double k_out, const double *mask, const int32_t *pairs,
-                          int n_pairs, const int32_t *row_code, const int32_t *xs, int n_x,
+                          int n_pairs, const uint8_t *pair_on, const int32_t *xs, int n_x,
                           const int32_t *x_on, const void *table, void *out, void *workspace,
                           size_t workspace_bytes, void *stream);
 /* out[p] = rfftn(X[i] X[j] - Z[i] Z[j]) (Z may be NULL) on the modes |k| < k_out for host (i, j)  */

@@ -613,20 +613,14 @@ class MaskedRows:
     def __init__(self, grid, mask):
         self.grid, self.mask = grid, mask
         self.table = transform_table(grid, mask.device)
-        n0, n1 = int(grid.n[0]), int(grid.n[1])
-        act = (mask != 0).any(2).cpu().numpy()
-        x, y = np.nonzero(act)                       # ordered by x, then y
-        rank = (np.cumsum(act, axis=1) - 1)[x, y]    # position among the rows of the same x
-        last = rank + 1 == act.sum(1)[x]
-        first, alone = rank % 2 == 0, (rank % 2 == 0) & last
-        row = (x * n1 + y).astype(np.int32)
-        nxt, prv = np.roll(y, -1), np.roll(y, 1)
-        code = np.full((n0, n1), -1, dtype=np.int32)
-        code[x, y] = np.where(alone, 4 * y, np.where(first, 4 * nxt + 1, 4 * prv + 2))
-        pairs = np.stack([row[first], np.where(alone, -1, np.roll(row, -1))[first]], axis=1)
+        n1 = int(grid.n[1])
+        act = (mask != 0).any(2)
+        act = torch.nn.functional.pad(act, (0, n1 % 2)).reshape(act.shape[0], -1, 2).any(2)   # by pair of rows
+        x, pair = torch.nonzero(act, as_tuple=True)
         on = act.any(1)
-        dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=mask.device)
-        self.pairs, self.code, self.xs, self.x_on = dev(pairs), dev(code), dev(np.nonzero(on)[0]), dev(on)
+        self.pairs = (x * n1 + 2 * pair).to(torch.int32)
+        self.pair_on = act.to(torch.uint8).contiguous()
+        self.xs, self.x_on = torch.nonzero(on)[:, 0].to(torch.int32), on.to(torch.int32)
 
     def run(self, src, maps, k_out, out, ws, src_stride=None):
         """out[m] = rfftn(mask * c2r(F_m)) on |k| < k_out (other modes of out are not written);
@@ -641,7 +635,7 @@ class MaskedRows:
         stride = src_stride if src_stride is not None else (src[0].numel() if src.dim() == 4 else 0)
         check(lib.pb_masked_rows(ctypes.byref(self.grid), ptr(src), stride, n_maps, n_legs, hptr(si), hptr(lo), hptr(hi),
                                  hptr(ell), hptr(sc), float(k_out), ptr(self.mask), ptr(self.pairs),
-                                 self.pairs.shape[0], ptr(self.code), ptr(self.xs), self.xs.numel(), ptr(self.x_on),
+                                 self.pairs.numel(), ptr(self.pair_on), ptr(self.xs), self.xs.numel(), ptr(self.x_on),
                                  ptr(self.table), ptr(out), ptr(buf), nbytes, stream_ptr()),
               "pb_masked_rows")
         _count(5 * ((n_maps + chunk - 1) // chunk))

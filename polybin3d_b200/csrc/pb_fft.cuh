@@ -202,11 +202,16 @@ __device__ __forceinline__ int div_r0(const Axis &ax, int e) { return (int)(((ui
 __device__ __forceinline__ int row_at(const Axis &ax, int e) { return ax.pad ? e + div_r0(ax, e) : e; }
 __host__ __device__ __forceinline__ int row_len(const Axis &ax) { return ax.pad ? ax.n + ax.n / ax.R[0] : ax.n; }
 
-// One pass of the lines of a block.  ld(e) gives element e (already in registers' reach), st(e, v)
-// takes it; `t` of `nt` threads share the line.  FIRST: no twiddles.
-template <typename T, int SIGN, int Q, typename LD, typename ST>
+// functor of line_pass that leaves the loaded elements as they are
+struct Keep {
+    template <typename C> __device__ __forceinline__ C operator()(int, C v) const { return v; }
+};
+
+// One pass (number Q) of the lines of a block.  ld(e) gives element e, fix(e, v) finishes it once all of
+// a butterfly's loads are on their way, st(e, v) takes a result; `t` of `nt` threads share the line.
+template <typename T, int SIGN, int Q, typename LD, typename ST, typename FX = Keep>
 __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const typename cplx<T>::type *tw, LD &&ld,
-                                          ST &&st) {
+                                          ST &&st, FX &&fix = FX()) {
     using C = typename cplx<T>::type;
     with_radix(ax.R[Q], [&](auto RC) {
         constexpr int R = decltype(RC)::value;
@@ -217,6 +222,8 @@ __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const t
             C v[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) v[r] = ld(j + r * nb);
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = fix(j + r * nb, v[r]);
             if (Q > 0) {
                 const C *w = tw + ax.tw[Q] + jm;
 #pragma unroll
@@ -233,16 +240,16 @@ __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const t
 // All passes of a line: operands from ld, results to st, exchanges through sm (element e of this
 // line at sm[at(e)]) and, for three passes, sm2.  Every thread of the block calls it; `on`: the
 // line exists (threads of other lines only join the barriers).
-template <typename T, int SIGN, typename AT, typename LD, typename ST>
+template <typename T, int SIGN, typename AT, typename LD, typename ST, typename FX = Keep>
 __device__ __forceinline__ void line_fft(const Axis &ax, int t, int nt, bool on, typename cplx<T>::type *sm,
                                          typename cplx<T>::type *sm2, const typename cplx<T>::type *tw, AT &&at,
-                                         LD &&ld, ST &&st) {
+                                         LD &&ld, ST &&st, FX &&fix = FX()) {
     using C = typename cplx<T>::type;
     if (ax.np == 1) {
-        if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, st);
+        if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, st, fix);
         return;
     }
-    if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, [&](int e, C v) { sm[at(e)] = v; });
+    if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, [&](int e, C v) { sm[at(e)] = v; }, fix);
     __syncthreads();
     if (ax.np == 2) {
         if (on) line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e) { return sm[at(e)]; }, st);

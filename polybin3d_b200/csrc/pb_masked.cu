@@ -98,7 +98,8 @@ using fft::Axis;
 
 constexpr int MR_MAX_MAPS = 32;   // maps per chunk
 constexpr int MR_MAX_LEGS = 3;
-constexpr int MR_THREADS = 256;
+constexpr int MR_THREADS = 256;       // z passes
+constexpr int MR_LINE_THREADS = 128;  // x and y passes: five blocks, 20 warps per SM
 constexpr int MR_SMEM = 100 * 1024;
 
 struct MrLeg {
@@ -145,7 +146,7 @@ __device__ __forceinline__ void load_table(double2 *dst, const double2 *src, int
 
 // ---- X: filter + inverse transform along x ---------------------------------------------
 // block (L lines of kz, threads per line); grid (columns x runs, maps)
-__global__ void __launch_bounds__(MR_THREADS, 2) mr_x_kernel(const __grid_constant__ MrParams p, const double2 *src,
+__global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_x_kernel(const __grid_constant__ MrParams p, const double2 *src,
                                                             const double2 *table, double2 *W) {
     extern __shared__ __align__(16) double2 mr_smem[];
     const Grid &g = p.g;
@@ -192,16 +193,11 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_x_kernel(const __grid_consta
 }
 
 // ---- Y: inverse (SIGN 1) and forward (SIGN -1) transforms along y, in place ---------------
-// row_code[x n1 + y]: -1 the mask is zero on the row; partner_y * 4 + kind otherwise (kind 0: alone, 1 / 2:
-// first / second row of a packed pair).  NULL: every row, (y, y + 1) packed for even y; xs NULL: every x
-__device__ __forceinline__ int code_of(const int32_t *code, int y, int n1) {
-    if (code) return code[y];
-    const int o = y ^ 1;
-    return o >= n1 ? 4 * y : 4 * o + 1 + (y & 1);
-}
+// Rows go in pairs (y even, y + 1), the last one alone when n1 is odd; pair_on[x ceil(n1 / 2) + y / 2]:
+// the mask is not zero on both (NULL: every pair).  xs: the planes x to do (NULL: all).
 template <int SIGN>
-__global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_constant__ MrParams p, const double2 *table,
-                                                            const int32_t *xs, const int32_t *row_code, double2 *W) {
+__global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_y_kernel(const __grid_constant__ MrParams p, const double2 *table,
+                                                            const int32_t *xs, const uint8_t *pair_on, double2 *W) {
     extern __shared__ __align__(16) double2 mr_smem[];
     const Grid &g = p.g;
     const MrMap &mp = p.maps[blockIdx.y];
@@ -214,7 +210,10 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_consta
     load_table(tw, table + p.tw_y, p.ay.tw_len);
     const int line = threadIdx.x, kz = kz0 + line;
     const bool on = kz <= kz_max;
-    const int32_t *code = row_code ? row_code + (int64_t)x * g.n1 : nullptr;
+    __shared__ uint8_t act[512];
+    const int half = (g.n1 + 1) / 2;
+    for (int i = threadIdx.y * L + line; i < half; i += L * blockDim.y) act[i] = pair_on ? pair_on[x * half + i] : 1;
+    __syncthreads();
     double2 *w = W + blockIdx.y * p.w_map + (int64_t)x * g.n1 * p.ldz + kz;
     const int ry = ky_radius(g, SIGN > 0 ? mp.hi2 : p.out2, kz), row = p.ldz * (int)sizeof(double2);
     auto at = [&](int e) { return e * L + line; };
@@ -224,23 +223,30 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_y_kernel(const __grid_consta
             p.ay, threadIdx.y, blockDim.y, on, sm, sm2, tw, at,
             [&](int e) { return abs(freq_index(e, g.n1)) <= ry ? elem(w, e, row) : zero; },
             [&](int y, double2 v) {
-                if (code_of(code, y, g.n1) >= 0) elem(w, y, row) = v;
+                if (act[y >> 1]) elem(w, y, row) = v;
             });
     } else {
+        // With F the packed transform of a pair (halved on its way in), row y even holds F[kz] and row
+        // y + 1 holds i conj(F[-kz]): the transform of either row is then own - i other.  The other
+        // comes from the lane 16 further where that lane reads row y ^ 1 in the same round
+        const bool shuffle = L == 16 && (p.ay.nb[0] & 1) == 0 && (g.n1 & 1) == 0;
+        const unsigned lanes = __ballot_sync(0xffffffffu, on);
         fft::line_fft<double, -1>(
             p.ay, threadIdx.y, blockDim.y, on, sm, sm2, tw, at,
-            [&](int y) {
-                const int c = code_of(code, y, g.n1);
-                if (c < 0) return zero;
-                const double2 a = elem(w, y, row);
-                if ((c & 3) == 0) return a;
-                // packed transform F of the pair: this row holds F[kz] (first) or F[-kz] (second)
-                const double2 b = elem(w, c >> 2, row);
-                return (c & 3) == 1 ? make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y))
-                                    : make_double2(0.5 * (b.y + a.y), 0.5 * (a.x - b.x));
-            },
+            [&](int y) { return act[y >> 1] ? elem(w, y, row) : zero; },
             [&](int e, double2 v) {
                 if (abs(freq_index(e, g.n1)) <= ry) elem(w, e, row) = v;
+            },
+            [&](int y, double2 v) {
+                double2 o;
+                if (shuffle) {
+                    o.x = __shfl_xor_sync(lanes, v.x, 16);
+                    o.y = __shfl_xor_sync(lanes, v.y, 16);
+                } else {
+                    if ((y ^ 1) >= g.n1) return v;
+                    o = act[y >> 1] ? elem(w, y ^ 1, row) : zero;
+                }
+                return make_double2(v.x + o.y, v.y - o.x);
             });
     }
 }
@@ -261,7 +267,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     load_table(twf, table + p.tw_zf, af.tw_len);
     const int pr = blockIdx.x * L + threadIdx.y;
     const bool on = pr < p.n_pairs;
-    const int ra = on ? pairs[2 * pr] : 0, rb = on ? pairs[2 * pr + 1] : -1;
+    const int ra = on ? pairs[pr] : 0, rb = on && (ra % g.n1) + 1 < g.n1 ? ra + 1 : -1;
     double2 *wa = W + blockIdx.y * p.w_map + (int64_t)ra * p.ldz;
     double2 *wb = W + blockIdx.y * p.w_map + (int64_t)(rb >= 0 ? rb : 0) * p.ldz;
     const double *ma = mask + (int64_t)ra * g.n2, *mb = mask + (int64_t)(rb >= 0 ? rb : 0) * g.n2;
@@ -277,12 +283,12 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
         if (kz == 0 || 2 * kz == n) return make_double2(a.x, b.x);
         return up ? make_double2(a.x + b.y, b.x - a.y) : make_double2(a.x - b.y, a.y + b.x);
     };
-    // F[e] of the forward transform: rows hold F[kz] and F[n - kz]
+    // F[e] of the forward transform: the rows hold F[kz] and i conj(F[n - kz])
     auto stf = [&](int e, double2 v) {
         if (e <= p.kz_out) wa[e] = v;
         if (rb >= 0) {
             const int kz = e == 0 ? 0 : n - e;
-            if (kz <= p.kz_out) wb[kz] = v;
+            if (kz <= p.kz_out) wb[kz] = make_double2(v.y, v.x);
         }
     };
     auto ati = [&](int e) { return fft::row_at(ai, e); };
@@ -320,7 +326,8 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 v[r].x *= ma[t + r * nb];
-                v[r].y *= rb >= 0 ? mb[t + r * nb] : 0.0;
+                if (rb >= 0) v[r].y *= mb[t + r * nb];
+                else v[r] = make_double2(2.0 * v[r].x, 0.0);  // (the legs carry 1/2 for the unpacking of a pair)
             }
             fft::Dft<R, -1, double, double2>::run(v);
         }
@@ -358,14 +365,15 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
                                                                   double2 *W) {
     extern __shared__ __align__(16) double2 mr_smem[];
     const Grid &g = p.g;
-    const Axis &ax = p.azi;
+    const Axis &ax = p.azf;
     const int L = blockDim.y, n = ax.n, ld = fft::row_len(ax);
     double2 *tw = mr_smem, *sm = tw + ax.tw_len + threadIdx.y * ld, *sm2 = sm + L * ld;
-    load_table(tw, table + p.tw_zi, ax.tw_len);
+    load_table(tw, table + p.tw_zf, ax.tw_len);
     const int half = (g.n1 + 1) / 2, q = blockIdx.y * L + threadIdx.y;
     const bool on = q < g.n0 * half;
     const int x = on ? q / half : 0, y = on ? 2 * (q - x * half) : 0;
     const bool two = y + 1 < g.n1;
+    const double h = two ? 0.5 : 1.0;
     const int64_t ra = (int64_t)x * g.n1 + y, oi = pr.i[blockIdx.x] * g.nreal, oj = pr.j[blockIdx.x] * g.nreal;
     const double *xi = X + oi + ra * n, *xj = X + oj + ra * n;
     const double *zi = Z ? Z + oi + ra * n : nullptr, *zj = Z ? Z + oj + ra * n : nullptr;
@@ -379,17 +387,19 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
                 v.y = xi[e + n] * xj[e + n];
                 if (Z) v.y -= zi[e + n] * zj[e + n];
             }
+            v.x *= h;
+            v.y *= h;
             return v;
         },
         [&](int e, double2 v) {
             if (e <= p.kz_out) wa[e] = v;
             const int kz = e == 0 ? 0 : n - e;
-            if (two && kz <= p.kz_out) wb[kz] = v;
+            if (two && kz <= p.kz_out) wb[kz] = make_double2(v.y, v.x);
         });
 }
 
 // ---- X': forward transform along x ---------------------------------------------------------
-__global__ void __launch_bounds__(MR_THREADS, 2) mr_out_kernel(const __grid_constant__ MrParams p, const double2 *table,
+__global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_out_kernel(const __grid_constant__ MrParams p, const double2 *table,
                                                               const int32_t *x_on, const double2 *W, double2 *out) {
     extern __shared__ __align__(16) double2 mr_smem[];
     const Grid &g = p.g;
@@ -420,7 +430,8 @@ struct MrLayout {
 };
 
 static int mr_layout(const Grid &G, MrLayout *L) {
-    if (!fft::plan_axis(G.n0, false, &L->ax) || !fft::plan_axis(G.n1, false, &L->ay) ||
+    // the larger radix where the operands come from memory: all of a thread's loads in one round
+    if (!fft::plan_axis(G.n0, true, &L->ax) || !fft::plan_axis(G.n1, true, &L->ay) ||
         !fft::plan_axis(G.n2, false, &L->azi) || !fft::plan_axis(G.n2, true, &L->azf))
         return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: grid dimensions must be products of 2, 3, 5, 7, 11 and 13 "
                                         "of at most three factors up to 16");
@@ -434,7 +445,7 @@ static int mr_layout(const Grid &G, MrLayout *L) {
 
 static int mr_row_stride(const Grid &G, double k_out) {
     const int kz = std::min(G.nh2 - 1, (int)std::floor(k_out / G.kf2));
-    return (kz + 2) & ~1;
+    return (kz + 8) & ~7;  // rows of whole 128-byte lines
 }
 
 // lines per block and threads per line of an x / y transform, and its shared memory
@@ -443,7 +454,7 @@ static void line_shape(const Axis &ax, int *L, int *nt, size_t *smem) {
     *L = ax.np == 1 ? 32 : 16;
     auto bytes = [&](int l) { return ((size_t)ax.tw_len + (size_t)bufs * l * ax.n) * sizeof(double2); };
     while (*L > 2 && bytes(*L) > (size_t)MR_SMEM) *L /= 2;
-    *nt = std::max(1, std::min(ax.nb[ax.np - 1], MR_THREADS / *L));
+    *nt = std::max(1, std::min(ax.nb[0], MR_LINE_THREADS / *L));
     *smem = bytes(*L);
 }
 
@@ -537,12 +548,12 @@ extern "C" int pb_masked_rows_workspace_size(const pb_grid_t *g, double k_out, i
 extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_stride, int n_maps, int n_legs,
                               const int32_t *src_idx, const double *lo, const double *hi, const int32_t *ell,
                               const double *scale, double k_out, const double *mask, const int32_t *pairs, int n_pairs,
-                              const int32_t *row_code, const int32_t *xs, int n_x, const int32_t *x_on,
+                              const uint8_t *pair_on, const int32_t *xs, int n_x, const int32_t *x_on,
                               const void *table, void *out, void *workspace, size_t workspace_bytes, void *stream) {
     Grid G;
     int st = make_grid(g, &G);
     if (st) return st;
-    if (!src || !src_idx || !lo || !hi || !ell || !scale || !mask || !pairs || !row_code || !xs || !x_on || !table || !out)
+    if (!src || !src_idx || !lo || !hi || !ell || !scale || !mask || !pairs || !pair_on || !xs || !x_on || !table || !out)
         return fail(PB_ERR_INVALID, "pb_masked_rows: NULL argument");
     if (n_maps < 1 || n_legs < 1 || n_legs > MR_MAX_LEGS || n_pairs < 1 || n_x < 1 || n_x > G.n0 || !(k_out > 0.0))
         return fail(PB_ERR_INVALID, "pb_masked_rows: bad sizes");
@@ -578,7 +589,7 @@ extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_s
             double top = 0.0, low = HUGE_VAL;
             for (int q = 0; q < n_legs; ++q) {
                 const int i = (m0 + m) * n_legs + q;
-                mp.leg[q] = MrLeg{threshold_sq(lo[i]), threshold_sq(hi[i]), scale[i], src_idx[i], ell[i]};
+                mp.leg[q] = MrLeg{threshold_sq(lo[i]), threshold_sq(hi[i]), 0.5 * scale[i], src_idx[i], ell[i]};
                 top = std::max(top, hi[i]);
                 low = std::min(low, std::max(lo[i], 0.0));
             }
@@ -589,11 +600,11 @@ extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_s
         const int runs_x = p.kz_out / sh.Lx + 1, runs_y = p.kz_out / sh.Ly + 1;
         mr_x_kernel<<<dim3(G.n1 * runs_x, nm), dim3(sh.Lx, sh.Tx), sh.sx, s>>>(p, (const double2 *)src, tab, W);
         PB_LAUNCH_CHECK("pb_masked_rows(x)");
-        mr_y_kernel<1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, row_code, W);
+        mr_y_kernel<1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, pair_on, W);
         PB_LAUNCH_CHECK("pb_masked_rows(y)");
         mr_z_kernel<<<dim3((n_pairs + sh.Lz - 1) / sh.Lz, nm), dim3(sh.Tz, sh.Lz), sh.sz, s>>>(p, tab, pairs, mask, W);
         PB_LAUNCH_CHECK("pb_masked_rows(z)");
-        mr_y_kernel<-1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, row_code, W);
+        mr_y_kernel<-1><<<dim3(n_x * runs_y, nm), dim3(sh.Ly, sh.Ty), sh.sy, s>>>(p, tab, xs, pair_on, W);
         PB_LAUNCH_CHECK("pb_masked_rows(y')");
         mr_out_kernel<<<dim3(G.n1 * runs_x, nm), dim3(sh.Lx, sh.Tx), sh.sx, s>>>(p, tab, x_on, W,
                                                                                  (double2 *)out + (int64_t)m0 * G.nhalf);
