@@ -11,6 +11,7 @@
 //   j + r nb, twiddled by e^{+-2 pi i r (j mod Ns) / (Ns R)}, to (j / Ns) Ns R + j mod Ns + r Ns.
 #pragma once
 #include <cmath>
+#include <type_traits>
 #include "pb_common.cuh"
 
 namespace pb {
@@ -261,11 +262,76 @@ __device__ __forceinline__ void line_fft(const Axis &ax, int t, int nt, bool on,
     if (on) line_pass<T, SIGN, 2>(ax, t, nt, tw, [&](int e) { return sm2[at(e)]; }, st);
 }
 
-// ---- host side ----------------------------------------------------------------------
-// Radices of n: two passes where possible (the larger radix last), else three; false when n has
-// another prime factor than 2, 3, 5, 7, 11, 13 or needs more passes.  `reversed`: the same radices in the
-// opposite order.
-bool plan_axis(int n, bool reversed, Axis *ax);
+// ---- planning -----------------------------------------------------------------------
+// n = R0 R1 with both radices at most 16 and R0 <= R1 as large as possible; 0 when impossible
+__host__ __device__ constexpr int balanced_radix(int n) {
+    for (int r = 16; r >= 2; --r)
+        if (n % r == 0 && n / r <= MAX_RADIX && n / r >= r) return r;
+    return 0;
+}
+
+// Radices of n: two passes where possible (the larger radix last), else three, the largest last radix
+// whose cofactor splits in two; np = 0 when n has another prime factor than 2, 3, 5, 7, 11, 13 or needs
+// more passes.  `reversed`: the same radices in the opposite order.
+__host__ __device__ constexpr Axis make_axis(int n, bool reversed) {
+    Axis ax{};
+    int r[3] = {n, 0, 0};
+    if (n < 2 || n > 1024) return ax;
+    int np = 0;
+    if (n <= MAX_RADIX) {
+        np = 1;
+    } else if (balanced_radix(n)) {
+        np = 2;
+        r[0] = balanced_radix(n);
+        r[1] = n / r[0];
+    } else {
+        for (int c = MAX_RADIX; c >= 2 && !np; --c) {
+            if (n % c) continue;
+            const int b = balanced_radix(n / c);
+            if (b && n / c / b <= c) {
+                np = 3;
+                r[0] = b;
+                r[1] = n / c / b;
+                r[2] = c;
+            }
+        }
+        if (!np) return ax;
+    }
+    if (reversed && np > 1) {
+        const int t = r[0];
+        r[0] = r[np - 1];
+        r[np - 1] = t;
+    }
+    ax.n = n;
+    ax.np = np;
+    int ns = 1;
+    for (int q = 0; q < np; ++q) {
+        ax.R[q] = r[q];
+        ax.nb[q] = n / r[q];
+        ax.ns[q] = ns;
+        ax.tw[q] = ax.tw_len;
+        if (q > 0) ax.tw_len += (r[q] - 1) * ns;
+        ns *= r[q];
+    }
+    ax.div_ns1 = ((1u << 20) + (uint32_t)r[0] - 1) / (uint32_t)r[0];
+    ax.pad = (r[0] % 2 == 0) ? 1 : 0;
+    return ax;
+}
+
+// The axis a kernel works with: the plan of a compile-time length N (radices, strides and counts fold
+// into the code), or for N = 0 the run-time plan.
+template <int N, bool REV> struct AxisUse {
+    Axis v;
+    __device__ __forceinline__ AxisUse(const Axis &) {
+        constexpr Axis c = make_axis(N, REV);
+        v = c;
+    }
+};
+template <bool REV> struct AxisUse<0, REV> {
+    const Axis &v;
+    __device__ __forceinline__ AxisUse(const Axis &a) : v(a) {}
+};
+
 // e^{2 pi i r jm / (Ns R)} of every pass into out[tw_len] (re, im pairs)
 void fill_twiddles(const Axis &ax, double *out);
 

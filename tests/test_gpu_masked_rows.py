@@ -42,6 +42,9 @@ def a_mask(kind, n, rng):
 @pytest.mark.parametrize("kind", ["full", "ragged", "row"])
 @pytest.mark.parametrize("n,kf,legs", [
     ((16, 12, 10), (1.0, 1.0, 1.0), 1),
+    ((60, 72, 90), (1.0, 1.0, 1.0), 1),
+    ((100, 64, 48), (1.0, 1.0, 1.0), 3),
+    ((216, 15, 200), (0.1, 1.0, 0.1), 1),
     ((32, 48, 64), (1.0, 1.0, 1.0), 1),
     ((27, 35, 22), (1.0, 0.8, 1.2), 3),
     ((128, 20, 26), (1.0, 1.0, 1.0), 3),
