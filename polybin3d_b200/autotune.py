@@ -8,8 +8,8 @@ processes -- set the winner before launching.  Tuned shapes:
 * the tensor-core triplet contraction (from plain maps and from a tiled set): voxels per
   tile (plain maps: 128 / 64), staging ring depth, the barrier-wait form, accumulator sets
   (never the TMEM chain length, which changes the FP32 rounding);
-* the k-bin reduction of many rows (>= 16): lane-per-row kernel (warps per block, blocks
-  per SM) against the mode-tile kernel;
+* the k-bin reduction of many rows (>= 16): the default (FP64: the staged kernel) against the
+  lane-per-row kernel (warps per block, blocks per SM) and the mode-tile kernel;
 * routes that do the same work two ways (choose_route): the bispectrum's cubic sums from
   plain maps or from a tiled set (synthesis and contraction timed together).
 
@@ -201,7 +201,7 @@ def bin_reduce(grid, precision, mode, a, b, n_rows, edges, ells, scale, out, ws,
     nk = len(edges) - 1
     n_ell = len(np.asarray(ells).reshape(-1)) // 2
     dev = out.device
-    key = "red|%s|%d,%d,%d|%d|%d|%d|%d|%d" % (device_tag(dev), grid.n[0], grid.n[1], grid.n[2], n_rows, nk, n_ell,
+    key = "red|staged|%s|%d,%d,%d|%d|%d|%d|%d|%d" % (device_tag(dev), grid.n[0], grid.n[1], grid.n[2], n_rows, nk, n_ell,
                                               precision, mode)
     scratch = None
 

@@ -220,6 +220,224 @@ __global__ void __launch_bounds__(RED_THREADS) binred_rows_kernel(Grid g, const 
     }
 }
 
+// bin (-1: none) and deg L_la L_lb of every mode, tabulated once per call for the many-row kernels
+template <typename B>
+__global__ void binred_geom_kernel(Grid g, RedParams p, B *mbin, double *mw) {
+    __shared__ double edges[PB_RED_MAX_BINS + 1];
+    for (int i = threadIdx.x; i <= p.nk; i += blockDim.x) edges[i] = p.edges[i];
+    __syncthreads();
+    const int ne = p.n_ell;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < g.nhalf;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const Mode md = mode_of(g, idx);
+        const int bin = find_bin(edges, p.nk, md.k);
+        mbin[idx] = (B)bin;
+        if (bin >= 0) {
+#pragma unroll
+            for (int e = 0; e < PB_RED_MAX_ELLS; ++e)
+                if (e < ne) mw[idx * ne + e] = md.deg * legendre(p.la[e], md.mu) * legendre(p.lb[e], md.mu);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Many FP64 rows, staged: a block owns up to 32 rows and walks the binned runs of its kz lines in
+// segments of 16 modes.  The rows' values arrive in shared memory by cp.async, 256 contiguous bytes
+// per row and two segments ahead, the segment's geometry (tabulated by binred_geom_kernel) and the
+// shared spectrum beside them; a lane owns one row (odd row stride: no bank conflicts) and the
+// multipoles of its warp's share, keeps the sums of the current bin in registers and adds
+// them to its own slot of the block's accumulators [bin][e][row] when the bin changes: no
+// atomics, a fixed order.  Streaming from memory bounds it; the lane-per-row kernel below read each
+// row by one lane, 64 bytes at a time with 11 warps per SM.  (Computing the geometry in a warp of its
+// own instead of reading the table took 375 us: its sqrt, search and Legendre chain per segment was longer
+// than everything else.)
+// Measured on a B200, 60 rows of 128^3, 20 bins, l = 0, 2, 4: 193 us against 450 us
+// for the lane-per-row kernel (finalize and table included; 120 rows, 40 bins 497 against 1130 us; 203 rows, 12 bins,
+// l = 0 307 against 690 us; the two tie at 64^3).
+// ------------------------------------------------------------------------------------
+constexpr int RT_SEG = 16;        // modes per segment
+constexpr int RT_STAGES = 3;
+constexpr int RT_ROWS = 32;       // rows per block (64 a block took 226 against 193 us)
+constexpr int RT_LD = RT_SEG + 1;
+constexpr int RT_SMEM = 220 * 1024;
+// warps of a block: groups of multipoles (one or two per thread) times parts of a segment (with one or
+// two multipoles, so that the block still has four warps)
+__host__ __device__ constexpr int rt_egroups(int ne) { return ne <= 4 ? ne : (ne + 1) / 2; }
+__host__ __device__ constexpr int rt_parts(int ne) { return ne == 1 ? 4 : ne == 2 ? 2 : 1; }
+__host__ __device__ constexpr int rt_warps(int ne) { return rt_egroups(ne) * rt_parts(ne); }
+
+__device__ __forceinline__ void rt_copy16(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+
+template <int BYTES> __device__ __forceinline__ void rt_copy(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gmem), "n"(BYTES));
+}
+
+__host__ __device__ constexpr size_t rt_smem(int nk, int ne) {
+    constexpr int RB = RT_ROWS;
+    return (size_t)RT_STAGES * ((size_t)RB * RT_LD * 16 + RT_SEG * 16 + (size_t)ne * RT_SEG * 8 + RT_SEG * 4) +
+           (size_t)rt_parts(ne) * nk * ne * RB * 8;
+}
+
+// the next segment of the block's lines: first mode and count (0: done)
+struct RtWalk {
+    int line, step, n_lines, l, l_end;
+    float fx, fy, lo2, hi2;
+    __device__ __forceinline__ int next(const Grid &g, int64_t &first) {
+        while (l >= l_end) {
+            line += step;
+            if (line >= n_lines) return 0;
+            // the run of the line that may hold binned modes, in units of kf2; FP32 with two modes of
+            // margin each side (the bins of the table decide)
+            const int i = (int)((uint32_t)line / (uint32_t)g.n1), j = (int)line - i * g.n1;
+            const float kx = freq_index(i, g.n0) * fx, ky = freq_index(j, g.n1) * fy;
+            const float r2 = kx * kx + ky * ky, h2 = hi2 * (1.0f + 1e-5f) - r2;
+            if (h2 < 0.0f) continue;
+            l = lo2 > r2 ? max(0, (int)sqrtf(lo2 - r2) - 2) : 0;
+            l_end = (int)fminf((float)g.nh2, sqrtf(h2) + 3.0f);
+        }
+        first = (int64_t)line * g.nh2 + l;
+        const int c = min(RT_SEG, l_end - l);
+        l += c;
+        return c;
+    }
+};
+
+template <int MODE, int NE>
+__global__ void __launch_bounds__(32 * rt_warps(NE)) binred_tile_kernel(Grid g, const double2 *a, const double2 *b,
+                                                                 int64_t row_stride, int n_rows, int nk, float lo,
+                                                                 float hi, const int32_t *mbin, const double *mw,
+                                                                 double *partials) {
+    constexpr int RB = RT_ROWS, EG = rt_egroups(NE), EP = (NE + EG - 1) / EG, MS = rt_parts(NE);
+    constexpr int NW = rt_warps(NE), NT = 32 * NW, PART = RT_SEG / MS;
+    extern __shared__ __align__(16) unsigned char rt_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2 *const rows = reinterpret_cast<double2 *>(rt_raw);                    // [stage][RB][RT_LD]
+    double2 *const as = rows + (size_t)RT_STAGES * RB * RT_LD;                    // [stage][RT_SEG]
+    double *const wt = reinterpret_cast<double *>(as + RT_STAGES * RT_SEG);       // [stage][RT_SEG][NE]
+    double *const acc = wt + RT_STAGES * NE * RT_SEG;                             // [part][bin][e][RB]
+    int *const bins = reinterpret_cast<int *>(acc + (size_t)MS * nk * NE * RB);   // [stage][RT_SEG]
+    const int r0 = blockIdx.y * RB, nr = min(RB, n_rows - r0);
+    const double2 *const src = (MODE == PB_RED_CROSS ? b : a) + (int64_t)r0 * row_stride;
+    for (int i = threadIdx.x; i < MS * nk * NE * RB; i += NT) acc[i] = 0.0;
+    const float inv = 1.0f / (float)g.kf2;
+    RtWalk walk{(int)blockIdx.x - (int)gridDim.x, (int)gridDim.x, g.n0 * g.n1, 0, 0,
+                (float)g.kf0 * inv, (float)g.kf1 * inv, lo > 0.0f ? lo * lo * inv * inv : 0.0f, hi * hi * inv * inv};
+    int count[RT_STAGES];  // of the segments in flight (every thread walks alike)
+    auto issue = [&](int st) -> int {
+        int64_t first = 0;
+        const int c = walk.next(g, first);
+        // half a warp per row: 256 contiguous bytes
+        const int m = lane & (RT_SEG - 1);
+        if (m < c) {
+            double2 *dst = rows + (size_t)st * RB * RT_LD + m;
+            const double2 *from = src + first + m;
+            for (int r = 2 * warp + (lane >> 4); r < nr; r += 2 * NW) rt_copy16(dst + r * RT_LD, from + (int64_t)r * row_stride);
+            if (MODE == PB_RED_CROSS && warp == NW - 1 && lane < RT_SEG) rt_copy16(as + st * RT_SEG + m, a + first + m);
+            if (warp == NW - 1 && lane >= RT_SEG) rt_copy<4>(bins + st * RT_SEG + m, mbin + first + m);
+        }
+        if (threadIdx.x < c * NE) rt_copy<8>(wt + st * RT_SEG * NE + threadIdx.x, mw + first * NE + threadIdx.x);
+        asm volatile("cp.async.commit_group;\n" ::);
+        return c;
+    };
+#pragma unroll
+    for (int st = 0; st < RT_STAGES - 1; ++st) count[st] = issue(st);
+    const int row = lane, eg = warp % EG, part = warp / EG;
+    const bool mine = row < nr;
+    double *const own = acc + (size_t)part * nk * NE * RB + row;
+    double sum[EP];
+#pragma unroll
+    for (int k = 0; k < EP; ++k) sum[k] = 0.0;
+    int cur = -1;
+    auto flush = [&]() {
+#pragma unroll
+        for (int k = 0; k < EP; ++k) {
+            const int e = eg + k * EG;
+            if (cur >= 0 && e < NE) own[((size_t)cur * NE + e) * RB] += sum[k];
+            sum[k] = 0.0;
+        }
+    };
+    bool more = true;
+    while (more) {
+#pragma unroll
+        for (int st = 0; st < RT_STAGES; ++st) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(RT_STAGES - 2));
+            __syncthreads();  // segment st is in shared memory; everyone is done with the one before it
+            count[(st + RT_STAGES - 1) % RT_STAGES] = issue((st + RT_STAGES - 1) % RT_STAGES);
+            const int c = count[st];
+            if (c == 0) {
+                more = false;
+                break;
+            }
+            if (mine) {
+                const double2 *v = rows + ((size_t)st * RB + row) * RT_LD, *u = as + st * RT_SEG;
+                const double *w = wt + st * RT_SEG * NE + eg;
+                const int *bn = bins + st * RT_SEG;
+                const int m1 = min(c, (part + 1) * PART);
+                for (int m = part * PART; m < m1; m += 4) {
+                    // four modes' operands before any is used (values past c are stale, their bins skip them)
+                    double f[4], ww[4][EP];
+                    int bb[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        bb[q] = m + q < m1 ? bn[m + q] : -1;
+                        const double2 x = v[m + q];
+                        if (MODE == PB_RED_CROSS) {
+                            const double2 y = u[m + q];
+                            f[q] = y.x * x.x + y.y * x.y;
+                        } else {
+                            f[q] = x.x * x.x + x.y * x.y;
+                        }
+#pragma unroll
+                        for (int k = 0; k < EP; ++k) ww[q][k] = eg + k * EG < NE ? w[(m + q) * NE + k * EG] : 0.0;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (bb[q] < 0) continue;
+                        if (bb[q] != cur) {
+                            flush();
+                            cur = bb[q];
+                        }
+#pragma unroll
+                        for (int k = 0; k < EP; ++k) sum[k] += f[q] * ww[q][k];
+                    }
+                }
+            }
+        }
+    }
+    if (mine) flush();
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    const int per = nk * NE;
+    for (int i = threadIdx.x; i < per * nr; i += NT) {
+        const int r = i / per, j = i - r * per, e = j / nk, bin = j - e * nk;
+        double x = 0.0;
+#pragma unroll
+        for (int k = 0; k < MS; ++k) x += acc[(((size_t)k * nk + bin) * NE + e) * RB + r];
+        partials[((int64_t)(r0 + r) * gridDim.x + blockIdx.x) * per + j] = x;
+    }
+}
+
+struct TileLaunch {
+    int gx;
+    size_t smem, geom_bytes;   // bins (int32, padded to 256 bytes) and weights of every mode
+};
+// the staged kernel serves 16 rows and more whose accumulators fit beside the stages
+static bool tile_plan(const Grid &G, int n_rows, int nk, int n_ell, TileLaunch *t) {
+    if (tuning().red_method != 0 || n_rows < 16) return false;
+    t->smem = rt_smem(nk, n_ell);
+    if (t->smem > (size_t)RT_SMEM) return false;
+    // as many blocks as are resident at once, shared among the groups of rows
+    const int groups = (n_rows + RT_ROWS - 1) / RT_ROWS;
+    const int per_sm = (int)std::min<size_t>(5, (225 * 1024) / (t->smem + 1024));
+    t->gx = (int)std::min<int64_t>((int64_t)G.n0 * G.n1, std::max(1, (per_sm * num_sms() + groups - 1) / groups));
+    t->geom_bytes = ((size_t)G.nhalf * 4 + 255) / 256 * 256 + (size_t)G.nhalf * n_ell * sizeof(double);
+    return true;
+}
+
 // ------------------------------------------------------------------------------------
 // Many rows, one lane per row.  The mode geometry (bin and deg x L_la L_lb per mode, FP64)
 // is tabulated once per call by binred_geom_kernel.  A warp then walks kz lines of the half
@@ -232,24 +450,6 @@ __global__ void __launch_bounds__(RED_THREADS) binred_rows_kernel(Grid g, const 
 // range is read (|k| grows along a kz line, so it is one contiguous run of modes).
 // ------------------------------------------------------------------------------------
 constexpr int BL_MODES = 4;  // modes per lane per step (the next step's values load meanwhile)
-
-__global__ void binred_geom_kernel(Grid g, RedParams p, int8_t *mbin, double *mw) {
-    __shared__ double edges[PB_RED_MAX_BINS + 1];
-    for (int i = threadIdx.x; i <= p.nk; i += blockDim.x) edges[i] = p.edges[i];
-    __syncthreads();
-    const int ne = p.n_ell;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < g.nhalf;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const Mode md = mode_of(g, idx);
-        const int bin = find_bin(edges, p.nk, md.k);
-        mbin[idx] = (int8_t)bin;
-        if (bin >= 0) {
-#pragma unroll
-            for (int e = 0; e < PB_RED_MAX_ELLS; ++e)
-                if (e < ne) mw[idx * ne + e] = md.deg * legendre(p.la[e], md.mu) * legendre(p.lb[e], md.mu);
-        }
-    }
-}
 
 template <typename T, int MODE, int NE>
 __global__ void __launch_bounds__(256) binred_lanes_kernel(Grid g, const typename cplx<T>::type *a,
@@ -695,6 +895,9 @@ extern "C" int pb_bin_reduce_workspace_size(const pb_grid_t *g, int n_rows, int 
     if (!bytes) return fail(PB_ERR_INVALID, "bytes is NULL");
     if (n_rows < 1 || nk < 1 || n_ell < 1) return fail(PB_ERR_INVALID, "pb_bin_reduce: empty reduction");
     *bytes = (size_t)n_rows * red_blocks(G) * nk * n_ell * sizeof(double);
+    TileLaunch t;
+    if (tile_plan(G, n_rows, nk, n_ell, &t))
+        *bytes = std::max(*bytes, t.geom_bytes + (size_t)n_rows * t.gx * nk * n_ell * sizeof(double));
     LanesLaunch L;
     if (lanes_plan(G, n_rows, nk, n_ell, &L))
         *bytes = std::max(*bytes, L.geom_bytes + (size_t)n_rows * L.gx * nk * n_ell * sizeof(double));
@@ -734,6 +937,40 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
     int nb = red_blocks(G);
     size_t need = (size_t)n_rows * nb * nk * n_ell * sizeof(double);
     cudaStream_t s = as_stream(stream);
+    TileLaunch TT;
+    if (mode != PB_RED_REAL2 && precision == PB_F64 && tile_plan(G, n_rows, nk, n_ell, &TT)) {
+        need = TT.geom_bytes + (size_t)n_rows * TT.gx * nk * n_ell * sizeof(double);
+        if (!workspace || workspace_bytes < need)
+            return fail(PB_ERR_WORKSPACE, "pb_bin_reduce: workspace too small (need " + std::to_string(need) + " bytes)");
+        int32_t *mbin = (int32_t *)workspace;
+        double *mw = (double *)((char *)workspace + ((size_t)G.nhalf * 4 + 255) / 256 * 256);
+        double *partials = (double *)((char *)workspace + TT.geom_bytes);
+        binred_geom_kernel<int32_t><<<(int)std::min<int64_t>((G.nhalf + 255) / 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
+            G, p, mbin, mw);
+        PB_LAUNCH_CHECK("pb_bin_reduce(geometry)");
+        const dim3 tgrid(TT.gx, (n_rows + RT_ROWS - 1) / RT_ROWS);
+#define PB_RT_CASE(M, NE)                                                                                       \
+    case NE:                                                                                                    \
+        PB_CUDA(cudaFuncSetAttribute(binred_tile_kernel<M, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+                                     (int)TT.smem));                                                            \
+        binred_tile_kernel<M, NE><<<tgrid, 32 * rt_warps(NE), TT.smem, s>>>(                                    \
+            G, (const double2 *)a, (const double2 *)b, row_stride, n_rows, nk, (float)edges[0], (float)edges[nk], \
+            mbin, mw, partials);                                                                                \
+        break;
+#define PB_RT_MODE(M)                                                                                       \
+    switch (n_ell) {                                                                                        \
+        PB_RT_CASE(M, 1) PB_RT_CASE(M, 2) PB_RT_CASE(M, 3) PB_RT_CASE(M, 4) PB_RT_CASE(M, 5) PB_RT_CASE(M, 6) \
+        PB_RT_CASE(M, 7) PB_RT_CASE(M, 8) PB_RT_CASE(M, 9)                                                   \
+    }
+        if (mode == PB_RED_ABS2) PB_RT_MODE(PB_RED_ABS2)
+        else PB_RT_MODE(PB_RED_CROSS)
+#undef PB_RT_MODE
+#undef PB_RT_CASE
+        PB_LAUNCH_CHECK("pb_bin_reduce(tile)");
+        launch_binred_finalize(partials, TT.gx, nk * n_ell, n_rows, scale, out, accumulate, s);
+        PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
+        return PB_OK;
+    }
     LanesLaunch LL;
     if (mode != PB_RED_REAL2 && lanes_plan(G, n_rows, nk, n_ell, &LL)) {
         // geometry table, then one lane per row (binred_lanes_kernel)
@@ -744,7 +981,7 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
         double *mw = (double *)((char *)workspace + ((size_t)G.nhalf + 255) / 256 * 256);
         double *partials = (double *)((char *)workspace + LL.geom_bytes);
         const int gg = (int)std::min<int64_t>((G.nhalf + 255) / 256, (int64_t)num_sms() * 8);
-        binred_geom_kernel<<<gg, 256, 0, s>>>(G, p, mbin, mw);
+        binred_geom_kernel<int8_t><<<gg, 256, 0, s>>>(G, p, mbin, mw);
         PB_LAUNCH_CHECK("pb_bin_reduce(geometry)");
         dim3 lgrid(LL.gx, (n_rows + 31) / 32);
         const void *rows = (mode == PB_RED_CROSS) ? b : a;
