@@ -1088,61 +1088,103 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
 
 // ------------------------------------------------------------------------------------
 // Fisher rows over one k-shell:  out[orow[r]][j] = scale * sum_{i} deg_i Re(conj(F[key_r](m_i)) Q_j(m_i))
-// over the shell's mode list m_i.  Chunked: each block stages SR_CH modes of <= SR_R rows
-// and SR_CT columns in shared memory, writes one partial per (chunk, row, column);
-// a second pass sums the chunks in order.
+// over the shell's mode list m_i: a dense product of <= 32 rows with all columns, FP64.  A block owns
+// 8 RPT rows and 64 columns and walks its part of the list 16 modes at a time: the next modes' values
+// (gathered, runs of kz) load into registers while the current ones, staged in shared memory with an
+// odd row stride, feed RPT x 4 sums per thread.  One partial per block, summed in order by a second
+// pass.  Reading Q (each mode once per group of rows) bounds it.  The kernel before took one
+// sum per shared-memory pair and wrote a partial every 32 modes: 90 us a shell of 17 rows, 203
+// columns and 37,000 modes at 128^3 (and 11 us to sum the partials) against 56 us.
 // ------------------------------------------------------------------------------------
 namespace pb {
-constexpr int SR_THREADS = 256;
-constexpr int SR_CH = 32;   // modes per chunk
+constexpr int SR_THREADS = 128;
+constexpr int SR_M = 16;    // modes per step
 constexpr int SR_R = 32;    // rows per launch
-constexpr int SR_CT = 32;   // columns per block
+constexpr int SR_CT = 64;   // columns per block
 
 struct ShellRowKeys {
     int32_t key[SR_R];
 };
 
-template <typename T>
+template <typename T, int RPT>
 __global__ void __launch_bounds__(SR_THREADS) shell_rows_kernel(Grid g, const typename cplx<T>::type *F,
                                                                const typename cplx<T>::type *Q, int n_rows,
                                                                int n_cols, const int64_t *modes, int64_t n_modes,
-                                                               ShellRowKeys keys, double *partials) {
+                                                               int64_t per_block, ShellRowKeys keys, double *partials) {
     using C = typename cplx<T>::type;
-    __shared__ double2 Fs[SR_R][SR_CH + 1];
-    __shared__ double2 Qs[SR_CT][SR_CH + 1];
-    const int chunk = blockIdx.x;
+    constexpr int NR = 8 * RPT, FL = NR * SR_M / SR_THREADS, QL = SR_CT * SR_M / SR_THREADS;
+    __shared__ double2 Fs[NR][SR_M + 1];
+    __shared__ double2 Qs[SR_CT][SR_M + 1];
+    const int tid = threadIdx.x, m = tid & (SR_M - 1), h = tid / SR_M;   // loads: mode m of rows h, h + 8, ...
+    const int tx = tid & 15, ty = tid >> 4;                              // sums: columns tx + 16 c, rows ty + 8 r
     const int j0 = blockIdx.y * SR_CT;
-    const int64_t m0 = (int64_t)chunk * SR_CH;
-    const int ncols_here = min(SR_CT, n_cols - j0);
-    for (int e = threadIdx.x; e < SR_R * SR_CH; e += SR_THREADS) {
-        int r = e / SR_CH, i = e - r * SR_CH;
-        double2 v = make_double2(0.0, 0.0);
-        if (r < n_rows && m0 + i < n_modes) {
-            int64_t idx = modes[m0 + i];
-            double deg = ((idx % g.nh2) > 0) ? 2.0 : 1.0;
-            C f = F[(int64_t)keys.key[r] * g.nhalf + idx];
-            v = make_double2(deg * (double)f.x, deg * (double)f.y);
+    const int64_t i0 = (int64_t)blockIdx.x * per_block, i1 = min(i0 + per_block, n_modes);
+    double acc[RPT][4];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+    C f[FL], q[QL];
+    double deg = 0.0;
+    // this thread's mode of the step from i, -1 past the end
+    auto mode_at = [&](int64_t i) -> int64_t { return i + m < i1 ? modes[i + m] : -1; };
+    auto fetch = [&](int64_t idx) {
+        deg = (uint64_t)idx % (uint64_t)g.nh2 > 0 ? 2.0 : 1.0;
+#pragma unroll
+        for (int k = 0; k < FL; ++k) {
+            const int r = h + 8 * k;
+            f[k].x = f[k].y = 0;
+            if (idx >= 0 && r < n_rows) f[k] = F[(int64_t)keys.key[r] * g.nhalf + idx];
         }
-        Fs[r][i] = v;
-    }
-    for (int e = threadIdx.x; e < SR_CT * SR_CH; e += SR_THREADS) {
-        int j = e / SR_CH, i = e - j * SR_CH;
-        double2 v = make_double2(0.0, 0.0);
-        if (j < ncols_here && m0 + i < n_modes) {
-            C q = Q[(int64_t)(j0 + j) * g.nhalf + modes[m0 + i]];
-            v = make_double2((double)q.x, (double)q.y);
+#pragma unroll
+        for (int k = 0; k < QL; ++k) {
+            const int j = j0 + h + 8 * k;
+            q[k].x = q[k].y = 0;
+            if (idx >= 0 && j < n_cols) q[k] = Q[(int64_t)j * g.nhalf + idx];
         }
-        Qs[j][i] = v;
+    };
+    int64_t next = mode_at(i0);
+    fetch(next);
+    next = mode_at(i0 + SR_M);
+    for (int64_t i = i0; i < i1; i += SR_M) {
+        __syncthreads();  // the step before has been used
+#pragma unroll
+        for (int k = 0; k < FL; ++k) Fs[h + 8 * k][m] = make_double2(deg * (double)f[k].x, deg * (double)f[k].y);
+#pragma unroll
+        for (int k = 0; k < QL; ++k) Qs[h + 8 * k][m] = make_double2((double)q[k].x, (double)q[k].y);
+        __syncthreads();
+        if (i + SR_M < i1) {
+            fetch(next);
+            next = mode_at(i + 2 * SR_M);
+        }
+#pragma unroll 4
+        for (int k = 0; k < SR_M; ++k) {
+            double2 a[RPT], b[4];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) a[r] = Fs[ty + 8 * r][k];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) b[c] = Qs[tx + 16 * c][k];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] += a[r].x * b[c].x + a[r].y * b[c].y;
+        }
     }
-    __syncthreads();
-    for (int o = threadIdx.x; o < SR_R * SR_CT; o += SR_THREADS) {
-        int r = o / SR_CT, j = o - r * SR_CT;
-        if (r >= n_rows || j >= ncols_here) continue;
-        double s = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < SR_CH; ++i) s += Fs[r][i].x * Qs[j][i].x + Fs[r][i].y * Qs[j][i].y;
-        partials[((int64_t)chunk * n_rows + r) * n_cols + j0 + j] = s;
-    }
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int row = ty + 8 * r, col = j0 + tx + 16 * c;
+            if (row < n_rows && col < n_cols) partials[((int64_t)blockIdx.x * n_rows + row) * n_cols + col] = acc[r][c];
+        }
+}
+
+// parts of the mode list: enough blocks for three per SM, at least eight steps each
+static int shell_parts(int64_t n_modes, int n_cols, int64_t *per_block) {
+    const int64_t steps = std::max<int64_t>(1, (n_modes + SR_M - 1) / SR_M), tiles = (n_cols + SR_CT - 1) / SR_CT;
+    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>((3LL * num_sms() + tiles - 1) / tiles, steps / 8));
+    *per_block = (steps + parts - 1) / parts * SR_M;
+    return (int)std::max<int64_t>(1, (n_modes + *per_block - 1) / *per_block);
 }
 
 struct ShellRowOut {
@@ -1164,8 +1206,8 @@ extern "C" int pb_shell_rows_workspace_size(int64_t n_modes, int n_rows, int n_c
     if (!bytes) return fail(PB_ERR_INVALID, "bytes is NULL");
     if (n_modes < 0 || n_rows < 1 || n_rows > SR_R || n_cols < 1)
         return fail(PB_ERR_INVALID, "pb_shell_rows_workspace_size: bad sizes");
-    int64_t n_chunks = std::max<int64_t>(1, (n_modes + SR_CH - 1) / SR_CH);
-    *bytes = (size_t)n_chunks * n_rows * n_cols * sizeof(double);
+    int64_t per_block;
+    *bytes = (size_t)shell_parts(n_modes, n_cols, &per_block) * n_rows * n_cols * sizeof(double);
     return PB_OK;
 }
 
@@ -1190,24 +1232,28 @@ extern "C" int pb_shell_rows(const pb_grid_t *g, int precision, const void *F, i
         if (r < n_rows && orow.orow[r] < 0) return fail(PB_ERR_INVALID, "pb_shell_rows: negative output row");
     }
     if (out_stride == 0) out_stride = n_cols;
-    int64_t n_chunks = std::max<int64_t>(1, (n_modes + SR_CH - 1) / SR_CH);
+    int64_t per_block;
+    const int n_chunks = shell_parts(n_modes, n_cols, &per_block);  // an empty shell: one block of zeros
     size_t need = (size_t)n_chunks * n_rows * n_cols * sizeof(double);
     if (!workspace || workspace_bytes < need) return fail(PB_ERR_WORKSPACE, "pb_shell_rows: workspace too small");
-    if (n_chunks > 2147483647) return fail(PB_ERR_INVALID, "pb_shell_rows: too many modes");
     cudaStream_t s = as_stream(stream);
     dim3 grid((unsigned)n_chunks, (n_cols + SR_CT - 1) / SR_CT);
     double *partials = (double *)workspace;
-    if (n_modes == 0) {
-        // empty shell: zero partials through a one-chunk launch with no modes
+    if (precision != PB_F64 && precision != PB_F32) return fail(PB_ERR_INVALID, "bad precision");
+#define PB_SR_LAUNCH(T, RPT)                                                                                       \
+    shell_rows_kernel<T, RPT><<<grid, SR_THREADS, 0, s>>>(G, (const cplx<T>::type *)F, (const cplx<T>::type *)Q,   \
+                                                          n_rows, n_cols, modes, n_modes, per_block, keys, partials)
+#define PB_SR_ROWS(T)                              \
+    switch ((n_rows + 7) / 8) {                    \
+        case 1: PB_SR_LAUNCH(T, 1); break;         \
+        case 2: PB_SR_LAUNCH(T, 2); break;         \
+        case 3: PB_SR_LAUNCH(T, 3); break;         \
+        default: PB_SR_LAUNCH(T, 4); break;        \
     }
-    if (precision == PB_F64)
-        shell_rows_kernel<double><<<grid, SR_THREADS, 0, s>>>(G, (const double2 *)F, (const double2 *)Q, n_rows,
-                                                              n_cols, modes, n_modes, keys, partials);
-    else if (precision == PB_F32)
-        shell_rows_kernel<float><<<grid, SR_THREADS, 0, s>>>(G, (const float2 *)F, (const float2 *)Q, n_rows, n_cols,
-                                                             modes, n_modes, keys, partials);
-    else
-        return fail(PB_ERR_INVALID, "bad precision");
+    if (precision == PB_F64) PB_SR_ROWS(double)
+    else PB_SR_ROWS(float)
+#undef PB_SR_ROWS
+#undef PB_SR_LAUNCH
     PB_LAUNCH_CHECK("pb_shell_rows");
     int total = n_rows * n_cols;
     shell_rows_finalize<<<(total + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(
