@@ -549,7 +549,7 @@ class BSpec:
 
     def _b3_route(self, xk, w, scale, rd=None):
         b = self.base
-        key = "b3route|%s|%s|%d|%d|%s" % (autotune.device_tag(b.device), ",".join(str(int(n)) for n in self.map_grid),
+        key = "b3route|lines|%s|%s|%d|%d|%s" % (autotune.device_tag(b.device), ",".join(str(int(n)) for n in self.map_grid),
                                           self.Nl * self.Nk_squeeze, self.Nk_squeeze, b.sightline)
         def tiled():
             if self._b3_tiled(xk, w, scale, rd) is None:

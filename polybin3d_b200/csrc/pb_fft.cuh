@@ -192,7 +192,7 @@ template <typename F> __device__ __forceinline__ void with_radix(int R, F &&f) {
 struct Axis {
     int n, np;            // length, passes (1 - 3)
     int R[3], nb[3], ns[3];
-    uint32_t div_ns1;     // ceil(2^20 / R0): j / R0 = j div_ns1 >> 20 for j < 1024
+    uint32_t div_ns1;     // ceil(2^20 / R0): j / R0 = j div_ns1 >> 20 for j < 4096
     int pad;              // 1: rows in shared memory get one element of padding per R0 (R0 even)
     int tw[3];            // offset of pass q's twiddles [r - 1][j mod Ns] in the axis's table
     int tw_len;
@@ -276,7 +276,7 @@ __host__ __device__ constexpr int balanced_radix(int n) {
 __host__ __device__ constexpr Axis make_axis(int n, bool reversed) {
     Axis ax{};
     int r[3] = {n, 0, 0};
-    if (n < 2 || n > 1024) return ax;
+    if (n < 2 || n > 4096) return ax;
     int np = 0;
     if (n <= MAX_RADIX) {
         np = 1;

@@ -34,7 +34,7 @@ static int mr_layout(const Grid &G, MrLayout *L) {
     L->ay = fft::make_axis(G.n1, true);
     L->azi = fft::make_axis(G.n2, false);
     L->azf = fft::make_axis(G.n2, true);
-    if (!L->ax.np || !L->ay.np || !L->azi.np)
+    if (!L->ax.np || !L->ay.np || !L->azi.np || std::max(G.n0, std::max(G.n1, G.n2)) > 1024)
         return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: grid dimensions must be products of 2, 3, 5, 7, 11 and 13 "
                                         "of at most three factors up to 16");
     L->tw_x = 0;

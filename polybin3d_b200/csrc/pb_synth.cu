@@ -4,9 +4,10 @@
 //   out[m](x) = sum_k F_m(k) e^{+2 pi i k.x / M}   (unnormalised, numpy irfftn x M^3 convention)
 //   F_m(k)    = scale_m * src[src_m](k) * w(k)^wpow_m * Theta(lo_m <= |k| < hi_m) L_l1(mu) L_l2(mu)
 //
-// F_m vanishes outside the ball |k| < hi_m, so only the planes kz <= hi_m / kF_z, and in each
-// plane only the columns and rows inside the band limit, carry data.  Three passes of
-// batched 1D transforms (Stockham, mixed radix 2/3/4/5/8, in shared memory):
+// Entry points, and the run-time Stockham form (mixed radix 2/3/4/5/8 in shared memory) for output lengths
+// that pb_synth_lines.cuh has no plan for (above 4096, or with more prime factors than three radices up to 16
+// hold, such as 1250).  F_m vanishes outside the ball |k| < hi_m, so only the planes
+// kz <= hi_m / kF_z, and in each plane only the columns and rows inside the band limit, carry data:
 //   S1  per (map, kz plane, chunk of ky columns): gather + filter the source modes of each
 //       column (kx inside the band), inverse transform along x -> U[m][kz][x][ky]
 //   S2  per (map, kz plane, chunk of x rows): ky inside the band -> inverse transform along
@@ -21,6 +22,7 @@
 #include <vector>
 #include <cuda_bf16.h>
 #include "pb_common.cuh"
+#include "pb_synth_lines.cuh"
 
 namespace pb {
 
@@ -195,178 +197,12 @@ __device__ __forceinline__ void stockham_pass(const typename cplx<T>::type *src,
     }
 }
 
-// Radix plan of a length: 8s first, then 4, 2, 3, 5 (so Ns stays a power of two through the
-// radix-2^k passes).  Shared by the compile-time and the run-time forms.
-__host__ __device__ constexpr int radix_of(int n) {
-    return n % 8 == 0 ? 8 : n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : n % 3 == 0 ? 3 : n % 5 == 0 ? 5 : 0;
-}
-__host__ __device__ constexpr int radix_at(int n, int q) {
-    for (int i = 0; i < q; ++i) n /= radix_of(n);
-    return radix_of(n);
-}
-__host__ __device__ constexpr int pass_count(int n) {
-    int c = 0;
-    while (n > 1) {
-        const int f = radix_of(n);
-        if (f == 0) return -1;
-        n /= f;
-        ++c;
-    }
-    return c;
-}
-
-// Compile-time-length pass: nb, Ns, the twiddle stride and the line stride are constants,
-// so the index arithmetic folds away.
-template <int R, typename T, int N, int NS>
-__device__ __forceinline__ void stockham_pass_ct(const typename cplx<T>::type *src, typename cplx<T>::type *dst,
-                                                 int lines, int lshift, const typename cplx<T>::type *tw) {
-    using C = typename cplx<T>::type;
-    constexpr int nb = N / R;
-    constexpr int tstep = N / (NS * R);
-    constexpr int ld = N + 1;
-    const int line = threadIdx.x & ((1 << lshift) - 1);
-    const int NG = blockDim.x >> lshift;
-    if (line >= lines) return;
-    const C *s = src + line * ld;
-    C *d = dst + line * ld;
-    for (int j = threadIdx.x >> lshift; j < nb; j += NG) {
-        const int jm = j % NS, jq = j / NS;
-        C v[R];
-        v[0] = s[j];
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            C x = s[j + r * nb];
-            if (NS > 1) x = cmul(x, tw[r * jm * tstep]);
-            v[r] = x;
-        }
-        if (R == 2) idft2<T, C>(v[0], v[1]);
-        else if (R == 3) idft3<T, C>(v);
-        else if (R == 4) idft4<T, C>(v[0], v[1], v[2], v[3]);
-        else if (R == 5) idft5<T, C>(v);
-        else idft8<T, C>(v);
-        const int o = jq * (NS * R) + jm;
-#pragma unroll
-        for (int r = 0; r < R; ++r) d[o + r * NS] = v[r];
-    }
-}
-
-template <typename T, int N, int Q, int NS>
-__device__ __forceinline__ void passes_ct(typename cplx<T>::type *&src, typename cplx<T>::type *&dst, int lines,
-                                          int lshift, const typename cplx<T>::type *tw) {
-    if constexpr (Q < pass_count(N)) {
-        constexpr int R = radix_at(N, Q);
-        stockham_pass_ct<R, T, N, NS>(src, dst, lines, lshift, tw);
-        __syncthreads();
-        typename cplx<T>::type *t = src;
-        src = dst;
-        dst = t;
-        passes_ct<T, N, Q + 1, NS * R>(src, dst, lines, lshift, tw);
-    }
-}
-
-__host__ __device__ constexpr int ns_at(int n, int q) {
-    int ns = 1;
-    for (int i = 0; i < q; ++i) ns *= radix_at(n, i);
-    return ns;
-}
-
-// A compile-time pass whose operands come from and go to functors: v[r] = ldf(line, j + r nb)
-// (twiddled), stf(line, o + r Ns, v[r]).  ELEM: threads run j-fastest along a line (for
-// loads or stores that are contiguous along the line in global memory); otherwise
-// line-fastest as in stockham_pass_ct.
-template <int R, typename T, int N, int NS, bool ELEM, typename LD, typename ST>
-__device__ __forceinline__ void io_pass(int lines, int lshift, const typename cplx<T>::type *tw, LD &&ldf,
-                                        ST &&stf) {
-    using C = typename cplx<T>::type;
-    constexpr int nb = N / R;
-    constexpr int tstep = N / (NS * R);
-    auto body = [&](int line, int j) {
-        const int jm = j % NS, jq = j / NS;
-        C v[R];
-        v[0] = ldf(line, j);
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            C x = ldf(line, j + r * nb);
-            if (NS > 1) x = cmul(x, tw[r * jm * tstep]);
-            v[r] = x;
-        }
-        if (R == 2) idft2<T, C>(v[0], v[1]);
-        else if (R == 3) idft3<T, C>(v);
-        else if (R == 4) idft4<T, C>(v[0], v[1], v[2], v[3]);
-        else if (R == 5) idft5<T, C>(v);
-        else idft8<T, C>(v);
-        const int o = jq * (NS * R) + jm;
-#pragma unroll
-        for (int r = 0; r < R; ++r) stf(line, o + r * NS, v[r]);
-    };
-    if (ELEM) {
-        for (int it = threadIdx.x; it < lines * nb; it += blockDim.x) {
-            const int line = it / nb;
-            body(line, it - line * nb);
-        }
-    } else {
-        const int line = threadIdx.x & ((1 << lshift) - 1);
-        if (line >= lines) return;
-        for (int j = threadIdx.x >> lshift; j < nb; j += blockDim.x >> lshift) body(line, j);
-    }
-}
-
-template <typename T, int N, int Q, int QEND>
-__device__ __forceinline__ void smem_passes(typename cplx<T>::type *&src, typename cplx<T>::type *&dst, int lines,
-                                            int lshift, const typename cplx<T>::type *tw) {
-    if constexpr (Q < QEND) {
-        stockham_pass_ct<radix_at(N, Q), T, N, ns_at(N, Q)>(src, dst, lines, lshift, tw);
-        __syncthreads();
-        typename cplx<T>::type *t = src;
-        src = dst;
-        dst = t;
-        smem_passes<T, N, Q + 1, QEND>(src, dst, lines, lshift, tw);
-    }
-}
-
-// Compile-time length, data in b0 (line stride N + 1): every pass but the last in shared
-// memory, the last one straight to stf(line, element, value).
-template <typename T, int N, bool LAST_ELEM, typename ST>
-__device__ __forceinline__ void line_ifft_tail(typename cplx<T>::type *b0, typename cplx<T>::type *b1, int lines,
-                                               int lshift, const typename cplx<T>::type *tw, ST &&stf) {
-    using C = typename cplx<T>::type;
-    constexpr int P = pass_count(N);
-    C *src = b0, *dst = b1;
-    smem_passes<T, N, 0, P - 1>(src, dst, lines, lshift, tw);
-    const C *s = src;
-    io_pass<radix_at(N, P - 1), T, N, ns_at(N, P - 1), LAST_ELEM>(
-        lines, lshift, tw, [&](int line, int e) { return s[line * (N + 1) + e]; }, stf);
-}
-
-// Compile-time length, first pass straight from ldf(line, element) (line-fastest), last pass
-// straight to stf; needs at least two passes.
-template <typename T, int N, bool LAST_ELEM, typename LD, typename ST>
-__device__ __forceinline__ void line_ifft_io(typename cplx<T>::type *b0, typename cplx<T>::type *b1, int lines,
-                                             int lshift, const typename cplx<T>::type *tw, LD &&ldf, ST &&stf) {
-    using C = typename cplx<T>::type;
-    constexpr int P = pass_count(N);
-    static_assert(P >= 2, "line_ifft_io needs two passes");
-    io_pass<radix_at(N, 0), T, N, 1, false>(lines, lshift, tw, ldf,
-                                            [&](int line, int e, C v) { b0[line * (N + 1) + e] = v; });
-    __syncthreads();
-    C *src = b0, *dst = b1;
-    smem_passes<T, N, 1, P - 1>(src, dst, lines, lshift, tw);
-    const C *s = src;
-    io_pass<radix_at(N, P - 1), T, N, ns_at(N, P - 1), LAST_ELEM>(
-        lines, lshift, tw, [&](int line, int e) { return s[line * (N + 1) + e]; }, stf);
-}
-
 // All passes of one axis; data starts in b0, returns the buffer holding the result.
-// N > 0: compile-time length; N == 0: the length and radices of `ax` at run time.
-template <typename T, int N>
+template <typename T>
 __device__ typename cplx<T>::type *line_ifft(typename cplx<T>::type *b0, typename cplx<T>::type *b1, int ld,
                                              int lines, const FftAxis &ax, const typename cplx<T>::type *tw) {
     using C = typename cplx<T>::type;
     C *src = b0, *dst = b1;
-    if constexpr (N > 0) {
-        passes_ct<T, N, 0, 1>(src, dst, lines, ax.lshift, tw);
-        return src;
-    }
     int Ns = 1;
     for (int q = 0; q < ax.np; ++q) {
         const int R = ax.rad[q];
@@ -424,13 +260,13 @@ __device__ __forceinline__ int find_map(const SynthParams &p, int b, int which) 
 // ---- S1: gather + filter + transform along x ------------------------------------------
 // S: the source spectrum's element type, the maps' complex type or (FP32 maps) complex FP64:
 // the filter product is formed in FP64 and rounded to T once
-template <typename T, int N, typename S = typename cplx<T>::type>
+template <typename T, typename S = typename cplx<T>::type>
 __global__ void __launch_bounds__(SY_THREADS) synth_x_kernel(SynthParams p, const S *src, const T *w,
                                                              typename cplx<T>::type *U) {
     using C = typename cplx<T>::type;
     extern __shared__ __align__(16) unsigned char sy_smem[];
     const FftAxis &ax = p.ax;
-    const int n = N > 0 ? N : ax.n, ld = n + 1, L = 1 << ax.lshift;
+    const int n = ax.n, ld = n + 1, L = 1 << ax.lshift;
     C *tw = reinterpret_cast<C *>(sy_smem);
     C *b0 = tw + n;
     C *b1 = b0 + L * ld;
@@ -487,13 +323,8 @@ __global__ void __launch_bounds__(SY_THREADS) synth_x_kernel(SynthParams p, cons
     __syncthreads();
     // U[m][kz][x][c]: consecutive threads take consecutive columns
     C *u = U + mp.u_off + (int64_t)kz * n * mp.wu;
-    if constexpr (N > 0) {
-        line_ifft_tail<T, N, false>(b0, b1, lines, ax.lshift, tw, [&](int line, int x, C v) {
-            const int c = c0 + line;
-            if (c >= col_first) u[(int64_t)x * mp.wu + c] = v;
-        });
-    } else {
-        C *res = line_ifft<T, N>(b0, b1, ld, lines, ax, tw);
+    {
+        C *res = line_ifft<T>(b0, b1, ld, lines, ax, tw);
         const int line = threadIdx.x & (L - 1), NG = blockDim.x >> ax.lshift;
         const int c = c0 + line;
         if (line < lines && c >= col_first)
@@ -503,13 +334,13 @@ __global__ void __launch_bounds__(SY_THREADS) synth_x_kernel(SynthParams p, cons
 }
 
 // ---- S2: transform along y --------------------------------------------------------------
-template <typename T, int N>
+template <typename T>
 __global__ void __launch_bounds__(SY_THREADS) synth_y_kernel(SynthParams p, const typename cplx<T>::type *U,
                                                              typename cplx<T>::type *H) {
     using C = typename cplx<T>::type;
     extern __shared__ __align__(16) unsigned char sy_smem[];
     const FftAxis &ay = p.ay;
-    const int n = N > 0 ? N : ay.n, ld = n + 1, L = 1 << ay.lshift;
+    const int n = ay.n, ld = n + 1, L = 1 << ay.lshift;
     C *tw = reinterpret_cast<C *>(sy_smem);
     C *b0 = tw + n;
     C *b1 = b0 + L * ld;
@@ -545,11 +376,8 @@ __global__ void __launch_bounds__(SY_THREADS) synth_y_kernel(SynthParams p, cons
     }
     __syncthreads();
     C *h = H + mp.h_off + ((int64_t)kz * p.m0 + x0) * p.m1;
-    if constexpr (N > 0) {
-        line_ifft_tail<T, N, true>(b0, b1, lines, ay.lshift, tw,
-                                   [&](int line, int y, C v) { h[(int64_t)line * p.m1 + y] = v; });
-    } else {
-        C *res = line_ifft<T, N>(b0, b1, ld, lines, ay, tw);
+    {
+        C *res = line_ifft<T>(b0, b1, ld, lines, ay, tw);
         for (int line = warp; line < lines; line += nw) {
             const C *row = res + (int64_t)line * ld;
             C *hrow = h + (int64_t)line * p.m1;
@@ -558,71 +386,15 @@ __global__ void __launch_bounds__(SY_THREADS) synth_y_kernel(SynthParams p, cons
     }
 }
 
-// ---- tiled-set output ------------------------------------------------------------------
-// voxel v of map m into a tiled set: FP32 copy of a factor map, bf16 hi and lo parts
-__device__ __forceinline__ void tiled_put(const SynthParams &p, int m, int64_t v, float val, char *out) {
-    if (m < p.t_factor) *reinterpret_cast<float *>(out + tiled_factor_byte(v, m, p.t_maps, p.t_factor)) = val;
-    const __nv_bfloat16 hi = __float2bfloat16_rn(val);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(val - __bfloat162float(hi));
-    *reinterpret_cast<__nv_bfloat16 *>(out + tiled_c_byte(v, m, p.t_maps, p.t_factor)) = hi;
-    *reinterpret_cast<__nv_bfloat16 *>(out + tiled_c_byte(v, tiled_cpad(p.t_maps) + m, p.t_maps, p.t_factor)) = lo;
-}
-
-// Staged values of map m (rows of NN voxels, row stride lds in stg; voxels v0 .. v0 + rows NN
-// - 1) into a tiled set, by warps wk = 0 .. nw - 1 of a group (the caller's warp index in it).
-// Each warp takes 64 consecutive voxels per step, a lane two neighbours: two 128-byte rows of
-// factor slabs (8-byte stores) and four 32-byte K-step rows each of the hi and lo parts
-// (bf16x2 stores), so the stores fill whole sectors; offsets inside a tile are per lane and
-// computed once per map, the tile base per chunk.  Per voxel (tiled_put) when the run is not
-// 64-aligned.
-template <int NN>
-__device__ void flush_tiled(const SynthParams &p, int m, int64_t v0, int rows, int lds, const float *stg, char *out,
-                            int wk, int nw) {
-    const int count = rows * NN;
-    const int lane = threadIdx.x & 31;
-    if ((NN & 1) != 0 || (v0 & 63) != 0 || (count & 63) != 0) {
-        for (int i = wk * 32 + lane; i < count; i += nw * 32) {
-            const int r = i / NN, z = i - r * NN;
-            tiled_put(p, m, v0 + i, stg[r * lds + z], out);
-        }
-        return;
-    }
-    const int F = tiled_frows(p.t_factor), P = tiled_cpad(p.t_maps);
-    const int64_t tb = tiled_tile_bytes(p.t_maps, p.t_factor);
-    const bool factor = m < p.t_factor;
-    // lane j holds voxels 2j, 2j + 1 of the chunk: slab j / 16, 4-voxel chunk (j % 16) / 2 of
-    // it; K step j / 8, 8-voxel half (j / 4) % 2, element 2 (j % 4)
-    const uint32_t off_f = (uint32_t)(lane >> 4) * F * 128u + (uint32_t)m * 128u +
-                           ((((uint32_t)(lane & 15) >> 1) ^ ((uint32_t)m & 7u)) << 4) + (lane & 1) * 8;
-    auto c_off = [&](int r) {
-        return (uint32_t)((lane >> 3) * 64 * P + (r >> 3) * 256 + (r & 7) * 32 +
-                          ((((lane >> 2) & 1) ^ ((r >> 2) & 1)) << 4) + (lane & 3) * 4);
-    };
-    const uint32_t off_hi = c_off(m), off_lo = c_off(P + m);
-    for (int u = wk * 64; u < count; u += nw * 64) {
-        const int i = u + 2 * lane, r = i / NN, z = i - r * NN;  // NN even: both voxels in row r
-        const float x0 = stg[r * lds + z], x1 = stg[r * lds + z + 1];
-        const int64_t v = v0 + u;  // 64-aligned: two slabs, four K steps of one tile
-        const int w = (int)(v & (TILED_VOX - 1));
-        char *const tile = out + (v >> 7) * tb;
-        if (factor) *reinterpret_cast<float2 *>(tile + (w >> 5) * F * 128 + off_f) = make_float2(x0, x1);
-        const __nv_bfloat162 hb = __floats2bfloat162_rn(x0, x1);
-        const __nv_bfloat162 lb = __floats2bfloat162_rn(x0 - __low2float(hb), x1 - __high2float(hb));
-        char *const cop = tile + 512 * F + (w >> 4) * 64 * P;
-        *reinterpret_cast<__nv_bfloat162 *>(cop + off_hi) = hb;
-        *reinterpret_cast<__nv_bfloat162 *>(cop + off_lo) = lb;
-    }
-}
-
 // ---- S3: real transform along z, two output lines per complex transform -----------------
-template <typename T, int N>
+template <typename T>
 // (FP32: two 768-thread blocks resident per SM, 42 registers; FP64 keeps its registers)
 __global__ void __launch_bounds__(SY_THREADS_Z, sizeof(T) == 4 ? 2 : 1) synth_z_kernel(SynthParams p, const typename cplx<T>::type *H,
                                                              T *out) {
     using C = typename cplx<T>::type;
     extern __shared__ __align__(16) unsigned char sy_smem[];
     const FftAxis &az = p.az;
-    const int n = N > 0 ? N : az.n, ld = n + 1, L = 1 << az.lshift;
+    const int n = az.n, ld = n + 1, L = 1 << az.lshift;
     C *tw = reinterpret_cast<C *>(sy_smem);
     C *b0 = tw + n;
     C *b1 = b0 + L * ld;
@@ -643,66 +415,8 @@ __global__ void __launch_bounds__(SY_THREADS_Z, sizeof(T) == 4 ? 2 : 1) synth_z_
     const int tiled = p.tiled;
     auto put = [&](int yy, int z, T val) {
         if (!tiled) o[(int64_t)yy * p.m2 + z] = val;
-        else tiled_put(p, m, v0 + (int64_t)yy * p.m2 + z, (float)val, reinterpret_cast<char *>(out));
+        else tiled_put(p.t_maps, p.t_factor, m, v0 + (int64_t)yy * p.m2 + z, (float)val, reinterpret_cast<char *>(out));
     };
-    if constexpr (N > 0 && pass_count(N) >= 2) {
-        // a tiled set's rows (2 L lines of n values) are staged in the transform buffer the last
-        // pass does not read (b1 after an even number of shared-memory passes, else b0) and
-        // written out together
-        float *const stg = reinterpret_cast<float *>((pass_count(N) - 2) % 2 == 0 ? b1 : b0);
-        constexpr int LDS = N + 1;  // odd row stride: the last pass's lanes write different rows
-        // first pass straight from H (a warp reads the (y, y+1) pairs of 32 lines at one kz:
-        // 512 contiguous bytes; it needs no twiddles), last pass straight to the real rows
-        const C *hb = H + mp.h_off + (int64_t)x * p.m1 + y0;
-        line_ifft_io<T, N, true>(
-            b0, b1, lines, az.lshift, tw,
-            [&](int line, int e) -> C {
-                int kz;
-                bool mirror = false;
-                if (e <= K) {
-                    kz = e;
-                } else if (e >= N - K) {
-                    kz = N - e;
-                    mirror = true;
-                } else {
-                    return cmake<T>(0.0, 0.0);
-                }
-                const C *hl = hb + 2 * line + kz * plane;
-                C a, b;
-                if constexpr (std::is_same<T, float>::value) {
-                    const float4 q = *reinterpret_cast<const float4 *>(hl);
-                    a = make_float2(q.x, q.y);
-                    b = make_float2(q.z, q.w);
-                } else {
-                    a = hl[0];
-                    b = hl[1];
-                }
-                if (kz == 0) return cmake<T>((double)a.x, (double)b.x);
-                C r;
-                if (!mirror) {
-                    r.x = a.x - b.y;
-                    r.y = a.y + b.x;
-                } else {
-                    r.x = a.x + b.y;
-                    r.y = b.x - a.y;
-                }
-                return r;
-            },
-            [&](int line, int z, C v) {
-                if (tiled) {
-                    stg[(2 * line) * LDS + z] = (float)v.x;
-                    stg[(2 * line + 1) * LDS + z] = (float)v.y;
-                } else {
-                    put(2 * line, z, v.x);
-                    put(2 * line + 1, z, v.y);
-                }
-            });
-        if (tiled) {
-            __syncthreads();
-            flush_tiled<N>(p, m, v0, ny, LDS, stg, reinterpret_cast<char *>(out), threadIdx.x >> 5, blockDim.x >> 5);
-        }
-        return;
-    }
     // line-fastest: consecutive threads read consecutive (y, y+1) pairs of one kz row
     const int line = threadIdx.x & (L - 1), NG = blockDim.x >> az.lshift;
     if (line < lines) {
@@ -738,7 +452,7 @@ __global__ void __launch_bounds__(SY_THREADS_Z, sizeof(T) == 4 ? 2 : 1) synth_z_
         }
     }
     __syncthreads();
-    C *res = line_ifft<T, N>(b0, b1, ld, lines, az, tw);
+    C *res = line_ifft<T>(b0, b1, ld, lines, az, tw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int yy = warp; yy < ny; yy += nw) {
         const C *row = res + (int64_t)(yy >> 1) * ld;
@@ -747,66 +461,6 @@ __global__ void __launch_bounds__(SY_THREADS_Z, sizeof(T) == 4 ? 2 : 1) synth_z_
         else
             for (int z = lane; z < n; z += 32) put(yy, z, row[z].x);
     }
-}
-
-// ---- S3 for a tiled set: a block per (x, 2 LY y-lines, group of SY_TMAPS maps) --------------
-// Its L = SY_TMAPS LY complex lines are (map, y pair) combinations (line l: map g0 SY_TMAPS +
-// l / LY, y pair l % LY), so the block writes neighbouring maps' rows of the same tiles -- one
-// 8-row atom of each factor slab and K step -- together instead of one map's row in many tiles.
-constexpr int SY_TMAPS = 8;  // a power of two (line -> map by shift)
-
-template <int N>
-__global__ void __launch_bounds__(SY_THREADS_Z, 2) synth_z_tiled_kernel(SynthParams p, const float2 *H, char *out) {
-    extern __shared__ __align__(16) unsigned char sy_smem[];
-    const FftAxis &az = p.az;
-    const int L = 1 << az.lshift, LY = L / SY_TMAPS, ly_shift = az.lshift - 3;  // SY_TMAPS = 8
-    float2 *tw = reinterpret_cast<float2 *>(sy_smem);
-    float2 *b0 = tw + N;
-    float2 *b1 = b0 + L * (N + 1);
-    const int ychunks = (p.m1 + 2 * LY - 1) / (2 * LY), mgroups = (p.n_maps + SY_TMAPS - 1) / SY_TMAPS;
-    int b = blockIdx.x;
-    const int g0 = b % mgroups;
-    b /= mgroups;
-    const int yc = b % ychunks, x = b / ychunks;
-    const int y0 = yc * 2 * LY, ny = min(2 * LY, p.m1 - y0);
-    const int nm = min(SY_TMAPS, p.n_maps - SY_TMAPS * g0);
-    make_twiddles<float>(tw, N);  // made visible by the barrier after the first pass
-    const int64_t plane = (int64_t)p.m0 * p.m1;
-    float *const stg = reinterpret_cast<float *>((pass_count(N) - 2) % 2 == 0 ? b1 : b0);
-    constexpr int LDS = N + 1;
-    line_ifft_io<float, N, true>(
-        b0, b1, nm * LY, az.lshift, tw,
-        [&](int line, int e) -> float2 {
-            const int mi = line >> ly_shift, y = y0 + 2 * (line & (LY - 1));
-            const SynthMap &mp = p.maps[SY_TMAPS * g0 + mi];
-            const int K = mp.kz_max;
-            int kz;
-            bool mirror = false;
-            if (y >= p.m1) return make_float2(0.f, 0.f);
-            if (e <= K) {
-                kz = e;
-            } else if (e >= N - K) {
-                kz = N - e;
-                mirror = true;
-            } else {
-                return make_float2(0.f, 0.f);
-            }
-            // the (y, y + 1) pair of line: one 16-byte load (m1 even)
-            const float4 q = *reinterpret_cast<const float4 *>(H + mp.h_off + kz * plane + (int64_t)x * p.m1 + y);
-            const float2 a = make_float2(q.x, q.y), c = make_float2(q.z, q.w);
-            if (kz == 0) return make_float2(a.x, c.x);
-            return mirror ? make_float2(a.x + c.y, c.x - a.y) : make_float2(a.x - c.y, a.y + c.x);
-        },
-        [&](int line, int z, float2 v) {
-            stg[(2 * line) * LDS + z] = v.x;
-            stg[(2 * line + 1) * LDS + z] = v.y;
-        });
-    __syncthreads();
-    const int64_t v0 = ((int64_t)x * p.m1 + y0) * p.m2;
-    // a group of warps per map, so each warp sets up one map's offsets and stores many chunks
-    const int nwb = blockDim.x >> 5, wpm = max(1, nwb / nm), warp = threadIdx.x >> 5;
-    for (int mi = warp / wpm; mi < nm; mi += max(1, nwb / wpm))
-        flush_tiled<N>(p, SY_TMAPS * g0 + mi, v0, ny, LDS, stg + 2 * mi * LY * LDS, out, warp % wpm, wpm);
 }
 
 // ---- host side ----------------------------------------------------------------------------
@@ -942,24 +596,6 @@ static cudaError_t set_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Lengths with a compile-time kernel; any other supported length runs the run-time form.
-template <typename F>
-static void with_length(int n, F &&f) {
-    switch (n) {
-        case 24: f(std::integral_constant<int, 24>()); break;
-        case 32: f(std::integral_constant<int, 32>()); break;
-        case 48: f(std::integral_constant<int, 48>()); break;
-        case 64: f(std::integral_constant<int, 64>()); break;
-        case 96: f(std::integral_constant<int, 96>()); break;
-        case 128: f(std::integral_constant<int, 128>()); break;
-        case 192: f(std::integral_constant<int, 192>()); break;
-        case 256: f(std::integral_constant<int, 256>()); break;
-        case 384: f(std::integral_constant<int, 384>()); break;
-        case 512: f(std::integral_constant<int, 512>()); break;
-        default: f(std::integral_constant<int, 0>()); break;
-    }
-}
-
 template <typename T, typename S = typename cplx<T>::type>
 static int launch_synth(const SynthLayout &L, const S *src, const T *w, typename cplx<T>::type *U,
                         typename cplx<T>::type *H, T *out, cudaStream_t s) {
@@ -967,53 +603,102 @@ static int launch_synth(const SynthLayout &L, const S *src, const T *w, typename
     const size_t c = sizeof(typename cplx<T>::type);
     auto smem = [&](const FftAxis &a) { return (size_t)(2 * (1 << a.lshift) * (a.n + 1) + a.n) * c; };
     const size_t smem_z = smem(p.az);
-    cudaError_t e = cudaSuccess;
-    with_length(p.ax.n, [&](auto NC) {
-        constexpr int N = decltype(NC)::value;
-        if (e == cudaSuccess)
-            e = set_smem(synth_x_kernel<T, N, S>, smem(p.ax));
-        if (e == cudaSuccess) {
-            synth_x_kernel<T, N, S><<<L.nb1, SY_THREADS, smem(p.ax), s>>>(p, src, w, U);
-            e = cudaGetLastError();
-        }
-    });
+    cudaError_t e = set_smem(synth_x_kernel<T, S>, smem(p.ax));
+    if (e == cudaSuccess) {
+        synth_x_kernel<T, S><<<L.nb1, SY_THREADS, smem(p.ax), s>>>(p, src, w, U);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return cuda_check(e, "pb_shell_synth (x)");
-    with_length(p.ay.n, [&](auto NC) {
-        constexpr int N = decltype(NC)::value;
-        if (e == cudaSuccess)
-            e = set_smem(synth_y_kernel<T, N>, smem(p.ay));
-        if (e == cudaSuccess) {
-            synth_y_kernel<T, N><<<L.nb2, SY_THREADS, smem(p.ay), s>>>(p, U, H);
-            e = cudaGetLastError();
-        }
-    });
+    e = set_smem(synth_y_kernel<T>, smem(p.ay));
+    if (e == cudaSuccess) {
+        synth_y_kernel<T><<<L.nb2, SY_THREADS, smem(p.ay), s>>>(p, U, H);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return cuda_check(e, "pb_shell_synth (y)");
-    with_length(p.az.n, [&](auto NC) {
-        constexpr int N = decltype(NC)::value;
-        if constexpr (std::is_same<T, float>::value && N > 0 && pass_count(N) >= 2) {
-            // a tiled set: blocks over groups of maps (rows of neighbouring maps written together)
-            const int Lz = 1 << p.az.lshift;
-            if (p.tiled && p.m1 % 2 == 0 && Lz >= SY_TMAPS) {
-                const int LY = Lz / SY_TMAPS;
-                const int64_t nb = (int64_t)p.m0 * ((p.m1 + 2 * LY - 1) / (2 * LY)) *
-                                   ((p.n_maps + SY_TMAPS - 1) / SY_TMAPS);
-                if (e == cudaSuccess)
-                    e = set_smem(synth_z_tiled_kernel<N>, smem_z);
-                if (e == cudaSuccess) {
-                    synth_z_tiled_kernel<N><<<(unsigned)nb, SY_THREADS_Z, smem_z, s>>>(p, H, reinterpret_cast<char *>(out));
-                    e = cudaGetLastError();
-                }
-                return;
-            }
-        }
-        if (e == cudaSuccess)
-            e = set_smem(synth_z_kernel<T, N>, smem_z);
-        if (e == cudaSuccess) {
-            synth_z_kernel<T, N><<<L.nb3, SY_THREADS_Z, smem_z, s>>>(p, H, out);
-            e = cudaGetLastError();
-        }
-    });
+    e = set_smem(synth_z_kernel<T>, smem_z);
+    if (e == cudaSuccess) {
+        synth_z_kernel<T><<<L.nb3, SY_THREADS_Z, smem_z, s>>>(p, H, out);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return cuda_check(e, "pb_shell_synth (z)");
+    return PB_OK;
+}
+
+// ---- the passes of pb_synth_lines.cuh ----------------------------------------------
+// Fills their parameters from a checked layout; false when an axis has no plan there (the kernels above
+// then make the maps).  bytes: workspace, twiddle table first.
+static bool sl_setup(const Grid &G, const SynthLayout &L, size_t csize, SlParams *q, size_t *bytes) {
+    const SynthParams &p = L.p;
+    memset(q, 0, sizeof(*q));
+    q->ax = fft::make_axis(p.m0, true);
+    q->ay = fft::make_axis(p.m1, true);
+    q->az = fft::make_axis(p.m2, true);
+    if (!q->ax.np || !q->ay.np || !q->az.np) return false;
+    // (longest lines: their exchange buffers must fit a block's shared memory)
+    const bool f64 = csize == 16;
+    const size_t most = std::max(std::max(f64 ? sl_line_bytes<double>(q->ax, sl_lines<double>(q->ax)) : sl_line_bytes<float>(q->ax, sl_lines<float>(q->ax)),
+                                          f64 ? sl_line_bytes<double>(q->ay, sl_lines<double>(q->ay)) : sl_line_bytes<float>(q->ay, sl_lines<float>(q->ay))),
+                                 std::max(f64 ? sl_z_bytes<double>(q->az, sl_z_pairs<double>(q->az)) : sl_z_bytes<float>(q->az, sl_z_pairs<float>(q->az)),
+                                          p.tiled ? sl_tile_bytes(q->az, sl_tile_pairs(q->az)) : (size_t)0));
+    if (most > (size_t)220 * 1024) return false;
+    q->g = G;
+    q->m0 = p.m0;
+    q->m1 = p.m1;
+    q->m2 = p.m2;
+    q->src_stride = p.src_stride;
+    q->tab_y = 0;
+    q->tab_z = q->ay.tw_len;
+    const int line = (int)(128 / csize);  // elements per 128 bytes
+    int64_t off = 0;
+    for (int m = 0; m < p.n_maps; ++m) {
+        const SynthMap &a = p.maps[m];
+        SlMap &b = q->maps[m];
+        auto threshold = [](double e) {  // smallest t with sqrt(t) >= e
+            if (!(e > 0.0)) return 0.0;
+            double t = e * e;
+            while (t > 0.0 && std::sqrt(t) >= e) t = std::nextafter(t, 0.0);
+            while (std::sqrt(t) < e) t = std::nextafter(t, HUGE_VAL);
+            return t;
+        };
+        b.lo = threshold(a.lo);
+        b.hi = threshold(a.hi);
+        b.lo2 = a.lo > 0.0 ? a.lo * a.lo : 0.0;
+        b.hi2 = a.hi * a.hi * (1.0 + 1e-12);
+        b.scale = a.scale;
+        b.src = a.src;
+        b.l1 = (int8_t)a.l1;
+        b.l2 = (int8_t)a.l2;
+        b.wpow = (int8_t)a.wpow;
+        b.kz_max = (int)std::floor(a.hi / p.kf2 * (1.0 + 1e-12));
+        b.ldz = (b.kz_max + line) / line * line;
+        b.w_off = off;
+        off += (int64_t)p.m0 * p.m1 * b.ldz;
+        q->kz_top = std::max(q->kz_top, (int)b.kz_max);
+    }
+    const size_t table = ((size_t)(q->ay.tw_len + q->az.tw_len) * csize + 255) / 256 * 256;
+    *bytes = table + (size_t)off * csize + 256;
+    return true;
+}
+
+static int sl_run(SlTypes ty, const SlParams &q, int n_maps, size_t csize, const void *src, const void *w, void *out,
+                  char *ws, cudaStream_t s) {
+    SlArgs a{};
+    a.src = src;
+    a.w = w;
+    a.out = out;
+    a.n_maps = n_maps;
+    a.table = ws;
+    a.W = ws + ((size_t)(q.ay.tw_len + q.az.tw_len) * csize + 255) / 256 * 256;
+    const int len[3] = {q.m0, q.m1, q.m2};
+    const SlStage stage[3] = {SL_X, SL_Y, q.t_maps ? SL_Z_TILED : SL_Z};
+    static const char *const where[3] = {"pb_shell_synth (x)", "pb_shell_synth (y)", "pb_shell_synth (z)"};
+    for (int i = 0; i < 3; ++i) {
+        cudaError_t e = cudaSuccess;
+        if (!sl_group_0(len[i], ty, stage[i], q, a, s, &e) && !sl_group_1(len[i], ty, stage[i], q, a, s, &e) &&
+            !sl_group_2(len[i], ty, stage[i], q, a, s, &e) && !sl_group_3(len[i], ty, stage[i], q, a, s, &e))
+            e = sl_dispatch<0>(ty, stage[i], q, a, s);
+        if (e != cudaSuccess) return cuda_check(e, where[i]);
+    }
     return PB_OK;
 }
 
@@ -1034,7 +719,14 @@ extern "C" int pb_shell_synth_workspace_size(const pb_grid_t *g, const int32_t *
                           nullptr, 0, &L);
     if (st) return st;
     const size_t c = precision == PB_F64 ? 16 : 8;
+    // the plain and the tiled form share the size
     *bytes = (size_t)(L.u_elems + L.h_elems) * c + 256;
+    Grid G;
+    st = make_grid(g, &G);
+    if (st) return st;
+    SlParams q;
+    size_t need;
+    if (sl_setup(G, L, c, &q, &need)) *bytes = std::max(*bytes, need);
     return PB_OK;
 }
 
@@ -1069,9 +761,22 @@ static int shell_synth(const pb_grid_t *g, const int32_t *out_n, int precision, 
     for (int m = 0; m < n_maps; ++m)
         if (L.p.maps[m].wpow != 0 && !w) return fail(PB_ERR_INVALID, "pb_shell_synth: wpow set but weight grid is NULL");
     const size_t c = precision == PB_F64 ? 16 : 8;
-    const size_t need = (size_t)(L.u_elems + L.h_elems) * c + 256;
-    if (!workspace || workspace_bytes < need) return fail(PB_ERR_INVALID, "pb_shell_synth: workspace too small");
+    size_t need = (size_t)(L.u_elems + L.h_elems) * c + 256;
     char *ws = (char *)(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
+    {
+        Grid G;
+        st = make_grid(g, &G);
+        if (st) return st;
+        SlParams q;
+        size_t lines;
+        if (sl_setup(G, L, c, &q, &lines)) {
+            if (!workspace || workspace_bytes < lines) return fail(PB_ERR_INVALID, "pb_shell_synth: workspace too small");
+            q.t_maps = tiled ? n_maps : 0;
+            q.t_factor = n_factor;
+            return sl_run(src64 ? SL_F32_SRC64 : precision == PB_F64 ? SL_F64 : SL_F32, q, n_maps, c, src, w, out, ws, s);
+        }
+    }
+    if (!workspace || workspace_bytes < need) return fail(PB_ERR_INVALID, "pb_shell_synth: workspace too small");
     if (src64) {
         float2 *U = (float2 *)ws;
         st = launch_synth<float, double2>(L, (const double2 *)src, (const float *)w, U, U + L.u_elems, (float *)out, s);

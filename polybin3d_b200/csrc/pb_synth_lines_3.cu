@@ -1,0 +1,6 @@
+// The synthesis passes for the lengths of SL_GROUP_3.
+#include "pb_synth_lines.cuh"
+
+namespace pb {
+SL_DEFINE_GROUP(3)
+}  // namespace pb
