@@ -193,23 +193,34 @@ struct Axis {
     int n, np;            // length, passes (1 - 3)
     int R[3], nb[3], ns[3];
     uint32_t div_ns1;     // ceil(2^20 / R0): j / R0 = j div_ns1 >> 20 for j < 4096
-    int pad;              // 1: rows in shared memory get one element of padding per R0 (R0 even)
+    int pad;              // rows in shared memory get one element of padding per 2^pad (0: none, R0 odd)
     int tw[3];            // offset of pass q's twiddles [r - 1][j mod Ns] in the axis's table
     int tw_len;
 };
 
 __device__ __forceinline__ int div_r0(const Axis &ax, int e) { return (int)(((uint32_t)e * ax.div_ns1) >> 20); }
-// element e of a padded row
-__device__ __forceinline__ int row_at(const Axis &ax, int e) { return ax.pad ? e + div_r0(ax, e) : e; }
-__host__ __device__ __forceinline__ int row_len(const Axis &ax) { return ax.pad ? ax.n + ax.n / ax.R[0] : ax.n; }
+// element e of a padded row: a first pass writes runs of R0 from neighbouring lanes, which the padding
+// puts on distinct banks
+__device__ __forceinline__ int row_at(const Axis &ax, int e) { return ax.pad ? e + (e >> ax.pad) : e; }
+__host__ __device__ __forceinline__ constexpr int row_len(const Axis &ax) {
+    return ax.pad ? ax.n + ((ax.n - 1) >> ax.pad) : ax.n;
+}
+
+// Half of the line that element e = j + r n / R lies in, known from r when R is even: -1 below n / 2, 1 from
+// n / 2 on, 0 not known.  The functors of the outer passes get it with the element, so that the frequency's
+// sign costs nothing where the compiler knows r.
+__device__ __forceinline__ int abs_label(int e, int n, int side) {  // |frequency| of element e
+    if (side == 0) return e < (n >> 1) ? e : n - e;
+    return side < 0 ? e : n - e;
+}
 
 // functor of line_pass that leaves the loaded elements as they are
 struct Keep {
     template <typename C> __device__ __forceinline__ C operator()(int, C v) const { return v; }
 };
 
-// One pass (number Q) of the lines of a block.  ld(e) gives element e, fix(e, v) finishes it once all of
-// a butterfly's loads are on their way, st(e, v) takes a result; `t` of `nt` threads share the line.
+// One pass (number Q) of the lines of a block.  ld(e, side) gives element e, fix(e, v) finishes it once all of
+// a butterfly's loads are on their way, st(e, v, side) takes a result; `t` of `nt` threads share the line.
 template <typename T, int SIGN, int Q, typename LD, typename ST, typename FX = Keep>
 __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const typename cplx<T>::type *tw, LD &&ld,
                                           ST &&st, FX &&fix = FX()) {
@@ -222,7 +233,7 @@ __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const t
             const int jm = Q == 0 ? 0 : j - jq * ns;
             C v[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = ld(j + r * nb);
+            for (int r = 0; r < R; ++r) v[r] = ld(j + r * nb, R % 2 ? 0 : (2 * r >= R ? 1 : -1));
 #pragma unroll
             for (int r = 0; r < R; ++r) v[r] = fix(j + r * nb, v[r]);
             if (Q > 0) {
@@ -233,7 +244,8 @@ __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const t
             Dft<R, SIGN, T, C>::run(v);
             const int o = jq * ns * R + jm;
 #pragma unroll
-            for (int r = 0; r < R; ++r) st(o + r * ns, v[r]);
+            for (int r = 0; r < R; ++r)
+                st(o + r * ns, v[r], R % 2 || Q != ax.np - 1 ? 0 : (2 * r >= R ? 1 : -1));
         }
     });
 }
@@ -250,16 +262,16 @@ __device__ __forceinline__ void line_fft(const Axis &ax, int t, int nt, bool on,
         if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, st, fix);
         return;
     }
-    if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, [&](int e, C v) { sm[at(e)] = v; }, fix);
+    if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, [&](int e, C v, int) { sm[at(e)] = v; }, fix);
     __syncthreads();
     if (ax.np == 2) {
-        if (on) line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e) { return sm[at(e)]; }, st);
+        if (on) line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, st);
         return;
     }
     if (on)
-        line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e) { return sm[at(e)]; }, [&](int e, C v) { sm2[at(e)] = v; });
+        line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, [&](int e, C v, int) { sm2[at(e)] = v; });
     __syncthreads();
-    if (on) line_pass<T, SIGN, 2>(ax, t, nt, tw, [&](int e) { return sm2[at(e)]; }, st);
+    if (on) line_pass<T, SIGN, 2>(ax, t, nt, tw, [&](int e, int) { return sm2[at(e)]; }, st);
 }
 
 // ---- planning -----------------------------------------------------------------------
@@ -314,7 +326,7 @@ __host__ __device__ constexpr Axis make_axis(int n, bool reversed) {
         ns *= r[q];
     }
     ax.div_ns1 = ((1u << 20) + (uint32_t)r[0] - 1) / (uint32_t)r[0];
-    ax.pad = (r[0] % 2 == 0) ? 1 : 0;
+    ax.pad = r[0] % 2 ? 0 : r[0] <= 2 ? 1 : r[0] <= 4 ? 2 : r[0] <= 8 ? 3 : 4;
     return ax;
 }
 

@@ -117,10 +117,10 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_x_kernel(const __grid_c
     double2 *w = W + blockIdx.y * p.w_map + (int64_t)iy * p.ldz + kz;
     fft::line_fft<double, 1>(
         ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
-        [&](int e) {
+        [&](int e, int side) {
             double2 v = make_double2(0.0, 0.0);
-            const int kx = freq_index(e, ax.n);
-            if (abs(kx) > r_out || abs(kx) < r_in) return v;
+            const int kx = fft::abs_label(e, ax.n, side);
+            if (kx > r_out || kx < r_in) return v;
             const double kxv = __dmul_rn((double)kx, g.kf0);
             const double s = __dadd_rn(__dadd_rn(__dmul_rn(kxv, kxv), ky2), kz2);
             for (int q = 0; q < p.n_legs; ++q) {
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_x_kernel(const __grid_c
             }
             return v;
         },
-        [&](int x, double2 v) { elem(w, x, wx) = v; });
+        [&](int x, double2 v, int) { elem(w, x, wx) = v; });
 }
 
 // ---- Y: inverse (SIGN 1) and forward (SIGN -1) transforms along y, in place ---------------
@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_y_kernel(const __grid_c
     if (SIGN > 0) {
         fft::line_fft<double, 1>(
             ay, threadIdx.y, NT, on, sm, sm2, tw, at,
-            [&](int e) { return abs(freq_index(e, ay.n)) <= ry ? elem(w, e, row) : zero; },
-            [&](int y, double2 v) {
+            [&](int e, int side) { return fft::abs_label(e, ay.n, side) <= ry ? elem(w, e, row) : zero; },
+            [&](int y, double2 v, int) {
                 if (real) v.y = 0.0;
                 if (act[y >> 1]) elem(w, y, row) = v;
             });
@@ -186,9 +186,9 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_y_kernel(const __grid_c
         const unsigned lanes = __ballot_sync(0xffffffffu, on);
         fft::line_fft<double, -1>(
             ay, threadIdx.y, NT, on, sm, sm2, tw, at,
-            [&](int y) { return act[y >> 1] ? elem(w, y, row) : zero; },
-            [&](int e, double2 v) {
-                if (abs(freq_index(e, ay.n)) <= ry) elem(w, e, row) = v;
+            [&](int y, int) { return act[y >> 1] ? elem(w, y, row) : zero; },
+            [&](int e, double2 v, int side) {
+                if (fft::abs_label(e, ay.n, side) <= ry) elem(w, e, row) = v;
             },
             [&](int y, double2 v) {
                 double2 o;
@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     const double *ma = mask + (int64_t)ra * g.n2, *mb = mask + (int64_t)(rb >= 0 ? rb : 0) * g.n2;
     const int K = mp.kz_max;
     // element e of the packed line a + i b (Y left the planes kz = 0 and n / 2 real)
-    auto ldf = [&](int e) {
-        const bool up = 2 * e > n;
+    auto ldf = [&](int e, int side) {
+        const bool up = side ? side > 0 : 2 * e > n;
         const int kz = up ? n - e : e;
         double2 v = make_double2(0.0, 0.0);
         if (kz > K) return v;
@@ -240,10 +240,10 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
         return up ? make_double2(a.x + b.y, b.x - a.y) : make_double2(a.x - b.y, a.y + b.x);
     };
     // F[e] of the forward transform: the rows hold F[kz] and i conj(F[n - kz])
-    auto stf = [&](int e, double2 v) {
+    auto stf = [&](int e, double2 v, int side) {
         if (e <= p.kz_out) wa[e] = v;
         if (rb >= 0) {
-            const int kz = e == 0 ? 0 : n - e;
+            const int kz = side < 0 && e > 0 ? n : e == 0 ? 0 : n - e;  // (the lower half has only kz = 0)
             if (kz <= p.kz_out) wb[kz] = make_double2(v.y, v.x);
         }
     };
@@ -251,13 +251,13 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     auto atf = [&](int e) { return fft::row_at(af, e); };
     double2 *in = sm;
     if (ai.np >= 2) {
-        if (on) fft::line_pass<double, 1, 0>(ai, t, nt, twi, ldf, [&](int e, double2 v) { sm[ati(e)] = v; });
+        if (on) fft::line_pass<double, 1, 0>(ai, t, nt, twi, ldf, [&](int e, double2 v, int) { sm[ati(e)] = v; });
         __syncthreads();
     }
     if (ai.np == 3) {
         if (on)
-            fft::line_pass<double, 1, 1>(ai, t, nt, twi, [&](int e) { return sm[ati(e)]; },
-                                         [&](int e, double2 v) { sm2[ati(e)] = v; });
+            fft::line_pass<double, 1, 1>(ai, t, nt, twi, [&](int e, int) { return sm[ati(e)]; },
+                                         [&](int e, double2 v, int) { sm2[ati(e)] = v; });
         __syncthreads();
         in = sm2;
     }
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
         if (act) {
             if (q == 0) {
 #pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = ldf(t + r * nb);
+                for (int r = 0; r < R; ++r) v[r] = ldf(t + r * nb, 0);
             } else {
 #pragma unroll
                 for (int r = 0; r < R; ++r) v[r] = in[ati(t + r * nb)];
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
         if (act) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                if (af.np == 1) stf(t + r, v[r]);
+                if (af.np == 1) stf(t + r, v[r], 0);
                 else sm[atf(t * R + r)] = v[r];
             }
         }
@@ -299,14 +299,14 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     if (af.np == 1) return;
     __syncthreads();
     if (af.np == 2) {
-        if (on) fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e) { return sm[atf(e)]; }, stf);
+        if (on) fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e, int) { return sm[atf(e)]; }, stf);
         return;
     }
     if (on)
-        fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e) { return sm[atf(e)]; },
-                                      [&](int e, double2 v) { sm2[atf(e)] = v; });
+        fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e, int) { return sm[atf(e)]; },
+                                      [&](int e, double2 v, int) { sm2[atf(e)] = v; });
     __syncthreads();
-    if (on) fft::line_pass<double, -1, 2>(af, t, nt, twf, [&](int e) { return sm2[atf(e)]; }, stf);
+    if (on) fft::line_pass<double, -1, 2>(af, t, nt, twf, [&](int e, int) { return sm2[atf(e)]; }, stf);
 }
 
 // ---- products: forward transform along z of X_i X_j - Z_i Z_j, two rows per complex line ----------
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
     double2 *wa = W + blockIdx.x * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
     fft::line_fft<double, -1>(
         ax, threadIdx.x, N ? ax.nb[0] : (int)blockDim.x, on, sm, sm2, tw, [&](int e) { return fft::row_at(ax, e); },
-        [&](int e) {
+        [&](int e, int) {
             double2 v = make_double2(xi[e] * xj[e], 0.0);
             if (Z) v.x -= zi[e] * zj[e];
             if (two) {
@@ -349,9 +349,9 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
             v.y *= h;
             return v;
         },
-        [&](int e, double2 v) {
+        [&](int e, double2 v, int side) {
             if (e <= p.kz_out) wa[e] = v;
-            const int kz = e == 0 ? 0 : n - e;
+            const int kz = side < 0 && e > 0 ? n : e == 0 ? 0 : n - e;
             if (two && kz <= p.kz_out) wb[kz] = make_double2(v.y, v.x);
         });
 }
@@ -378,9 +378,9 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_out_kernel(const __grid
     const int rx = index_radius(p.out2, (ky * g.kf1) * (ky * g.kf1) + (kz * g.kf2) * (kz * g.kf2), g.kf0);
     fft::line_fft<double, -1>(
         ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
-        [&](int x) { return !x_on || x_on[x] ? elem(w, x, wx) : make_double2(0.0, 0.0); },
-        [&](int e, double2 v) {
-            if (abs(freq_index(e, ax.n)) <= rx) elem(o, e, ox) = v;
+        [&](int x, int) { return !x_on || x_on[x] ? elem(w, x, wx) : make_double2(0.0, 0.0); },
+        [&](int e, double2 v, int side) {
+            if (fft::abs_label(e, ax.n, side) <= rx) elem(o, e, ox) = v;
         });
 }
 

@@ -40,7 +40,7 @@ struct SlParams {
 template <typename T> struct SlShape;
 // lines of 16 (FP64) or 32 (FP32) kz: 256 bytes
 template <> struct SlShape<double> { static constexpr int LINES = 16, THREADS = 128, BLOCKS = 5, ZBLOCKS = 4; };
-template <> struct SlShape<float> { static constexpr int LINES = 32, THREADS = 256, BLOCKS = 3, ZBLOCKS = 6; };
+template <> struct SlShape<float> { static constexpr int LINES = 32, THREADS = 256, BLOCKS = 3, ZBLOCKS = 8; };
 constexpr int SL_SMEM = 100 * 1024;
 
 template <typename T> __host__ __device__ constexpr size_t sl_line_bytes(const fft::Axis &ax, int L) {
@@ -56,10 +56,11 @@ template <typename T> __host__ __device__ constexpr int sl_threads(const fft::Ax
     const int most = SlShape<T>::THREADS / sl_lines<T>(ax), rounds = (ax.nb[0] + most - 1) / most;
     return (ax.nb[0] + rounds - 1) / rounds;
 }
-// threads per line of the z pass: the count up to 16 with the fewest idle butterfly slots (larger on a tie)
+// threads per line of the z pass: eight for two passes (16 for 192 took 386 against 348 us for 32 FP32 maps: a
+// quarter of them idle in the first pass), the count up to 32 with the fewest idle butterfly slots for three
 __host__ __device__ constexpr int sl_z_threads(const fft::Axis &ax) {
     int best = 1, cost = 1 << 30;
-    for (int t = ax.np == 1 ? 1 : 8; t <= (ax.np == 3 ? 32 : 16); ++t) {
+    for (int t = ax.np == 1 ? 1 : 8; t <= (ax.np == 3 ? 32 : 8); ++t) {
         int c = 0;
         for (int q = 0; q < ax.np; ++q) c += (ax.nb[q] + t - 1) / t * t * ax.R[q];
         if (c <= cost) {
@@ -146,11 +147,12 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
     C *o = W + mp.w_off + (int64_t)iy * mp.ldz + kz;
     fft::line_fft<T, 1>(
         ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
-        [&](int e) {
+        [&](int e, int side) {
             C v;
             v.x = v.y = (T)0;
-            const int kx = freq_index(e, ax.n);
-            if (abs(kx) > r_out || abs(kx) < r_in) return v;
+            const int ka = fft::abs_label(e, ax.n, side);
+            if (ka > r_out || ka < r_in) return v;
+            const int kx = (side ? side > 0 : e >= (ax.n >> 1)) ? -ka : ka;
             const double kxv = __dmul_rn((double)kx, g.kf0);
             const double s = __dadd_rn(__dadd_rn(__dmul_rn(kxv, kxv), ky2), kz2);
             if (!(mp.lo <= s && s < mp.hi)) return v;
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
             }
             return v;
         },
-        [&](int x, C v) { sl_elem(o, x, wx) = v; });
+        [&](int x, C v, int) { sl_elem(o, x, wx) = v; });
 }
 
 // ---- Y: inverse transform along y, in place ----------------------------------------------
@@ -199,13 +201,13 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
     C *w = W + mp.w_off + (int64_t)x * p.m1 * mp.ldz + kz;
     fft::line_fft<T, 1>(
         ay, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
-        [&](int e) {
+        [&](int e, int side) {
             C v;
             v.x = v.y = (T)0;
-            if (abs(freq_index(e, ay.n)) <= ry) v = sl_elem(w, e, row);
+            if (fft::abs_label(e, ay.n, side) <= ry) v = sl_elem(w, e, row);
             return v;
         },
-        [&](int y, C v) {
+        [&](int y, C v, int) {
             if (kz == 0) v.y = (T)0;  // the z pass reads the real part of the plane kz = 0
             sl_elem(w, y, row) = v;
         });
@@ -231,8 +233,8 @@ __global__ void __launch_bounds__(128, SlShape<T>::ZBLOCKS)
     const int K = mp.kz_max;
     fft::line_fft<T, 1>(
         az, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
-        [&](int e) {
-            const bool up = 2 * e > n;
+        [&](int e, int side) {
+            const bool up = side ? side > 0 : 2 * e > n;
             const int kz = up ? n - e : e;
             C v;
             v.x = v.y = (T)0;
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(128, SlShape<T>::ZBLOCKS)
             v.y = up ? b.x - a.y : a.y + b.x;
             return v;
         },
-        [&](int z, C v) {
+        [&](int z, C v, int) {
             oa[z] = v.x;
             ob[z] = v.y;
         });
@@ -335,14 +337,14 @@ __global__ void __launch_bounds__(256, 2)
     const int K = mp.kz_max;
     fft::line_fft<float, 1>(
         az, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
-        [&](int e) {
-            const bool up = 2 * e > n;
+        [&](int e, int side) {
+            const bool up = side ? side > 0 : 2 * e > n;
             const int kz = up ? n - e : e;
             if (kz > K) return make_float2(0.f, 0.f);
             const float2 a = wa[kz], b = wb[kz];
             return up ? make_float2(a.x + b.y, b.x - a.y) : make_float2(a.x - b.y, a.y + b.x);
         },
-        [&](int z, float2 v) {
+        [&](int z, float2 v, int) {
             stg[(2 * line) * lds + z] = v.x;
             stg[(2 * line + 1) * lds + z] = v.y;
         });
