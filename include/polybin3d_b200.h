@@ -137,7 +137,12 @@ PB_API int pb_spectral_filter(const pb_grid_t *g, const int32_t *out_n, int prec
 /* pair) when a band reaches a grid's Nyquist frequency, an upper edge is infinite, or an */
 /* output length has a prime factor other than 2, 3, 5.  Workspace from                 */
 /* pb_shell_synth_workspace_size (same grids, precision and upper edges).                */
+/* l1 may also be PB_HARMONIC + l^2 + m (l = 1..4, m = 0..2l): the real harmonic Y_lm of k  */
+/* takes the place of L_l1 (the weights of the symmetry factors, PolyBin3D/bspec.py:235-276;  */
+/* order and normalisation of utils.pyx:518-609).  PB_ERR_UNSUPPORTED where the output       */
+/* lengths need the run-time transform.                                                     */
 /* ---------------------------------------------------------------------------------- */
+#define PB_HARMONIC 16
 PB_API int pb_shell_synth_workspace_size(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps,
                                          const double *hi, size_t *bytes);
 PB_API int pb_shell_synth(const pb_grid_t *g, const int32_t *out_n, int precision, const void *src,

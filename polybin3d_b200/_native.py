@@ -15,6 +15,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpb_b200.so")
 
 PB_F32, PB_F64 = 0, 1
+PB_HARMONIC = 16    # shell_synth: l1 = PB_HARMONIC + l^2 + m weights by the real harmonic Y_lm(k)
 PB_F32_SRC_F64 = 2  # shell_synth only: FP32 maps from a complex128 source
 PB_FFT_R2C, PB_FFT_C2R = 0, 1
 PB_RED_ABS2, PB_RED_CROSS, PB_RED_REAL2 = 0, 1, 2

@@ -387,24 +387,19 @@ class BSpec:
             nks = self.Nk_squeeze
             w = self._invp_device()
             bins = self._binned_maps(None, [(i, 0, 0, 1.0) for i in range(nks)], w, torch.float64)
-            kg = b.k_grids
-            invP = np.ones(b.nhalf_shape) if self._unit_w else self.invPk0
             for l in range(2, self.lmax + 1, 2):
                 rows = self.all_bins[self.all_bins[:, 3] == l]
                 need = sorted({int(r[2]) for r in rows if (r[0] != r[1] and r[1] == r[2]) or (r[0] == r[1] == r[2])})
                 # sum over m of bins-weighted squares of the Y_lm-weighted binning functions
                 pair_idx = sorted({(int(r[0]), int(r[2])) for r in rows if r[0] != r[1] and r[1] == r[2]} |
                                   {(int(r[2]), int(r[2])) for r in rows if r[0] == r[1] == r[2]})
-                num = {p: 0.0 for p in pair_idx}
                 if pair_idx:
-                    for y in real_harmonics(kg, l):
-                        wy = torch.as_tensor(invP * y, device=b.device)
-                        ym = self._binned_maps(None, [(i, 0, 0, 1.0) for i in need], wy, torch.float64)
-                        pos = {bb: i for i, bb in enumerate(need)}
-                        idx = np.asarray([(p[0], pos[p[1]], pos[p[1]]) for p in pair_idx], dtype=np.int32)
-                        vals = self._contract(None, bins, ym, ym, idx).cpu().numpy()
-                        for p, v in zip(pair_idx, vals):
-                            num[p] += v
+                    pos = {bb: i for i, bb in enumerate(need)}
+                    idx = np.asarray([(p[0], pos[p[1]], pos[p[1]]) for p in pair_idx], dtype=np.int32)
+                    total = 0
+                    for ym in self._harmonic_maps(l, need, w):
+                        total = total + self._contract(('sym_num', l), bins, ym, ym, idx)
+                    num = dict(zip(pair_idx, total.cpu().numpy()))
                     idx3 = np.asarray([(p[0], p[1], p[1]) for p in pair_idx], dtype=np.int32)
                     den = dict(zip(pair_idx, self._contract(('sym_den', l), bins, bins, bins, idx3).cpu().numpy()))
                 for (b1, b2, b3, ll) in rows:
@@ -418,6 +413,28 @@ class BSpec:
                         sym.append(2. * (1. + 2. * num[(b3, b3)] / den[(b3, b3)]))
         self.sym_factor = np.asarray(sym)
         assert len(self.sym_factor) == self.N_bins
+
+    def _harmonic_maps(self, l, need, w):
+        """For each m, the FP64 maps irfftn(Theta_b Y_lm(k) w) of the bins in `need`: the harmonics are
+        evaluated inside the synthesis, or uploaded as weight grids where it cannot (band limit, length)."""
+        b = self.base
+        ks = self.k_bins_squeeze
+        dims = self.map_grid
+        for mi in range(2 * l + 1):
+            if self.synthesis != 'cufft' and self._synth_ok.get(dims, True):
+                maps = [(0, ks[i], ks[i + 1], nat.PB_HARMONIC + l * l + mi, 0, 1.0 / b.nreal, 0 if w is None else 1)
+                        for i in need]
+                out = torch.empty((len(need),) + tuple(dims), dtype=torch.float64, device=b.device)
+                try:
+                    nat.shell_synth(b.grid, nat.PB_F64, None, out, maps, dims, b.ws, w=w, src_stride=b.nhalf)
+                    b.n_FFTs_reverse += len(need)
+                    yield out
+                    continue
+                except NotImplementedError:
+                    pass
+            y = real_harmonics(b.k_grids, l)[mi]
+            wy = torch.as_tensor(y if self._unit_w else self.invPk0 * y, device=b.device)
+            yield self._binned_maps(None, [(i, 0, 0, 1.0) for i in need], wy, torch.float64)
 
     # ------------------------------------------------------------------------------
     # numerator (bspec.py:895-983)

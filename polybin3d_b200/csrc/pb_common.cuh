@@ -109,6 +109,43 @@ __device__ __forceinline__ double block_column_sum(const double *src, int64_t st
     return s;
 }
 
+// Real spherical harmonics of the direction (x, y, z) / r, codes PB_HARMONIC + l^2 + m for l = 1..4,
+// m = 0..2l (PolyBin3D/cython/utils.pyx:518-609, the order and normalisation of harmonics.py:
+// sum_m Y_lm(a) Y_lm(b) = L_l(a.b)); 0 at r = 0 except the constant of l = 4
+__device__ __forceinline__ double real_harmonic(int code, double x, double y, double z, double r) {
+    const double q = r != 0.0 ? 1.0 / r : 0.0;
+    x *= q;
+    y *= q;
+    z *= q;
+    const double x2 = x * x, y2 = y * y, z2 = z * z;
+    switch (code - PB_HARMONIC) {
+        case 1: return y;
+        case 2: return z;
+        case 3: return x;
+        case 4: return 6.0 * x * y * sqrt(1.0 / 12.0);
+        case 5: return 3.0 * y * z * sqrt(1.0 / 3.0);
+        case 6: return z2 - 0.5 * x2 - 0.5 * y2;
+        case 7: return 3.0 * x * z * sqrt(1.0 / 3.0);
+        case 8: return (3.0 * x2 - 3.0 * y2) * sqrt(1.0 / 12.0);
+        case 9: return (45.0 * x2 * y - 15.0 * y2 * y) * sqrt(1.0 / 360.0);
+        case 10: return 30.0 * x * y * z * sqrt(1.0 / 60.0);
+        case 11: return (-1.5 * x2 * y - 1.5 * y2 * y + 6.0 * y * z2) * sqrt(1.0 / 6.0);
+        case 12: return -1.5 * x2 * z - 1.5 * y2 * z + z2 * z;
+        case 13: return (-1.5 * x2 * x - 1.5 * x * y2 + 6.0 * x * z2) * sqrt(1.0 / 6.0);
+        case 14: return (15.0 * x2 * z - 15.0 * y2 * z) * sqrt(1.0 / 60.0);
+        case 15: return (15.0 * x2 * x - 45.0 * x * y2) * sqrt(1.0 / 360.0);
+        case 16: return (420.0 * x2 * x * y - 420.0 * x * y2 * y) * sqrt(1.0 / 20160.0);
+        case 17: return (315.0 * x2 * y * z - 105.0 * y2 * y * z) * sqrt(1.0 / 2520.0);
+        case 18: return (-15.0 * x2 * x * y - 15.0 * x * y2 * y + 90.0 * x * y * z2) * sqrt(1.0 / 180.0);
+        case 19: return (-7.5 * x2 * y * z - 7.5 * y2 * y * z + 10.0 * y * z2 * z) * sqrt(1.0 / 10.0);
+        case 20: return 35.0 / 8.0 * z2 * z2 - 15.0 / 4.0 * z2 + 3.0 / 8.0;
+        case 21: return (-7.5 * x2 * x * z - 7.5 * x * y2 * z + 10.0 * x * z2 * z) * sqrt(1.0 / 10.0);
+        case 22: return (-7.5 * x2 * x2 + 45.0 * x2 * z2 + 7.5 * y2 * y2 - 45.0 * y2 * z2) * sqrt(1.0 / 180.0);
+        case 23: return (105.0 * x2 * x * z - 315.0 * x * y2 * z) * sqrt(1.0 / 2520.0);
+        default: return (105.0 * x2 * x2 - 630.0 * x2 * y2 + 105.0 * y2 * y2) * sqrt(1.0 / 20160.0);
+    }
+}
+
 template <typename T> struct cplx;
 template <> struct cplx<float> { using type = float2; };
 template <> struct cplx<double> { using type = double2; };

@@ -539,7 +539,8 @@ static int synth_layout(const pb_grid_t *g, const int32_t *out_n, int precision,
         SynthMap &mp = p.maps[m];
         if (!(hi[m] > 0.0) || !std::isfinite(hi[m]))
             return fail(PB_ERR_UNSUPPORTED, "pb_shell_synth: every map needs a finite upper edge");
-        if (l1[m] < 0 || l1[m] > 4 || l2[m] < 0 || l2[m] > 4)
+        const bool harmonic = l1[m] > PB_HARMONIC && l1[m] <= PB_HARMONIC + 24 && l2[m] == 0;
+        if (!harmonic && (l1[m] < 0 || l1[m] > 4 || l2[m] < 0 || l2[m] > 4))
             return fail(PB_ERR_INVALID, "pb_shell_synth: Legendre order must be in [0, 4]");
         const int wp = wpow ? wpow[m] : 0;
         if (wp < -1 || wp > 2) return fail(PB_ERR_INVALID, "pb_shell_synth: wpow must be -1, 0, 1 or 2");
@@ -777,6 +778,8 @@ static int shell_synth(const pb_grid_t *g, const int32_t *out_n, int precision, 
         }
     }
     if (!workspace || workspace_bytes < need) return fail(PB_ERR_INVALID, "pb_shell_synth: workspace too small");
+    for (int m = 0; m < n_maps; ++m)
+        if (l1[m] > 4) return fail(PB_ERR_UNSUPPORTED, "pb_shell_synth: harmonic weights need line transforms");
     if (src64) {
         float2 *U = (float2 *)ws;
         st = launch_synth<float, double2>(L, (const double2 *)src, (const float *)w, U, U + L.u_elems, (float *)out, s);
