@@ -149,7 +149,9 @@ def get_tuning():
 
 
 def stream_ptr():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream (its raw handle: building a torch Stream object for it
+    costs several microseconds a call)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t):
@@ -158,7 +160,7 @@ def ptr(t):
 
 def hptr(a):
     """Host numpy array -> void*."""
-    return ctypes.c_void_p(a.ctypes.data)
+    return ctypes.c_void_p(a.__array_interface__["data"][0])
 
 
 def precision_of(dtype):
@@ -553,13 +555,28 @@ class BilinearPlan:
         c = np.ascontiguousarray(c, dtype=np.float64)
         nbytes = ctypes.c_size_t()
         n = np.zeros(1, dtype=np.int32)
-        check(lib.pb_bilinear_plan(n_g, n_out, hptr(o), hptr(i), hptr(j), hptr(c), len(o), None, ctypes.byref(nbytes),
-                                   hptr(n)), "pb_bilinear_plan")
+        self.slot = np.zeros(max(1, len(o)), dtype=np.int32)
+        check(lib.pb_bilinear_block_plan(n_g, n_out, hptr(o), hptr(i), hptr(j), hptr(c), len(o), None,
+                                         ctypes.byref(nbytes), hptr(n), None), "pb_bilinear_block_plan")
         host = np.zeros(nbytes.value, dtype=np.uint8)
-        check(lib.pb_bilinear_plan(n_g, n_out, hptr(o), hptr(i), hptr(j), hptr(c), len(o), hptr(host),
-                                   ctypes.byref(nbytes), hptr(n)), "pb_bilinear_plan")
+        check(lib.pb_bilinear_block_plan(n_g, n_out, hptr(o), hptr(i), hptr(j), hptr(c), len(o), hptr(host),
+                                         ctypes.byref(nbytes), hptr(n), hptr(self.slot)), "pb_bilinear_block_plan")
         self.n_g, self.n_out, self.n_table = n_g, n_out, int(n[0])
+        self.host, self.slot = host, self.slot[:len(o)]
         self.table = torch.from_numpy(host).to(device)
+
+    def with_coefficients(self, c):
+        """The plan of the same terms with other coefficients c (in the order given at first)."""
+        p = object.__new__(BilinearPlan)
+        p.__dict__.update(self.__dict__)
+        host = self.host.copy()
+        head = len(host) - 64 * self.n_table
+        c4 = np.bincount(self.slot, weights=c, minlength=4 * self.n_table).reshape(-1, 4)
+        host[head:].view(np.float64).reshape(-1, 8)[:, 4:] = c4
+        host[head:].view(np.float32).reshape(-1, 16)[:, 4:8] = c4
+        p.host = host
+        p.table = torch.from_numpy(host).to(self.table.device)
+        return p
 
     def maps(self, G, out=None):
         """out[o] = sum_t c_t G[i_t] G[j_t]; G (n_g, ...) real maps."""
@@ -567,8 +584,8 @@ class BilinearPlan:
             raise ValueError("BilinearPlan.maps: the plan was built for %d maps" % self.n_g)
         if out is None:
             out = torch.empty((self.n_out,) + tuple(G.shape[1:]), dtype=G.dtype, device=G.device)
-        check(load().pb_bilinear_maps(precision_of(G.dtype), G[0].numel(), ptr(G), self.n_g, ptr(self.table),
-                                      self.n_table, self.n_out, ptr(out), stream_ptr()), "pb_bilinear_maps")
+        check(load().pb_bilinear_block_maps(precision_of(G.dtype), G[0].numel(), ptr(G), self.n_g, ptr(self.table),
+                                            self.n_table, self.n_out, ptr(out), stream_ptr()), "pb_bilinear_block_maps")
         _count(1)
         return out
 

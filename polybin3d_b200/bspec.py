@@ -777,23 +777,17 @@ class BSpec:
             u = self._binned_maps(None, [(bb, l, 0, 1.0) for l in range(0, self.lmax + 1, 2) for bb in range(nks)], w,
                                   torch.float64)
             u0 = u[:nks]
+            same12, same23 = idx3[:, 0] == idx3[:, 1], idx3[:, 1] == idx3[:, 2]
             for l in range(0, self.lmax + 1, 2):
                 for lp in range(l, self.lmax + 1, 2):
                     ull = self._binned_maps(None, [(bb, l, lp, 1.0) for bb in range(nks)], w, torch.float64)
                     T1 = self._contract('fid', u0, u0, ull, idx3).cpu().numpy()
                     T2 = self._contract('fid', u0, u[l // 2 * nks:(l // 2 + 1) * nks],
                                         u[lp // 2 * nks:(lp // 2 + 1) * nks], idx3).cpu().numpy()
-                    for i in range(self.N3):
-                        b1, b2, b3 = idx3[i]
-                        if b1 != b2 and b2 != b3:
-                            v = T1[i]
-                        elif b1 == b2 and b2 != b3:
-                            v = 2. * T1[i]
-                        elif b1 != b2 and b2 == b3:
-                            v = T2[i] + T1[i]
-                        else:
-                            v = 4. * T2[i] + 2. * T1[i]
-                        fish[l // 2 * self.N3 + i, lp // 2 * self.N3 + i] = v
+                    # T1 for distinct bins, 2 T1 for b1 = b2, T2 + T1 for b2 = b3, 4 T2 + 2 T1 for all equal
+                    v = np.where(same12, 2. * T1, T1) + np.where(same23, np.where(same12, 4. * T2, T2), 0.)
+                    at = np.arange(self.N3)
+                    fish[l // 2 * self.N3 + at, lp // 2 * self.N3 + at] = v
             fish = fish + fish.T - np.diag(np.diag(fish))
             scaling = b.gridsize.prod() ** 2 / b.volume
             fish = fish / np.outer(self.sym_factor, self.sym_factor) * scaling
