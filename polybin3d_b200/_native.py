@@ -65,6 +65,8 @@ SIGNATURES = {
     "pb_binned_filter": ([_GP, _I, _P, _P, _P, _I, _P, _I, _P, _P, _I, _D, _P], _I),
     "pb_bilinear_plan": ([_I, _I, _P, _P, _P, _P, _I, _P, ctypes.POINTER(_SZ), _P], _I),
     "pb_bilinear_maps": ([_I, _I64, _P, _I, _P, _I, _I, _P, _P], _I),
+    "pb_bilinear_block_plan": ([_I, _I, _P, _P, _P, _P, _I, _P, ctypes.POINTER(_SZ), _P, _P], _I),
+    "pb_bilinear_block_maps": ([_I, _I64, _P, _I, _P, _I, _I, _P, _P], _I),
     "pb_shell_synth_workspace_size": ([_GP, _P, _I, _I, _P, ctypes.POINTER(_SZ)], _I),
     "pb_shell_synth": ([_GP, _P, _I, _P, _I64, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _SZ, _P], _I),
     "pb_bin_reduce_workspace_size": ([_GP, _I, _I, _I, ctypes.POINTER(_SZ)], _I),
@@ -545,7 +547,7 @@ def _shell_synth_tiled(lib, grid, precision, src, out, maps, out_n, ws, w, src_s
 
 
 class BilinearPlan:
-    """Device table of pb_bilinear_plan for host terms (o, i, j, c)."""
+    """Device table of pb_bilinear_block_plan for host terms (o, i, j, c)."""
 
     def __init__(self, n_g, n_out, o, i, j, c, device):
         lib = load()

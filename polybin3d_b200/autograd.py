@@ -199,6 +199,20 @@ class BkNumerator(torch.autograd.Function):
         return B3 * norm
 
     @staticmethod
+    def _legs(bs, rows, coef, n_maps):
+        """The legs of the triplets `rows` (b1, b2, b3, l): outputs [(bin C, multipole lc)], by multipole
+        then bin, and the plan of the terms that end on them (first leg b1 of every triplet, then
+        b2, then b3)."""
+        nks = bs.Nk_squeeze
+        b1, b2, b3, l = rows.T
+        c3 = l // 2 * nks + b3
+        end = np.concatenate([b1, b2, c3])          # lc / 2 * nks + C
+        ends, o = np.unique(end, return_inverse=True)
+        plan = nat.BilinearPlan(n_maps, len(ends), o, np.concatenate([b2, b1, b1]), np.concatenate([c3, c3, b2]),
+                                np.concatenate([coef, coef, coef]), bs.base.device)
+        return [(int(e % nks), 2 * int(e // nks)) for e in ends], plan
+
+    @staticmethod
     def backward(ctx, g):
         _settle()
         bs = ctx.bs
@@ -207,44 +221,36 @@ class BkNumerator(torch.autograd.Function):
         rd = d.dtype
         prec = nat.precision_of(rd)
         cd = torch.complex128 if rd == torch.float64 else torch.complex64
+        gam = g.to(torch.float64).cpu().numpy()   # read before the maps are queued: the table below is built meanwhile
         G = BkNumerator._maps(bs, d)  # recomputed, not stored
         Mdims = tuple(int(n) for n in G.shape[1:])
         nks = bs.Nk_squeeze
         ks = bs.k_bins_squeeze
         ab = bs.all_bins
-        gam = g.to(torch.float64).cpu().numpy()
         N3 = float(b.gridsize.prod())
         M3 = float(np.prod(Mdims))
         # coefficient of triplet i: V / (sym_i N^3) * (N^3/M^3) [map-grid transform] / N^3 [c2r]
         coef = gam * b.volume / (bs.sym_factor * N3 * M3)
-        legs = {}
-        keys = {}
-
-        def key_of(i, j):
-            return keys.setdefault((i, j), len(keys))
-
-        for t, (b1, b2, b3, l) in enumerate(ab.tolist()):
-            if coef[t] == 0.0:
-                continue
-            c3 = (l // 2) * nks + b3
-            for (kk, C, lc) in ((key_of(b2, c3), b1, 0), (key_of(b1, c3), b2, 0), (key_of(b1, b2), b3, l)):
-                legs[(kk, C, lc)] = legs.get((kk, C, lc), 0.0) + coef[t]
         # local sightline: the l > 0 maps are IFT(Theta_b H_l x), so a leg ending on (C, l > 0)
         # goes through the bin filter alone into an accumulator per l, and H_l^dag is applied
         # once per l below (H_l^dag v = FT[sum_m Y_lm(r) IFT(Y_lm(k) v)])
         local = b.sightline == 'local' and bs.lmax > 0
         n_acc = 1 + (bs.lmax // 2 if local else 0)
         grad_spec = torch.zeros((n_acc,) + b.nhalf_shape, dtype=cd, device=b.device)
-        if keys:
+        if np.any(coef):
             # one real-space map per leg (bin C, multipole lc): the coefficient-weighted sum of
             # the products of the other two maps of every triplet ending on it (pb_bilinear_maps);
-            # then one forward transform per leg and one accumulating filter into the gradient
-            pairs = sorted(keys, key=keys.get)
-            outs = sorted({(C, lc) for (kk, C, lc) in legs})
-            opos = {oc: n for n, oc in enumerate(outs)}
-            tl = [(opos[(C, lc)], pairs[kk][0], pairs[kk][1], v) for (kk, C, lc), v in legs.items()]
-            plan = nat.BilinearPlan(G.shape[0], len(outs), [t[0] for t in tl], [t[1] for t in tl],
-                                    [t[2] for t in tl], [t[3] for t in tl], b.device)
+            # then one forward transform per leg and one accumulating filter into the gradient.
+            # The terms depend on the binning alone: the table of all triplets is kept and only its
+            # coefficients change (a cotangent with zeros gets a table of its own, without their legs)
+            if np.all(coef):
+                if getattr(bs, '_leg_plan', None) is None:
+                    bs._leg_plan = BkNumerator._legs(bs, ab, coef, G.shape[0])
+                outs, plan = bs._leg_plan
+                plan = plan.with_coefficients(np.concatenate([coef, coef, coef]))
+            else:
+                use = coef != 0.0
+                outs, plan = BkNumerator._legs(bs, ab[use], coef[use], G.shape[0])
             R = plan.maps(G)
             del G
             per_out = R[0].numel() * R.element_size() * 2
