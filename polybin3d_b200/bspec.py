@@ -420,6 +420,7 @@ class BSpec:
         b = self.base
         ks = self.k_bins_squeeze
         dims = self.map_grid
+        grids = None
         for mi in range(2 * l + 1):
             if self.synthesis != 'cufft' and self._synth_ok.get(dims, True):
                 maps = [(0, ks[i], ks[i + 1], nat.PB_HARMONIC + l * l + mi, 0, 1.0 / b.nreal, 0 if w is None else 1)
@@ -432,7 +433,8 @@ class BSpec:
                     continue
                 except NotImplementedError:
                     pass
-            y = real_harmonics(b.k_grids, l)[mi]
+            grids = real_harmonics(b.k_grids, l) if grids is None else grids
+            y = grids[mi]
             wy = torch.as_tensor(y if self._unit_w else self.invPk0 * y, device=b.device)
             yield self._binned_maps(None, [(i, 0, 0, 1.0) for i in need], wy, torch.float64)
 

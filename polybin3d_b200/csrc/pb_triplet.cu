@@ -1,6 +1,7 @@
-// Triplet contraction  out[t] = scale * sum_x A[i1](x) B[i2](x) C[i3](x)  on CUDA cores.
+// Triplet contraction  out[t] = scale * sum_x A[i1](x) B[i2](x) C[i3](x): FP32 maps on CUDA cores,
+// FP64 maps by FP64 matrix instructions (triplet_f64_kernel below).
 //
-// The triplet list is tiled on the host into "items": one A map, up to TB B maps and up
+// FP32: the triplet list is tiled on the host into "items": one A map, up to TB B maps and up
 // to TC C maps, so one thread forms TB pair products and TB x TC FMAs per voxel from
 // 1 + TB + TC shared-memory loads.  A CTA stages a tile of TV voxels of every map in
 // shared memory, P threads share an item (voxels strided by P), per-tile sums are kept in
@@ -101,14 +102,14 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
-template <typename T>
+template <typename T, int TV>
 __device__ __forceinline__ void simt_stage(T *buf, const T *A, int n_a, const T *B, int n_b, int off_b, const T *C,
                                            int off_c, int n_rows, int64_t n_vox, int64_t v0, bool vec) {
-    constexpr int LD = SIMT_TV + SIMT_PAD;
+    constexpr int LD = TV + SIMT_PAD;
     constexpr int EPV = 16 / sizeof(T);  // elements per 16-byte copy
     if (vec) {
-        const int per_row = SIMT_TV / EPV;
-        for (int e = threadIdx.x; e < n_rows * per_row; e += SIMT_THREADS) {
+        const int per_row = TV / EPV;
+        for (int e = threadIdx.x; e < n_rows * per_row; e += blockDim.x) {
             int r = e / per_row, c = e - r * per_row;
             const T *src;
             int m;
@@ -122,8 +123,8 @@ __device__ __forceinline__ void simt_stage(T *buf, const T *A, int n_a, const T 
             cp_async16(buf + r * LD + c * EPV, g, bytes);
         }
     } else {
-        for (int e = threadIdx.x; e < n_rows * SIMT_TV; e += SIMT_THREADS) {
-            int r = e / SIMT_TV, v = e - r * SIMT_TV;
+        for (int e = threadIdx.x; e < n_rows * TV; e += blockDim.x) {
+            int r = e / TV, v = e - r * TV;
             const T *src;
             int m;
             if (r < n_a) { src = A; m = r; }
@@ -143,13 +144,13 @@ __device__ __forceinline__ void simt_stage(T *buf, const T *A, int n_a, const T 
     cp_async_commit();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(SIMT_THREADS, sizeof(T) == 4 ? 3 : 1) triplet_simt_kernel(const T *A, int n_a, const T *B, int n_b,
-                                                                      int off_b, const T *C, int n_c, int off_c,
-                                                                      int n_rows, int64_t n_vox,
-                                                                      const TripletItem *items, int n_items,
-                                                                      int group_p, double *partials, int n_trip,
-                                                                      int vec) {
+__global__ void __launch_bounds__(SIMT_THREADS, 3) triplet_simt_kernel(const float *A, int n_a, const float *B, int n_b,
+                                                                       int off_b, const float *C, int n_c, int off_c,
+                                                                       int n_rows, int64_t n_vox,
+                                                                       const TripletItem *items, int n_items,
+                                                                       int group_p, double *partials, int n_trip,
+                                                                       int vec) {
+    using T = float;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int LD = SIMT_TV + SIMT_PAD;
     T *buf0 = reinterpret_cast<T *>(smem_raw);
@@ -192,13 +193,13 @@ __global__ void __launch_bounds__(SIMT_THREADS, sizeof(T) == 4 ? 3 : 1) triplet_
 
     const int64_t n_tiles = (n_vox + SIMT_TV - 1) / SIMT_TV;
     int64_t tt = blockIdx.x;
-    if (tt < n_tiles) simt_stage<T>(buf0, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * SIMT_TV, vec);
+    if (tt < n_tiles) simt_stage<T, SIMT_TV>(buf0, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * SIMT_TV, vec);
     int cur = 0, since_flush = 0;
     for (; tt < n_tiles; tt += gridDim.x) {
         T *tile = cur ? buf1 : buf0;
         const int64_t nxt = tt + gridDim.x;
         if (nxt < n_tiles) {
-            simt_stage<T>(cur ? buf0 : buf1, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, nxt * SIMT_TV, vec);
+            simt_stage<T, SIMT_TV>(cur ? buf0 : buf1, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, nxt * SIMT_TV, vec);
             cp_async_wait1();
         } else {
             cp_async_wait0();
@@ -239,6 +240,127 @@ __global__ void __launch_bounds__(SIMT_THREADS, sizeof(T) == 4 ? 3 : 1) triplet_
     }
 }
 
+// ------------------------------------------------------------------------------------
+// FP64 maps: a dense product on the FP64 matrix instruction.
+//
+// out[pair][c] = sum_x (A_a B_b)(x) C_c(x) is a product of the distinct pairs (a, b) of the list (sorted)
+// with the C maps, over the voxels.  Tiles of D_TV voxels of every map are staged as above.  A warp
+// holds D_U tiles of 8 pairs against up to four tiles of 8 C maps: per 4 voxels a lane forms one product of
+// each pair tile, takes one value of each C tile and feeds every (pair tile, C tile) that holds a triplet
+// of the list to mma.m8n8k4 (the others are skipped: of 12 bins, l = 0, 2, about half).  Sums stay in the
+// FP64 accumulators; at the end the warps that share pair tiles (KS of them, each on its voxels)
+// add up in shared memory in order and the block writes one partial per triplet.
+// Reading a fragment is 8 rows of 32 contiguous bytes: the row stride of 4 mod 16 elements puts them on
+// distinct banks.  The form before, 4 x 8 outputs per thread on CUDA cores, had its 32 FP64 sums, half of
+// them empty, in registers that left 8 warps per SM.
+// D_MEASURED
+// ------------------------------------------------------------------------------------
+constexpr int D_TV = 64;            // voxels per tile
+constexpr int D_U = 2;              // pair tiles per warp
+constexpr int D_PT = 32;            // pair tiles per block (grid.y: more), 16 warps at most
+constexpr int D_CT = 4;             // C tiles per block (grid.y: more)
+
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// grid: (parts of the voxels, pair groups x C groups); block: G x KS warps
+template <int NCT>
+__global__ void __launch_bounds__(512) triplet_f64_kernel(const double *A, int n_a, const double *B, int n_b, int off_b,
+                                                         const double *C, int n_c, int off_c, int n_rows, int64_t n_vox,
+                                                         const int32_t *pairs, int n_pairs, const int32_t *tmap,
+                                                         int n_trip, int G, int c_groups, double *partials, int vec) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned used[D_PT];   // C tiles of each pair tile that hold a triplet
+    constexpr int LD = D_TV + SIMT_PAD, ML = 8 * NCT + 1;
+    double *const buf = reinterpret_cast<double *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, KS = (blockDim.x >> 5) / G, g = warp % G, ks = warp / G;
+    const int p0 = (blockIdx.y / c_groups) * D_PT * 8, c0 = (blockIdx.y % c_groups) * D_CT * 8;
+    const int np = min(D_PT * 8, n_pairs - p0);
+    for (int i = threadIdx.x; i < D_PT; i += blockDim.x) used[i] = 0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < n_trip; t += blockDim.x) {
+        const int row = tmap[2 * t] - p0, col = tmap[2 * t + 1] - c0;
+        if (row >= 0 && row < np && col >= 0 && col < 8 * NCT) atomicOr(&used[row >> 3], 1u << (col >> 3));
+    }
+    __syncthreads();
+    // rows clamped into the staged tile: a table built for other map counts cannot index outside it
+    const int r8 = lane >> 2, k4 = lane & 3;
+    int ra[D_U], rb[D_U], rc[NCT];
+    unsigned on[D_U], any = 0;
+    double acc[D_U][NCT][2];
+#pragma unroll
+    for (int u = 0; u < D_U; ++u) {
+        const int pt = u * G + g;
+        on[u] = pt < D_PT && pt * 8 < np ? used[pt] : 0u;
+        any |= on[u];
+        const int pr = min(p0 + pt * 8 + r8, n_pairs - 1);
+        ra[u] = min(max(pairs[2 * pr], 0), n_rows - 1) * LD + k4;
+        rb[u] = min(max(off_b + pairs[2 * pr + 1], 0), n_rows - 1) * LD + k4;
+#pragma unroll
+        for (int j = 0; j < NCT; ++j) acc[u][j][0] = acc[u][j][1] = 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < NCT; ++j) rc[j] = min(off_c + min(c0 + 8 * j + r8, n_c - 1), n_rows - 1) * LD + k4;
+
+    const int64_t n_tiles = (n_vox + D_TV - 1) / D_TV;
+    int64_t tt = blockIdx.x;
+    if (tt < n_tiles) simt_stage<double, D_TV>(buf, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * D_TV, vec);
+    int cur = 0;
+    for (; tt < n_tiles; tt += gridDim.x) {
+        const double *tile = buf + (cur ? n_rows * LD : 0);
+        const int64_t nxt = tt + gridDim.x;
+        if (nxt < n_tiles) {
+            simt_stage<double, D_TV>(buf + (cur ? 0 : n_rows * LD), A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox,
+                                     nxt * D_TV, vec);
+            cp_async_wait1();
+        } else {
+            cp_async_wait0();
+        }
+        __syncthreads();
+        if (any) {
+#pragma unroll 2
+            for (int v = 4 * ks; v < D_TV; v += 4 * KS) {
+                double c[NCT];
+#pragma unroll
+                for (int j = 0; j < NCT; ++j) c[j] = tile[rc[j] + v];
+#pragma unroll
+                for (int u = 0; u < D_U; ++u) {
+                    const double p = tile[ra[u] + v] * tile[rb[u] + v];
+#pragma unroll
+                    for (int j = 0; j < NCT; ++j)
+                        if (on[u] >> j & 1u) mma_f64(acc[u][j], p, c[j]);
+                }
+            }
+        }
+        __syncthreads();
+        cur ^= 1;
+    }
+    // sums[pair][c] over the KS warps of a pair tile, in order
+    double *const sums = buf;
+    for (int q = 0; q < KS; ++q) {
+        if (ks == q) {
+#pragma unroll
+            for (int u = 0; u < D_U; ++u) {
+                if (!on[u]) continue;
+                double *row = sums + ((u * G + g) * 8 + r8) * ML + 2 * k4;
+#pragma unroll
+                for (int j = 0; j < NCT; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) row[8 * j + h] = q ? row[8 * j + h] + acc[u][j][h] : acc[u][j][h];
+            }
+        }
+        __syncthreads();
+    }
+    double *dst = partials + (int64_t)blockIdx.x * n_trip;
+    for (int t = threadIdx.x; t < n_trip; t += blockDim.x) {
+        const int row = tmap[2 * t] - p0, col = tmap[2 * t + 1] - c0;
+        if (row >= 0 && row < np && col >= 0 && col < 8 * NCT) dst[t] = sums[row * ML + col];
+    }
+}
+
 __global__ void triplet_finalize(const double *partials, int n_parts, int n_trip, double scale, double *out) {
     const int t = blockIdx.x * SUM_COLS + threadIdx.x;
     const double s = block_column_sum(partials + t, n_trip, n_parts, t < n_trip);
@@ -259,9 +381,28 @@ int simt_geometry(int64_t n_vox, int n_items, int *grid_x, int *grid_y, int *gro
     return PB_OK;
 }
 
+template <int NCT>
+static cudaError_t launch_f64(const double *A, int n_a, const double *B, int n_b, int off_b, const double *C, int n_c,
+                              int off_c, int n_rows, int64_t n_vox, const int32_t *pairs, int n_pairs,
+                              const int32_t *tmap, int n_trip, int parts, double *partials, int vec, cudaStream_t s) {
+    const int pt = std::min(D_PT, (n_pairs + 7) / 8), G = (pt + D_U - 1) / D_U;
+    int KS = 1;                       // a power of two (16 steps of 4 voxels a tile), up to 12 warps per block
+    while (KS < 8 && 2 * KS * G <= 12) KS *= 2;
+    const int c_groups = (n_c + 8 * D_CT - 1) / (8 * D_CT), p_groups = (n_pairs + 8 * D_PT - 1) / (8 * D_PT);
+    const size_t smem = std::max((size_t)2 * n_rows * (D_TV + SIMT_PAD), (size_t)pt * 8 * (8 * NCT + 1)) * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(triplet_f64_kernel<NCT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    triplet_f64_kernel<NCT><<<dim3(parts, p_groups * c_groups), 32 * G * KS, smem, s>>>(
+        A, n_a, B, n_b, off_b, C, n_c, off_c, n_rows, n_vox, pairs, n_pairs, tmap, n_trip, G, c_groups, partials, vec);
+    return cudaGetLastError();
+}
+
 int launch_triplet_simt(int precision, const void *A, int n_a, const void *B, int n_b, const void *C, int n_c,
-                        int64_t n_vox, const TripletItem *items_dev, int n_items, int n_trip, double scale,
-                        double *out, void *workspace, size_t workspace_bytes, cudaStream_t s) {
+                        int64_t n_vox, const unsigned char *table, const int32_t *counts, double scale, double *out,
+                        void *workspace, size_t workspace_bytes, cudaStream_t s) {
+    const TableLayout L = table_layout(counts);
+    const TripletItem *items_dev = (const TripletItem *)(table + L.off_items);
+    const int n_items = counts[0], n_trip = counts[3];
     int gx, gy, gp;
     simt_geometry(n_vox, n_items, &gx, &gy, &gp);
     size_t need = (size_t)gx * n_trip * sizeof(double);
@@ -284,15 +425,23 @@ int launch_triplet_simt(int precision, const void *A, int n_a, const void *B, in
     dim3 grid(gx, gy);
     double *partials = (double *)workspace;
     if (precision == PB_F32) {
-        PB_CUDA(cudaFuncSetAttribute(triplet_simt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        triplet_simt_kernel<float><<<grid, SIMT_THREADS, smem, s>>>(
+        PB_CUDA(cudaFuncSetAttribute(triplet_simt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        triplet_simt_kernel<<<grid, SIMT_THREADS, smem, s>>>(
             (const float *)A, n_a, (const float *)B, n_b, off_b, (const float *)C, n_c, off_c, n_rows, n_vox,
             items_dev, n_items, gp, partials, n_trip, vec);
     } else {
-        PB_CUDA(cudaFuncSetAttribute(triplet_simt_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        triplet_simt_kernel<double><<<grid, SIMT_THREADS, smem, s>>>(
-            (const double *)A, n_a, (const double *)B, n_b, off_b, (const double *)C, n_c, off_c, n_rows, n_vox,
-            items_dev, n_items, gp, partials, n_trip, vec);
+        const int32_t *pairs = (const int32_t *)(table + L.off_pairs), *tmap = (const int32_t *)(table + L.off_tmap);
+        auto run = [&](auto NCT) {
+            return launch_f64<decltype(NCT)::value>((const double *)A, n_a, (const double *)B, n_b, off_b, (const double *)C,
+                                                    n_c, off_c, n_rows, n_vox, pairs, counts[1], tmap, n_trip, gx,
+                                                    partials, vec, s);
+        };
+        switch (std::min(D_CT, (n_c + 7) / 8)) {
+            case 1: PB_CUDA(run(std::integral_constant<int, 1>())); break;
+            case 2: PB_CUDA(run(std::integral_constant<int, 2>())); break;
+            case 3: PB_CUDA(run(std::integral_constant<int, 3>())); break;
+            default: PB_CUDA(run(std::integral_constant<int, 4>()));
+        }
     }
     PB_LAUNCH_CHECK("pb_triplet_contract(simt)");
     triplet_finalize<<<(n_trip + SUM_COLS - 1) / SUM_COLS, dim3(SUM_COLS, SUM_ROWS), 0, s>>>(partials, gx, n_trip, scale, out);
@@ -422,9 +571,8 @@ extern "C" int pb_triplet_contract(int precision, int method, const void *A, int
                                  as_stream(stream));
     }
     if (method != PB_TRIPLET_SIMT) return fail(PB_ERR_INVALID, "bad method");
-    TableLayout L = table_layout(counts);
-    return launch_triplet_simt(precision, A, n_a, B, n_b, C, n_c, n_vox, (const TripletItem *)(T + L.off_items),
-                               counts[0], counts[3], scale, out, workspace, workspace_bytes, as_stream(stream));
+    return launch_triplet_simt(precision, A, n_a, B, n_b, C, n_c, n_vox, T, counts, scale, out, workspace,
+                               workspace_bytes, as_stream(stream));
 }
 
 extern "C" int pb_tiled_maps_bytes(int n_maps, int n_factor, int64_t n_vox, size_t *bytes) {
