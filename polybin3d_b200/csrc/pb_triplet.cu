@@ -102,10 +102,10 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
-template <typename T, int TV>
+template <typename T, int TV, int PAD>
 __device__ __forceinline__ void simt_stage(T *buf, const T *A, int n_a, const T *B, int n_b, int off_b, const T *C,
                                            int off_c, int n_rows, int64_t n_vox, int64_t v0, bool vec) {
-    constexpr int LD = TV + SIMT_PAD;
+    constexpr int LD = TV + PAD;
     constexpr int EPV = 16 / sizeof(T);  // elements per 16-byte copy
     if (vec) {
         const int per_row = TV / EPV;
@@ -193,13 +193,13 @@ __global__ void __launch_bounds__(SIMT_THREADS, 3) triplet_simt_kernel(const flo
 
     const int64_t n_tiles = (n_vox + SIMT_TV - 1) / SIMT_TV;
     int64_t tt = blockIdx.x;
-    if (tt < n_tiles) simt_stage<T, SIMT_TV>(buf0, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * SIMT_TV, vec);
+    if (tt < n_tiles) simt_stage<T, SIMT_TV, SIMT_PAD>(buf0, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * SIMT_TV, vec);
     int cur = 0, since_flush = 0;
     for (; tt < n_tiles; tt += gridDim.x) {
         T *tile = cur ? buf1 : buf0;
         const int64_t nxt = tt + gridDim.x;
         if (nxt < n_tiles) {
-            simt_stage<T, SIMT_TV>(cur ? buf0 : buf1, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, nxt * SIMT_TV, vec);
+            simt_stage<T, SIMT_TV, SIMT_PAD>(cur ? buf0 : buf1, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, nxt * SIMT_TV, vec);
             cp_async_wait1();
         } else {
             cp_async_wait0();
@@ -244,37 +244,39 @@ __global__ void __launch_bounds__(SIMT_THREADS, 3) triplet_simt_kernel(const flo
 // FP64 maps: a dense product on the FP64 matrix instruction.
 //
 // out[pair][c] = sum_x (A_a B_b)(x) C_c(x) is a product of the distinct pairs (a, b) of the list (sorted)
-// with the C maps, over the voxels.  Tiles of D_TV voxels of every map are staged as above.  A warp
-// holds D_U tiles of 8 pairs against up to four tiles of 8 C maps: per 4 voxels a lane forms one product of
-// each pair tile, takes one value of each C tile and feeds every (pair tile, C tile) that holds a triplet
-// of the list to mma.m8n8k4 (the others are skipped: of 12 bins, l = 0, 2, about half).  Sums stay in the
-// FP64 accumulators; at the end the warps that share pair tiles (KS of them, each on its voxels)
-// add up in shared memory in order and the block writes one partial per triplet.
-// Reading a fragment is 8 rows of 32 contiguous bytes: the row stride of 4 mod 16 elements puts them on
-// distinct banks.  The form before, 4 x 8 outputs per thread on CUDA cores, had its 32 FP64 sums, half of
-// them empty, in registers that left 8 warps per SM.
-// D_MEASURED
+// with the C maps, over the voxels.  Tiles of 128 (64) voxels of every map are staged as above.  A warp
+// holds two tiles of 8 pairs against up to four tiles of 8 C maps: per 8 voxels a lane takes two voxels of
+// one row of each pair tile and C tile (16-byte reads), forms the pair products and feeds each C tile that
+// holds a triplet of its pairs to two mma.m16n8k4.  Sums stay in the FP64 accumulators; at the end
+// the warps that share pair tiles (KS of them, each on its voxels) add up in shared memory in order and
+// the block writes one partial per triplet.  The row stride of 8 mod 16 elements puts the rows of a read on
+// distinct banks.
+// The FP64 rate bounds it: 16 bins, l = 0, 2, on 192^3 take 2.52 ms, 26 TFLOP/s of matrix products.  The
+// form before, 4 x 8 outputs per thread on CUDA cores, held its 32 FP64 sums, half of them empty, in
+// registers that left 8 warps per SM: 12 bins on 120^3 400 us, now 196 us (m8n8k4 and 8-byte reads: 214 us;
+// four pair tiles per warp: 241 us); 9 bins, l = 0, 2, on 90 x 120 x 100 260 us, now 119 us.
 // ------------------------------------------------------------------------------------
-constexpr int D_TV = 64;            // voxels per tile
+constexpr int D_PAD = 8;            // row padding
 constexpr int D_U = 2;              // pair tiles per warp
 constexpr int D_PT = 32;            // pair tiles per block (grid.y: more), 16 warps at most
 constexpr int D_CT = 4;             // C tiles per block (grid.y: more)
 
-__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
+// two pair tiles against one C tile
+__device__ __forceinline__ void mma_f64(double (&d)[2], double (&e)[2], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};\n"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(e[0]), "+d"(e[1])
+                 : "d"(a0), "d"(a1), "d"(b));
 }
 
-// grid: (parts of the voxels, pair groups x C groups); block: G x KS warps
-template <int NCT>
+// grid: (parts of the voxels, pair groups x C groups); block: G x KS warps; D_TV voxels per tile
+template <int NCT, int D_TV>
 __global__ void __launch_bounds__(512) triplet_f64_kernel(const double *A, int n_a, const double *B, int n_b, int off_b,
                                                          const double *C, int n_c, int off_c, int n_rows, int64_t n_vox,
                                                          const int32_t *pairs, int n_pairs, const int32_t *tmap,
                                                          int n_trip, int G, int c_groups, double *partials, int vec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned used[D_PT];   // C tiles of each pair tile that hold a triplet
-    constexpr int LD = D_TV + SIMT_PAD, ML = 8 * NCT + 1;
+    constexpr int LD = D_TV + D_PAD, ML = 8 * NCT + 1;
     double *const buf = reinterpret_cast<double *>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, KS = (blockDim.x >> 5) / G, g = warp % G, ks = warp / G;
     const int p0 = (blockIdx.y / c_groups) * D_PT * 8, c0 = (blockIdx.y % c_groups) * D_CT * 8;
@@ -293,27 +295,27 @@ __global__ void __launch_bounds__(512) triplet_f64_kernel(const double *A, int n
     double acc[D_U][NCT][2];
 #pragma unroll
     for (int u = 0; u < D_U; ++u) {
-        const int pt = u * G + g;
+        const int pt = g * D_U + u;
         on[u] = pt < D_PT && pt * 8 < np ? used[pt] : 0u;
         any |= on[u];
         const int pr = min(p0 + pt * 8 + r8, n_pairs - 1);
-        ra[u] = min(max(pairs[2 * pr], 0), n_rows - 1) * LD + k4;
-        rb[u] = min(max(off_b + pairs[2 * pr + 1], 0), n_rows - 1) * LD + k4;
+        ra[u] = min(max(pairs[2 * pr], 0), n_rows - 1) * LD + 2 * k4;
+        rb[u] = min(max(off_b + pairs[2 * pr + 1], 0), n_rows - 1) * LD + 2 * k4;
 #pragma unroll
         for (int j = 0; j < NCT; ++j) acc[u][j][0] = acc[u][j][1] = 0.0;
     }
 #pragma unroll
-    for (int j = 0; j < NCT; ++j) rc[j] = min(off_c + min(c0 + 8 * j + r8, n_c - 1), n_rows - 1) * LD + k4;
+    for (int j = 0; j < NCT; ++j) rc[j] = min(off_c + min(c0 + 8 * j + r8, n_c - 1), n_rows - 1) * LD + 2 * k4;
 
     const int64_t n_tiles = (n_vox + D_TV - 1) / D_TV;
     int64_t tt = blockIdx.x;
-    if (tt < n_tiles) simt_stage<double, D_TV>(buf, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * D_TV, vec);
+    if (tt < n_tiles) simt_stage<double, D_TV, D_PAD>(buf, A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox, tt * D_TV, vec);
     int cur = 0;
     for (; tt < n_tiles; tt += gridDim.x) {
         const double *tile = buf + (cur ? n_rows * LD : 0);
         const int64_t nxt = tt + gridDim.x;
         if (nxt < n_tiles) {
-            simt_stage<double, D_TV>(buf + (cur ? 0 : n_rows * LD), A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox,
+            simt_stage<double, D_TV, D_PAD>(buf + (cur ? 0 : n_rows * LD), A, n_a, B, n_b, off_b, C, off_c, n_rows, n_vox,
                                      nxt * D_TV, vec);
             cp_async_wait1();
         } else {
@@ -322,17 +324,23 @@ __global__ void __launch_bounds__(512) triplet_f64_kernel(const double *A, int n
         __syncthreads();
         if (any) {
 #pragma unroll 2
-            for (int v = 4 * ks; v < D_TV; v += 4 * KS) {
-                double c[NCT];
+            for (int v = 8 * ks; v < D_TV; v += 8 * KS) {
+                // voxels v + 2 k4 and the next, one instruction each
+                double2 c[NCT], p[D_U];
 #pragma unroll
-                for (int j = 0; j < NCT; ++j) c[j] = tile[rc[j] + v];
+                for (int j = 0; j < NCT; ++j) c[j] = *reinterpret_cast<const double2 *>(tile + rc[j] + v);
 #pragma unroll
                 for (int u = 0; u < D_U; ++u) {
-                    const double p = tile[ra[u] + v] * tile[rb[u] + v];
-#pragma unroll
-                    for (int j = 0; j < NCT; ++j)
-                        if (on[u] >> j & 1u) mma_f64(acc[u][j], p, c[j]);
+                    const double2 a = *reinterpret_cast<const double2 *>(tile + ra[u] + v);
+                    const double2 b = *reinterpret_cast<const double2 *>(tile + rb[u] + v);
+                    p[u] = make_double2(a.x * b.x, a.y * b.y);
                 }
+#pragma unroll
+                for (int j = 0; j < NCT; ++j)
+                    if (any >> j & 1u) {
+                        mma_f64(acc[0][j], acc[1][j], p[0].x, p[1].x, c[j].x);
+                        mma_f64(acc[0][j], acc[1][j], p[0].y, p[1].y, c[j].y);
+                    }
             }
         }
         __syncthreads();
@@ -345,7 +353,7 @@ __global__ void __launch_bounds__(512) triplet_f64_kernel(const double *A, int n
 #pragma unroll
             for (int u = 0; u < D_U; ++u) {
                 if (!on[u]) continue;
-                double *row = sums + ((u * G + g) * 8 + r8) * ML + 2 * k4;
+                double *row = sums + ((g * D_U + u) * 8 + r8) * ML + 2 * k4;
 #pragma unroll
                 for (int j = 0; j < NCT; ++j)
 #pragma unroll
@@ -381,18 +389,18 @@ int simt_geometry(int64_t n_vox, int n_items, int *grid_x, int *grid_y, int *gro
     return PB_OK;
 }
 
-template <int NCT>
+template <int NCT, int D_TV>
 static cudaError_t launch_f64(const double *A, int n_a, const double *B, int n_b, int off_b, const double *C, int n_c,
                               int off_c, int n_rows, int64_t n_vox, const int32_t *pairs, int n_pairs,
                               const int32_t *tmap, int n_trip, int parts, double *partials, int vec, cudaStream_t s) {
     const int pt = std::min(D_PT, (n_pairs + 7) / 8), G = (pt + D_U - 1) / D_U;
-    int KS = 1;                       // a power of two (16 steps of 4 voxels a tile), up to 12 warps per block
+    int KS = 1;                       // a power of two (a tile has at least 8 steps of 8 voxels), up to 12 warps per block
     while (KS < 8 && 2 * KS * G <= 12) KS *= 2;
     const int c_groups = (n_c + 8 * D_CT - 1) / (8 * D_CT), p_groups = (n_pairs + 8 * D_PT - 1) / (8 * D_PT);
-    const size_t smem = std::max((size_t)2 * n_rows * (D_TV + SIMT_PAD), (size_t)pt * 8 * (8 * NCT + 1)) * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(triplet_f64_kernel<NCT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = std::max((size_t)2 * n_rows * (D_TV + D_PAD), (size_t)pt * 8 * (8 * NCT + 1)) * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(triplet_f64_kernel<NCT, D_TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    triplet_f64_kernel<NCT><<<dim3(parts, p_groups * c_groups), 32 * G * KS, smem, s>>>(
+    triplet_f64_kernel<NCT, D_TV><<<dim3(parts, p_groups * c_groups), 32 * G * KS, smem, s>>>(
         A, n_a, B, n_b, off_b, C, n_c, off_c, n_rows, n_vox, pairs, n_pairs, tmap, n_trip, G, c_groups, partials, vec);
     return cudaGetLastError();
 }
@@ -431,8 +439,11 @@ int launch_triplet_simt(int precision, const void *A, int n_a, const void *B, in
             items_dev, n_items, gp, partials, n_trip, vec);
     } else {
         const int32_t *pairs = (const int32_t *)(table + L.off_pairs), *tmap = (const int32_t *)(table + L.off_tmap);
+        // 128 voxels a tile where three blocks per SM fit: 12 bins, l = 0, on 120^3 196 against 214 us
+        const bool wide = (size_t)3 * 2 * n_rows * (128 + D_PAD) * sizeof(double) <= (size_t)220 * 1024;
         auto run = [&](auto NCT) {
-            return launch_f64<decltype(NCT)::value>((const double *)A, n_a, (const double *)B, n_b, off_b, (const double *)C,
+            constexpr int N = decltype(NCT)::value;
+            return (wide ? launch_f64<N, 128> : launch_f64<N, 64>)((const double *)A, n_a, (const double *)B, n_b, off_b, (const double *)C,
                                                     n_c, off_c, n_rows, n_vox, pairs, counts[1], tmap, n_trip, gx,
                                                     partials, vec, s);
         };

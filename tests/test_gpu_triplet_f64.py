@@ -1,5 +1,5 @@
-"""FP64 triplet contraction (matrix-instruction kernel) at the edges of its tiles: 8 pairs, 8 C maps, 64 voxels,
-256 pairs and 32 C maps per block."""
+"""FP64 triplet contraction (matrix-instruction kernel) at the edges of its tiles: 8 pairs, 8 C maps, 128 or 64
+voxels, 256 pairs and 32 C maps per block."""
 import numpy as np
 import pytest
 import torch
@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n_a,n_b,n_c,n_trip,n_vox,shared", [
     (1, 1, 1, 1, 1, False),
-    (2, 4, 8, 17, 63, False),          # one pair tile, one C tile; a ragged, unaligned voxel tile
-    (3, 3, 9, 40, 64, False),          # 9 pairs, 9 C maps: one of each past a tile
+    (2, 4, 8, 17, 127, False),          # one pair tile, one C tile; a ragged, unaligned voxel tile
+    (3, 3, 9, 40, 128, False),          # 9 pairs, 9 C maps: one of each past a tile
     (16, 17, 33, 2000, 4097, False),   # 272 pairs and 33 C maps: a second group of both, odd rows (4-byte copies)
     (12, 12, 12, 150, 30_000, True),   # one set of maps
     (20, 5, 24, 300, 100_002, False),
@@ -37,7 +37,7 @@ def test_f64_contraction(n_a, n_b, n_c, n_trip, n_vox, shared):
     for t0 in range(0, len(idx), 256):
         t = i[t0:t0 + 256]
         terms = A[t[:, 0]] * B[t[:, 1]] * C[t[:, 2]]
-        # a term's two roundings and at most 4 tiles of 64 voxels per block, 8 warps and 44 blocks in a chain,
+        # a term's two roundings and at most 256 voxels per block, 8 warps and 44 blocks in a chain,
         # as many again for the reference: fewer than 700 roundings, each of at most the sum of moduli
         bound = 0.5 * 700 * 2.0 ** -53 * terms.abs().sum(1)
         assert torch.all((out[t0:t0 + 256] - 0.5 * terms.sum(1)).abs() <= bound)
