@@ -389,12 +389,17 @@ PB_API int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_strid
                           int n_pairs, const uint8_t *pair_on, const int32_t *xs, int n_x,
                           const int32_t *x_on, const void *table, void *out, void *workspace,
                           size_t workspace_bytes, void *stream);
-/* out[p] = rfftn(X[i] X[j] - Z[i] Z[j]) (Z may be NULL) on the modes |k| < k_out for host (i, j)  */
-/* pairs of FP64 real maps: the products of the bispectrum's Q maps (bspec.py:579-597).  Same      */
-/* table, workspace and grid lengths as pb_masked_rows.                                           */
-PB_API int pb_product_rows(const pb_grid_t *g, const double *X, const double *Z, const int32_t *pairs,
-                           int n_pairs, double k_out, const void *table, void *out, void *workspace,
+/* out[p] = rfftn(X[i] Y[j] - Z[i] Z[j]) (Y NULL: X; Z may be NULL) on the modes |k| < k_out for    */
+/* host (i, j) pairs of FP64 real maps: the products of the bispectrum's Q maps (bspec.py:579-597), */
+/* a field times harmonics of the position.  Same table, workspace and grid lengths as             */
+/* pb_masked_rows.                                                                                */
+PB_API int pb_product_rows(const pb_grid_t *g, const double *X, const double *Y, const double *Z,
+                           const int32_t *pairs, int n_pairs, double k_out, const void *table, void *out, void *workspace,
                            size_t workspace_bytes, void *stream);
+/* out(k) = sum_m Y_lm(k) F[m](k) over m = 0..2l for |k| < k_out, 0 for other modes: FP64 spectra   */
+/* F[m] = F + m stride of the grid, l = 1..4 (harmonics as PB_HARMONIC; PolyBin3D/base.py:391-411). */
+PB_API int pb_harmonic_sum(const pb_grid_t *g, int l, const void *F, int64_t stride, double k_out, void *out,
+                           void *stream);
 
 #ifdef __cplusplus
 }

@@ -91,7 +91,8 @@ SIGNATURES = {
     "pb_masked_rows_workspace_size": ([_GP, _D, _I, ctypes.POINTER(_SZ)], _I),
     "pb_masked_rows": ([_GP, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _D, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _SZ, _P],
                        _I),
-    "pb_product_rows": ([_GP, _P, _P, _P, _I, _D, _P, _P, _P, _SZ, _P], _I),
+    "pb_product_rows": ([_GP, _P, _P, _P, _P, _I, _D, _P, _P, _P, _SZ, _P], _I),
+    "pb_harmonic_sum": ([_GP, _I, _P, _I64, _D, _P, _P], _I),
 }
 
 
@@ -615,14 +616,22 @@ def _rows_workspace(grid, k_out, n_maps, ws):
     return ws.get(chunk * one.value, "masked"), chunk * one.value, chunk
 
 
-def product_rows(grid, X, Z, pairs, k_out, out, table, ws):
-    """out[p] = rfftn(X[i] X[j] - Z[i] Z[j]) on |k| < k_out (other modes of out are not written);
-    X, Z: (n, n0, n1, n2) FP64 maps, Z may be None."""
+def product_rows(grid, X, Z, pairs, k_out, out, table, ws, Y=None):
+    """out[p] = rfftn(X[i] Y[j] - Z[i] Z[j]) on |k| < k_out (other modes of out are not written);
+    X, Y, Z: (n, n0, n1, n2) FP64 maps, Y None: X, Z may be None."""
     pairs = np.ascontiguousarray(np.asarray(pairs, dtype=np.int32).reshape(-1, 2))
     buf, nbytes, chunk = _rows_workspace(grid, k_out, len(pairs), ws)
-    check(load().pb_product_rows(ctypes.byref(grid), ptr(X), ptr(Z), hptr(pairs), len(pairs), float(k_out), ptr(table),
+    check(load().pb_product_rows(ctypes.byref(grid), ptr(X), ptr(Y), ptr(Z), hptr(pairs), len(pairs), float(k_out), ptr(table),
                                  ptr(out), ptr(buf), nbytes, stream_ptr()), "pb_product_rows")
     _count(3 * ((len(pairs) + chunk - 1) // chunk))
+    return out
+
+
+def harmonic_sum(grid, l, F, k_out, out):
+    """out(k) = sum_m Y_lm(k) F[m](k) on |k| < k_out, 0 elsewhere; F: (2l + 1, half) complex128."""
+    check(load().pb_harmonic_sum(ctypes.byref(grid), int(l), ptr(F), F[0].numel(), float(k_out), ptr(out),
+                                 stream_ptr()), "pb_harmonic_sum")
+    _count(1)
     return out
 
 

@@ -88,7 +88,7 @@ class PkNumerator(torch.autograd.Function):
         x_real = b.to_real(xk)
         for li in range(1, ps.Nl):
             l = li * (2 - ps.odd_l)
-            lm = b.harmonics.apply_fourier(x_real, l)
+            lm = b.harmonics.apply_fourier(x_real, l, k_out=float(ps.k_bins[-1]))
             if l % 2:
                 lm = lm * (-1j)
             nat.bin_reduce(b.grid, nat.PB_F64, nat.PB_RED_CROSS, xk, lm, 1, ps.k_bins, [(0, 0)], scale,
@@ -115,7 +115,8 @@ class PkNumerator(torch.autograd.Function):
         u = torch.empty_like(xk)
         for li in range(1, ps.Nl):
             l = li * (2 - ps.odd_l)
-            nat.binned_filter(b.grid, harm.apply_fourier(x_real, l), t, ps.k_bins, [0], coef[li:li + 1], scale=0.5)
+            h = harm.apply_fourier(x_real, l, k_out=float(ps.k_bins[-1]))
+            nat.binned_filter(b.grid, h, t, ps.k_bins, [0], coef[li:li + 1], scale=0.5)
             S.add_(t * (-1j) if l % 2 else t)
             # H^dag Theta_g x; conj(p) = i goes in before the inverse transform, where it makes
             # the odd-l spectrum Hermitian again

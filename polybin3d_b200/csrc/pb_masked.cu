@@ -211,9 +211,9 @@ extern "C" int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_s
     return PB_OK;
 }
 
-extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double *Z, const int32_t *pairs, int n_pairs,
-                               double k_out, const void *table, void *out, void *workspace, size_t workspace_bytes,
-                               void *stream) {
+extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double *Y, const double *Z,
+                               const int32_t *pairs, int n_pairs, double k_out, const void *table, void *out,
+                               void *workspace, size_t workspace_bytes, void *stream) {
     Grid G;
     int st = make_grid(g, &G);
     if (st) return st;
@@ -232,6 +232,7 @@ extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double
     p.n_x = G.n0;
     MrArgs a{};
     a.X = X;
+    a.Y = Y ? Y : X;
     a.Z = Z;
     a.table = (const double2 *)table;
     a.W = (double2 *)workspace;

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     if (on) fft::line_pass<double, -1, 2>(af, t, nt, twf, [&](int e, int) { return sm2[atf(e)]; }, stf);
 }
 
-// ---- products: forward transform along z of X_i X_j - Z_i Z_j, two rows per complex line ----------
+// ---- products: forward transform along z of X_i Y_j - Z_i Z_j, two rows per complex line ----------
 // block (threads per line, L pairs of rows); grid (products, row pairs / L): the products of a few
 // rows follow each other, so the maps' rows come from L2 after the first
 struct MrPairs {
@@ -318,8 +318,8 @@ struct MrPairs {
 template <int N>
 __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_constant__ MrParams p,
                                                                   const __grid_constant__ MrPairs pr,
-                                                                  const double2 *table, const double *X, const double *Z,
-                                                                  double2 *W) {
+                                                                  const double2 *table, const double *X, const double *Y,
+                                                                  const double *Z, double2 *W) {
     extern __shared__ __align__(16) double2 mr_smem[];
     const Grid &g = p.g;
     const fft::AxisUse<N, true> use(p.azf);
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
     const bool two = y + 1 < g.n1;
     const double h = two ? 0.5 : 1.0;
     const int64_t ra = (int64_t)x * g.n1 + y, oi = pr.i[blockIdx.x] * g.nreal, oj = pr.j[blockIdx.x] * g.nreal;
-    const double *xi = X + oi + ra * n, *xj = X + oj + ra * n;
+    const double *xi = X + oi + ra * n, *xj = Y + oj + ra * n;
     const double *zi = Z ? Z + oi + ra * n : nullptr, *zj = Z ? Z + oj + ra * n : nullptr;
     double2 *wa = W + blockIdx.x * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
     fft::line_fft<double, -1>(
@@ -391,7 +391,7 @@ struct MrShapes {
 };
 struct MrArgs {
     const double2 *src, *table;
-    const double *mask, *X, *Z;
+    const double *mask, *X, *Y, *Z;
     const int32_t *pairs, *xs, *x_on;
     const uint8_t *pair_on;
     double2 *W, *out;
@@ -427,7 +427,7 @@ cudaError_t mr_launch(MrStage stage, const MrParams &p, const MrShapes &sh, cons
             const int rows = p.g.n0 * ((p.g.n1 + 1) / 2);
             if ((e = mr_allow(mr_product_kernel<N>, sh.sz)) != cudaSuccess) return e;
             mr_product_kernel<N><<<dim3(nm, (rows + sh.Lz - 1) / sh.Lz), dim3(sh.Tz, sh.Lz), sh.sz, s>>>(
-                p, a.products, a.table, a.X, a.Z, a.W);
+                p, a.products, a.table, a.X, a.Y, a.Z, a.W);
             break;
         }
         case MR_Y_BACK:

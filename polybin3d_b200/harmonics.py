@@ -69,11 +69,20 @@ class Harmonics:
             self._grids[key] = g
         return g
 
-    def apply_fourier(self, a_real, l):
+    def apply_fourier(self, a_real, l, k_out=None):
         """sum_m Y_lm(k) rfftn(Y_lm(r) a(r)) as a half spectrum of a_real's precision: the
-        2l+1 products in one elementwise launch, one batched r2c, the m-sum on the device."""
+        2l+1 products in one elementwise launch, one batched r2c, the m-sum on the device.
+        k_out: only the modes |k| < k_out are wanted (0 elsewhere where that saves work: FP64 maps
+        whose products, transforms and sum run as one band-limited chain; l = 2 on 150 x 135 x 144 to 0.8
+        of the Nyquist frequency 311 -> 223 us)."""
         b = self.base
         yr = self._grid('r', l, a_real.dtype)
+        if k_out is not None and a_real.dtype == torch.float64 and b.rows_table() is not None:
+            b.n_FFTs_forward += yr.shape[0]
+            F = torch.empty((yr.shape[0],) + b.nhalf_shape, dtype=torch.complex128, device=b.device)
+            nat.product_rows(b.grid, a_real.contiguous(), None, [(0, m) for m in range(yr.shape[0])], k_out, F,
+                             b.rows_table(), b.ws, Y=yr)
+            return nat.harmonic_sum(b.grid, l, F, k_out, torch.empty_like(F[0]))
         yk = self._grid('k', l, a_real.dtype)
         prod = nat.elementwise(nat.PB_EW_MUL, yr, a_real.contiguous(), y_period=b.nreal)
         b.n_FFTs_forward += yr.shape[0]

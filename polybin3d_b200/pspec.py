@@ -227,7 +227,7 @@ class PSpec:
         x_real = b.to_real(xk)
         for li in range(1, Nl):
             l = li * (2 - odd)
-            lm = b.harmonics.apply_fourier(x_real, l)
+            lm = b.harmonics.apply_fourier(x_real, l, k_out=float(self.k_bins[-1]))
             if l % 2:
                 lm = lm * (-1j)
             nat.bin_reduce(b.grid, prec, nat.PB_RED_CROSS, xk, lm, 1, self.k_bins, [(0, 0)], scale,
@@ -689,7 +689,7 @@ class PSpec:
         a_real = b.to_real(a)
         for li in range(1, self.Nl):
             l = li * (2 - self.odd_l)
-            lm = b.harmonics.apply_fourier(a_real, l)
+            lm = b.harmonics.apply_fourier(a_real, l, k_out=float(self.k_bins[-1]))
             if l % 2:
                 lm = lm * (-1j)
             nat.bin_reduce(b.grid, F64, nat.PB_RED_CROSS, lm, sna, 1, self.k_bins, [(0, 0)], scale,
