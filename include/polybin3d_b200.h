@@ -396,6 +396,18 @@ PB_API int pb_masked_rows(const pb_grid_t *g, const void *src, int64_t src_strid
 PB_API int pb_product_rows(const pb_grid_t *g, const double *X, const double *Y, const double *Z,
                            const int32_t *pairs, int n_pairs, double k_out, const void *table, void *out, void *workspace,
                            size_t workspace_bytes, void *stream);
+/* The adjoint of pb_shell_synth for the legs of a gradient: for every map m of R (real, grid out_n)     */
+/*   grad[dst[m]](k) += scale[m] Theta(lo[m] <= |k| < hi[m]) L_l[m](mu) rfftn(R[m])(k)                 */
+/* (spectra of grid g, dst NULL: 0, grad_stride apart; mu of grid g).  n_maps <= 64, precision PB_F32 or   */
+/* PB_F64, l = 0..4.  PB_ERR_UNSUPPORTED where a band reaches a grid's Nyquist frequency or a length of    */
+/* out_n has no line transform.                                                                          */
+PB_API int pb_leg_gather_workspace_size(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps,
+                                        const double *hi, size_t *bytes);
+PB_API int pb_leg_gather(const pb_grid_t *g, const int32_t *out_n, int precision, const void *R, int n_maps,
+                         const double *lo, const double *hi, const int32_t *l, const double *scale,
+                         const int32_t *dst, void *grad, int64_t grad_stride, void *workspace,
+                         size_t workspace_bytes, void *stream);
+
 /* out(k) = sum_m Y_lm(k) F[m](k) over m = 0..2l for |k| < k_out, 0 for other modes: FP64 spectra   */
 /* F[m] = F + m stride of the grid, l = 1..4 (harmonics as PB_HARMONIC; PolyBin3D/base.py:391-411). */
 PB_API int pb_harmonic_sum(const pb_grid_t *g, int l, const void *F, int64_t stride, double k_out, void *out,

@@ -92,6 +92,8 @@ SIGNATURES = {
     "pb_masked_rows": ([_GP, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _D, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _SZ, _P],
                        _I),
     "pb_product_rows": ([_GP, _P, _P, _P, _P, _I, _D, _P, _P, _P, _SZ, _P], _I),
+    "pb_leg_gather_workspace_size": ([_GP, _P, _I, _I, _P, ctypes.POINTER(_SZ)], _I),
+    "pb_leg_gather": ([_GP, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I64, _P, _SZ, _P], _I),
     "pb_harmonic_sum": ([_GP, _I, _P, _I64, _D, _P, _P], _I),
 }
 
@@ -518,6 +520,38 @@ def shell_synth(grid, precision, src, out, maps, out_n, ws, w=None, src_stride=N
         _count(3)
         c0 += nc
     return out
+
+
+def leg_gather(grid, R, legs, grad, ws):
+    """grad[dst](k) += scale Theta(lo <= |k| < hi) L_l(mu) rfftn(R[m])(k) for every map m of R (n_maps, *out_n)
+    with legs[m] = (lo, hi, l, scale, dst); grad: (n, *half) complex, of R's precision.  In passes of up to 64
+    maps.  Raises NotImplementedError (before any work) when the band limits or lengths do not allow it."""
+    lib = load()
+    prec = precision_of(R.dtype)
+    on = np.ascontiguousarray(R.shape[1:], dtype=np.int32)
+    arr = np.asarray(legs, dtype=np.float64)
+    lo, hi, sc = (np.ascontiguousarray(arr[:, k]) for k in (0, 1, 3))
+    ell, dst = (np.ascontiguousarray(arr[:, k].astype(np.int32)) for k in (2, 4))
+    nbytes = ctypes.c_size_t()
+    chunks = []
+    c0 = 0
+    while c0 < len(legs):
+        nc = min(SYNTH_MAX_MAPS, len(legs) - c0)
+        while True:
+            check(lib.pb_leg_gather_workspace_size(ctypes.byref(grid), hptr(on), prec, nc, hptr(hi[c0:]),
+                                                   ctypes.byref(nbytes)), "pb_leg_gather_workspace_size")
+            if nbytes.value <= SYNTH_WS_BYTES or nc == 1:
+                break
+            nc = (nc + 1) // 2
+        chunks.append((c0, nc, nbytes.value))
+        c0 += nc
+    for c0, nc, size in chunks:
+        buf = ws.get(size, "synth")
+        check(lib.pb_leg_gather(ctypes.byref(grid), hptr(on), prec, ptr(R[c0:c0 + nc]), nc, hptr(lo[c0:]), hptr(hi[c0:]),
+                                hptr(ell[c0:]), hptr(sc[c0:]), hptr(dst[c0:]), ptr(grad), grad[0].numel(), ptr(buf),
+                                buf.numel(), stream_ptr()), "pb_leg_gather")
+        _count(4)
+    return grad
 
 
 def _shell_synth_tiled(lib, grid, precision, src, out, maps, out_n, ws, w, src_stride):

@@ -19,8 +19,8 @@ its derivative is the sum over the three legs of irfftn(Theta_leg L_leg / W FT[p
 other two maps]) times m, the same construction as the reference's Q-maps (bspec.py:600-640).
 The backward recomputes the bin-filtered maps (nothing is stored by the forward), sums, in
 real space, the products of the other two maps of every leg that ends on the same (bin,
-multipole) with pb_bilinear_maps (one map per leg instead of one per pair of maps),
-transforms those, and gathers them into one spectrum with the accumulating spectral filter.  Maps, products and their transforms live
+multipole) with pb_bilinear_block_maps (one map per leg instead of one per pair of maps),
+and transforms those into one spectrum, each through its bin filter (pb_leg_gather).  Maps, products and their transforms live
 on the dealiased map grid, which is exact for every frequency inside the bins.  With the
 local sightline the l > 0 maps are IFT(Theta_b H_l x): their legs are gathered through the bin
 filter alone, one spectrum per l, and the adjoint H_l^dag applied once per l.
@@ -214,6 +214,20 @@ class BkNumerator(torch.autograd.Function):
         return [(int(e % nks), 2 * int(e // nks)) for e in ends], plan
 
     @staticmethod
+    def _gather_whole(b, prec, R, legs, Mdims, grad_spec):
+        """The legs by whole transforms and the accumulating filter: bands or lengths that pb_leg_gather refuses."""
+        chunk = int(max(1, min(len(legs), KEY_CHUNK_BYTES // (R[0].numel() * R.element_size() * 2))))
+        for o0 in range(0, len(legs), chunk):
+            part = legs[o0:o0 + chunk]
+            FT = b.fft_r2c(R[o0:o0 + chunk])
+            b.n_FFTs_forward += len(part)
+            entries = [(n, lo, hi, l, 0, scale, 0) for n, (lo, hi, l, scale, dst) in enumerate(part)]
+            nat.spectral_filter(b.grid_of(Mdims), prec, FT, grad_spec, entries, accumulate=True,
+                                src_stride=FT[0].numel(), out_n=[int(n) for n in b.gridsize],
+                                dst=[leg[4] for leg in part])
+            del FT
+
+    @staticmethod
     def backward(ctx, g):
         _settle()
         bs = ctx.bs
@@ -241,7 +255,7 @@ class BkNumerator(torch.autograd.Function):
         if np.any(coef):
             # one real-space map per leg (bin C, multipole lc): the coefficient-weighted sum of
             # the products of the other two maps of every triplet ending on it (pb_bilinear_maps);
-            # then one forward transform per leg and one accumulating filter into the gradient.
+            # then one forward transform per leg, filtered into the gradient in its last pass.
             # The terms depend on the binning alone: the table of all triplets is kept and only its
             # coefficients change (a cotangent with zeros gets a table of its own, without their legs)
             if np.all(coef):
@@ -254,18 +268,12 @@ class BkNumerator(torch.autograd.Function):
                 outs, plan = BkNumerator._legs(bs, ab[use], coef[use], G.shape[0])
             R = plan.maps(G)
             del G
-            per_out = R[0].numel() * R.element_size() * 2
-            chunk = int(max(1, min(len(outs), KEY_CHUNK_BYTES // per_out)))
-            for o0 in range(0, len(outs), chunk):
-                o1 = min(len(outs), o0 + chunk)
-                FT = b.fft_r2c(R[o0:o1])
-                b.n_FFTs_forward += o1 - o0
-                entries = [(n - o0, ks[C], ks[C + 1], 0 if local else lc, 0, 1.0, 0)
-                           for n, (C, lc) in enumerate(outs[o0:o1], o0)]
-                dst = [lc // 2 if local else 0 for (C, lc) in outs[o0:o1]]
-                nat.spectral_filter(b.grid_of(Mdims), prec, FT, grad_spec, entries, accumulate=True,
-                                    src_stride=FT[0].numel(), out_n=[int(n) for n in b.gridsize], dst=dst)
-                del FT
+            legs = [(ks[C], ks[C + 1], 0 if local else lc, 1.0, lc // 2 if local else 0) for (C, lc) in outs]
+            try:
+                nat.leg_gather(b.grid, R, legs, grad_spec, b.ws)
+                b.n_FFTs_forward += len(outs)
+            except NotImplementedError:
+                BkNumerator._gather_whole(b, prec, R, legs, Mdims, grad_spec)
         if n_acc > 1:
             harm = b.harmonics
             R = torch.zeros((1,) + tuple(int(n) for n in b.gridsize), dtype=rd, device=b.device)

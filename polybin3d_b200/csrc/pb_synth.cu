@@ -22,7 +22,7 @@
 #include <vector>
 #include <cuda_bf16.h>
 #include "pb_common.cuh"
-#include "pb_synth_lines.cuh"
+#include "pb_legs.cuh"
 
 namespace pb {
 
@@ -809,4 +809,96 @@ extern "C" int pb_shell_synth_tiled(const pb_grid_t *g, const int32_t *out_n, in
                                     void *workspace, size_t workspace_bytes, void *stream) {
     return shell_synth(g, out_n, precision, src, src_stride, n_maps, src_idx, lo, hi, l1, l2, scale, wpow, w, out,
                        workspace, workspace_bytes, stream, true, n_factor);
+}
+
+// ---- legs of a gradient (pb_legs.cuh) ----------------------------------------------------
+static int leg_setup(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps, const double *lo,
+                     const double *hi, const int32_t *l, const double *scale, const int32_t *dst, SlParams *q,
+                     size_t *bytes) {
+    std::vector<double> zero(n_maps, 0.0), one(n_maps, 1.0);
+    std::vector<int32_t> none(n_maps, 0);
+    SynthLayout L;
+    int st = synth_layout(g, out_n, precision, n_maps, lo ? lo : zero.data(), hi, dst, l ? l : none.data(), none.data(),
+                          scale ? scale : one.data(), nullptr, 0, &L);
+    if (st) return st;
+    Grid G;
+    st = make_grid(g, &G);
+    if (st) return st;
+    const size_t c = precision == PB_F64 ? 16 : 8;
+    if (!sl_setup(G, L, c, q, bytes) ||
+        (c == 16 ? fl_z_bytes<double>(q->az, fl_z_pairs<double>(q->az)) : fl_z_bytes<float>(q->az, fl_z_pairs<float>(q->az))) >
+            (size_t)220 * 1024)
+        return fail(PB_ERR_UNSUPPORTED, "pb_leg_gather: no line transform of this length");
+    return PB_OK;
+}
+
+extern "C" int pb_leg_gather_workspace_size(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps,
+                                            const double *hi, size_t *bytes) {
+    if (!bytes || !hi) return fail(PB_ERR_INVALID, "pb_leg_gather_workspace_size: NULL argument");
+    if (n_maps < 1 || n_maps > SL_MAX_MAPS)
+        return fail(PB_ERR_INVALID, "pb_leg_gather_workspace_size: n_maps must be in [1, 64]");
+    SlParams q;
+    return leg_setup(g, out_n, precision, n_maps, nullptr, hi, nullptr, nullptr, nullptr, &q, bytes);
+}
+
+extern "C" int pb_leg_gather(const pb_grid_t *g, const int32_t *out_n, int precision, const void *R, int n_maps,
+                             const double *lo, const double *hi, const int32_t *l, const double *scale,
+                             const int32_t *dst, void *grad, int64_t grad_stride, void *workspace,
+                             size_t workspace_bytes, void *stream) {
+    if (!R || !lo || !hi || !l || !scale || !grad) return fail(PB_ERR_INVALID, "pb_leg_gather: NULL argument");
+    if (n_maps < 1 || n_maps > SL_MAX_MAPS) return fail(PB_ERR_INVALID, "pb_leg_gather: n_maps must be in [1, 64]");
+    for (int m = 0; m < n_maps; ++m)
+        if (l[m] < 0 || l[m] > 4) return fail(PB_ERR_INVALID, "pb_leg_gather: Legendre order must be in [0, 4]");
+    SlParams q;
+    size_t need;
+    int st = leg_setup(g, out_n, precision, n_maps, lo, hi, l, scale, dst, &q, &need);
+    if (st) return st;
+    if (!workspace || workspace_bytes < need) return fail(PB_ERR_WORKSPACE, "pb_leg_gather: workspace too small");
+    q.src_stride = grad_stride;
+    // shells: maps of equal edges together; where two different shells overlap, one shell of all maps
+    FlShells sh{};
+    std::vector<int> order(n_maps);
+    for (int m = 0; m < n_maps; ++m) order[m] = m;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return lo[a] != lo[b] ? lo[a] < lo[b] : hi[a] < hi[b];
+    });
+    bool apart = true;
+    double top = 0.0;
+    for (int i = 0; i < n_maps; ++i) {
+        const int m = order[i], before = i ? order[i - 1] : -1;
+        if (i == 0 || lo[m] != lo[before] || hi[m] != hi[before]) {
+            if (i && !(lo[m] >= top)) apart = false;
+            sh.first[sh.n++] = i;
+        }
+        top = std::max(top, hi[m]);
+    }
+    if (!apart) {
+        sh.n = 1;
+        for (int i = 0; i < n_maps; ++i) order[i] = i;
+    }
+    sh.first[sh.n] = n_maps;
+    for (int i = 0; i < n_maps; ++i) sh.order[i] = (int8_t)order[i];
+    const bool f64 = precision == PB_F64;
+    const size_t csize = f64 ? 16 : 8;
+    char *ws = (char *)(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
+    cudaStream_t s = as_stream(stream);
+    SlArgs a{};
+    a.src = R;
+    a.out = grad;
+    a.n_maps = n_maps;
+    a.table = ws;
+    a.W = ws + ((size_t)(q.ay.tw_len + q.az.tw_len) * csize + 255) / 256 * 256;
+    if (f64) fl_table_kernel<double><<<1, 256, 0, s>>>(q, (double2 *)a.table);
+    else fl_table_kernel<float><<<1, 256, 0, s>>>(q, (float2 *)a.table);
+    PB_LAUNCH_CHECK("pb_leg_gather(table)");
+    const int len[3] = {q.m2, q.m1, q.m0};
+    const FlStage stage[3] = {FL_Z, FL_Y, FL_X};
+    for (int i = 0; i < 3; ++i) {
+        cudaError_t e = cudaSuccess;
+        if (!fl_group_0(len[i], f64, stage[i], q, sh, a, s, &e) && !fl_group_1(len[i], f64, stage[i], q, sh, a, s, &e) &&
+            !fl_group_2(len[i], f64, stage[i], q, sh, a, s, &e) && !fl_group_3(len[i], f64, stage[i], q, sh, a, s, &e))
+            e = f64 ? fl_launch<double, 0>(stage[i], q, sh, a, s) : fl_launch<float, 0>(stage[i], q, sh, a, s);
+        if (e != cudaSuccess) return cuda_check(e, "pb_leg_gather");
+    }
+    return PB_OK;
 }
