@@ -188,6 +188,20 @@ template <typename F> __device__ __forceinline__ void with_radix(int R, F &&f) {
 }
 #undef PB_RADIX_CASE
 
+// f(radix of pass Q) for the plan AX (AxisUse below): the one radix of a compile-time length, or a switch.  (Left
+// to the optimiser, the switches took the compiler ten times as long.)
+template <int Q, typename AX, typename F> __device__ __forceinline__ void with_pass_radix(const AX &use, F &&f) {
+    if constexpr (AX::FIXED) {
+        if constexpr (Q < AX::PASSES) f(std::integral_constant<int, AX::PLAN.R[Q]>());
+    } else {
+        with_radix(use.v.R[Q], f);
+    }
+}
+template <typename AX, typename F> __device__ __forceinline__ void with_last_radix(const AX &use, F &&f) {
+    if constexpr (AX::FIXED) f(std::integral_constant<int, AX::PLAN.R[AX::PASSES - 1]>());
+    else with_radix(use.v.R[use.v.np - 1], f);
+}
+
 // ---- plan of an axis ----------------------------------------------------------------
 struct Axis {
     int n, np;            // length, passes (1 - 3)
@@ -221,11 +235,12 @@ struct Keep {
 
 // One pass (number Q) of the lines of a block.  ld(e, side) gives element e, fix(e, v) finishes it once all of
 // a butterfly's loads are on their way, st(e, v, side) takes a result; `t` of `nt` threads share the line.
-template <typename T, int SIGN, int Q, typename LD, typename ST, typename FX = Keep>
-__device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const typename cplx<T>::type *tw, LD &&ld,
+template <typename T, int SIGN, int Q, typename AX, typename LD, typename ST, typename FX = Keep>
+__device__ __forceinline__ void line_pass(const AX &use, int t, int nt, const typename cplx<T>::type *tw, LD &&ld,
                                           ST &&st, FX &&fix = FX()) {
     using C = typename cplx<T>::type;
-    with_radix(ax.R[Q], [&](auto RC) {
+    const Axis &ax = use.v;
+    with_pass_radix<Q>(use, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         const int nb = ax.nb[Q], ns = Q == 0 ? 1 : ax.ns[Q];
         for (int j = t; j < nb; j += nt) {
@@ -253,25 +268,26 @@ __device__ __forceinline__ void line_pass(const Axis &ax, int t, int nt, const t
 // All passes of a line: operands from ld, results to st, exchanges through sm (element e of this
 // line at sm[at(e)]) and, for three passes, sm2.  Every thread of the block calls it; `on`: the
 // line exists (threads of other lines only join the barriers).
-template <typename T, int SIGN, typename AT, typename LD, typename ST, typename FX = Keep>
-__device__ __forceinline__ void line_fft(const Axis &ax, int t, int nt, bool on, typename cplx<T>::type *sm,
+template <typename T, int SIGN, typename AX, typename AT, typename LD, typename ST, typename FX = Keep>
+__device__ __forceinline__ void line_fft(const AX &use, int t, int nt, bool on, typename cplx<T>::type *sm,
                                          typename cplx<T>::type *sm2, const typename cplx<T>::type *tw, AT &&at,
                                          LD &&ld, ST &&st, FX &&fix = FX()) {
     using C = typename cplx<T>::type;
+    const Axis &ax = use.v;
     if (ax.np == 1) {
-        if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, st, fix);
+        if (on) line_pass<T, SIGN, 0>(use, t, nt, tw, ld, st, fix);
         return;
     }
-    if (on) line_pass<T, SIGN, 0>(ax, t, nt, tw, ld, [&](int e, C v, int) { sm[at(e)] = v; }, fix);
+    if (on) line_pass<T, SIGN, 0>(use, t, nt, tw, ld, [&](int e, C v, int) { sm[at(e)] = v; }, fix);
     __syncthreads();
     if (ax.np == 2) {
-        if (on) line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, st);
+        if (on) line_pass<T, SIGN, 1>(use, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, st);
         return;
     }
     if (on)
-        line_pass<T, SIGN, 1>(ax, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, [&](int e, C v, int) { sm2[at(e)] = v; });
+        line_pass<T, SIGN, 1>(use, t, nt, tw, [&](int e, int) { return sm[at(e)]; }, [&](int e, C v, int) { sm2[at(e)] = v; });
     __syncthreads();
-    if (on) line_pass<T, SIGN, 2>(ax, t, nt, tw, [&](int e, int) { return sm2[at(e)]; }, st);
+    if (on) line_pass<T, SIGN, 2>(use, t, nt, tw, [&](int e, int) { return sm2[at(e)]; }, st);
 }
 
 // ---- planning -----------------------------------------------------------------------
@@ -333,6 +349,9 @@ __host__ __device__ constexpr Axis make_axis(int n, bool reversed) {
 // The axis a kernel works with: the plan of a compile-time length N (radices, strides and counts fold
 // into the code), or for N = 0 the run-time plan.
 template <int N, bool REV> struct AxisUse {
+    static constexpr bool FIXED = true;
+    static constexpr Axis PLAN = make_axis(N, REV);
+    static constexpr int PASSES = PLAN.np;
     Axis v;
     __device__ __forceinline__ AxisUse(const Axis &) {
         constexpr Axis c = make_axis(N, REV);
@@ -340,6 +359,7 @@ template <int N, bool REV> struct AxisUse {
     }
 };
 template <bool REV> struct AxisUse<0, REV> {
+    static constexpr bool FIXED = false;
     const Axis &v;
     __device__ __forceinline__ AxisUse(const Axis &a) : v(a) {}
 };

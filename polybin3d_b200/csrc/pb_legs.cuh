@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(128, SlShape<T>::ZBLOCKS)
     const int K = mp.kz_max;
     __syncthreads();   // the table
     fft::line_fft<T, -1>(
-        az, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
+        use, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
         [&](int e, int) {
             C v;
             v.x = ra[e];
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
     C *w = W + mp.w_off + (int64_t)x * p.m1 * mp.ldz + kz;
     __syncthreads();
     fft::line_fft<T, -1>(
-        ay, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+        use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
         [&](int e, int) { return sl_elem(w, e, row); },
         [&](int e, C v, int side) {
             if (fft::abs_label(e, ay.n, side) <= ry) sl_elem(w, e, row) = v;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
         const C *w = W + mp.w_off + (int64_t)iy * mp.ldz + kz;
         C *o = grad + mp.src * p.src_stride + col;
         fft::line_fft<T, -1>(
-            ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+            use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
             [&](int e, int) { return sl_elem(w, e, wx); },
             [&](int e, C v, int side) {
                 const int ka = fft::abs_label(e, ax.n, side);

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_x_kernel(const __grid_c
     const int xs = g.n1 * g.nh2 * (int)sizeof(double2), wx = g.n1 * p.ldz * (int)sizeof(double2);
     double2 *w = W + blockIdx.y * p.w_map + (int64_t)iy * p.ldz + kz;
     fft::line_fft<double, 1>(
-        ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+        use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
         [&](int e, int side) {
             double2 v = make_double2(0.0, 0.0);
             const int kx = fft::abs_label(e, ax.n, side);
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_y_kernel(const __grid_c
     const bool real = kz == 0 || 2 * kz == g.n2;  // planes whose c2r reads real parts only
     if (SIGN > 0) {
         fft::line_fft<double, 1>(
-            ay, threadIdx.y, NT, on, sm, sm2, tw, at,
+            use, threadIdx.y, NT, on, sm, sm2, tw, at,
             [&](int e, int side) { return fft::abs_label(e, ay.n, side) <= ry ? elem(w, e, row) : zero; },
             [&](int y, double2 v, int) {
                 if (real) v.y = 0.0;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_y_kernel(const __grid_c
         const bool shuffle = L == 16 && (ay.nb[0] & 1) == 0 && (NT & 1) == 0 && (ay.n & 1) == 0;
         const unsigned lanes = __ballot_sync(0xffffffffu, on);
         fft::line_fft<double, -1>(
-            ay, threadIdx.y, NT, on, sm, sm2, tw, at,
+            use, threadIdx.y, NT, on, sm, sm2, tw, at,
             [&](int y, int) { return act[y >> 1] ? elem(w, y, row) : zero; },
             [&](int e, double2 v, int side) {
                 if (fft::abs_label(e, ay.n, side) <= ry) elem(w, e, row) = v;
@@ -251,19 +251,19 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     auto atf = [&](int e) { return fft::row_at(af, e); };
     double2 *in = sm;
     if (ai.np >= 2) {
-        if (on) fft::line_pass<double, 1, 0>(ai, t, nt, twi, ldf, [&](int e, double2 v, int) { sm[ati(e)] = v; });
+        if (on) fft::line_pass<double, 1, 0>(use_i, t, nt, twi, ldf, [&](int e, double2 v, int) { sm[ati(e)] = v; });
         __syncthreads();
     }
     if (ai.np == 3) {
         if (on)
-            fft::line_pass<double, 1, 1>(ai, t, nt, twi, [&](int e, int) { return sm[ati(e)]; },
+            fft::line_pass<double, 1, 1>(use_i, t, nt, twi, [&](int e, int) { return sm[ati(e)]; },
                                          [&](int e, double2 v, int) { sm2[ati(e)] = v; });
         __syncthreads();
         in = sm2;
     }
     // last inverse pass, mask and first forward pass in registers: thread t holds z = t + r n / R
     const int q = ai.np - 1, nb = ai.nb[q];
-    fft::with_radix(ai.R[q], [&](auto RC) {
+    fft::with_last_radix(use_i, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         double2 v[R];
         const bool act = on && t < nb;
@@ -299,14 +299,14 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
     if (af.np == 1) return;
     __syncthreads();
     if (af.np == 2) {
-        if (on) fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e, int) { return sm[atf(e)]; }, stf);
+        if (on) fft::line_pass<double, -1, 1>(use_f, t, nt, twf, [&](int e, int) { return sm[atf(e)]; }, stf);
         return;
     }
     if (on)
-        fft::line_pass<double, -1, 1>(af, t, nt, twf, [&](int e, int) { return sm[atf(e)]; },
+        fft::line_pass<double, -1, 1>(use_f, t, nt, twf, [&](int e, int) { return sm[atf(e)]; },
                                       [&](int e, double2 v, int) { sm2[atf(e)] = v; });
     __syncthreads();
-    if (on) fft::line_pass<double, -1, 2>(af, t, nt, twf, [&](int e, int) { return sm2[atf(e)]; }, stf);
+    if (on) fft::line_pass<double, -1, 2>(use_f, t, nt, twf, [&](int e, int) { return sm2[atf(e)]; }, stf);
 }
 
 // ---- products: forward transform along z of X_i Y_j - Z_i Z_j, two rows per complex line ----------
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
     const double *zi = Z ? Z + oi + ra * n : nullptr, *zj = Z ? Z + oj + ra * n : nullptr;
     double2 *wa = W + blockIdx.x * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
     fft::line_fft<double, -1>(
-        ax, threadIdx.x, N ? ax.nb[0] : (int)blockDim.x, on, sm, sm2, tw, [&](int e) { return fft::row_at(ax, e); },
+        use, threadIdx.x, N ? ax.nb[0] : (int)blockDim.x, on, sm, sm2, tw, [&](int e) { return fft::row_at(ax, e); },
         [&](int e, int) {
             double2 v = make_double2(xi[e] * xj[e], 0.0);
             if (Z) v.x -= zi[e] * zj[e];
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(MR_LINE_THREADS, 5) mr_out_kernel(const __grid
     double2 *o = out + blockIdx.y * g.nhalf + (int64_t)iy * g.nh2 + kz;
     const int rx = index_radius(p.out2, (ky * g.kf1) * (ky * g.kf1) + (kz * g.kf2) * (kz * g.kf2), g.kf0);
     fft::line_fft<double, -1>(
-        ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+        use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
         [&](int x, int) { return !x_on || x_on[x] ? elem(w, x, wx) : make_double2(0.0, 0.0); },
         [&](int e, double2 v, int side) {
             if (fft::abs_label(e, ax.n, side) <= rx) elem(o, e, ox) = v;

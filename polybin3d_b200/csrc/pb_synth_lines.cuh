@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
     const int wx = p.m1 * mp.ldz * (int)sizeof(C);
     C *o = W + mp.w_off + (int64_t)iy * mp.ldz + kz;
     fft::line_fft<T, 1>(
-        ax, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+        use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
         [&](int e, int side) {
             C v;
             v.x = v.y = (T)0;
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(SlShape<T>::THREADS, SlShape<T>::BLOCKS)
     const int ry = sl_ky_radius(p.g, mp.hi2, kz);
     C *w = W + mp.w_off + (int64_t)x * p.m1 * mp.ldz + kz;
     fft::line_fft<T, 1>(
-        ay, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
+        use, threadIdx.y, NT, on, sm, sm2, tw, [&](int e) { return e * L + line; },
         [&](int e, int side) {
             C v;
             v.x = v.y = (T)0;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(128, SlShape<T>::ZBLOCKS)
     T *oa = out + ((int64_t)blockIdx.y * pairs + (on ? pair : 0)) * 2 * n, *ob = oa + n;
     const int K = mp.kz_max;
     fft::line_fft<T, 1>(
-        az, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
+        use, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
         [&](int e, int side) {
             const bool up = side ? side > 0 : 2 * e > n;
             const int kz = up ? n - e : e;
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256, 2)
     const float2 *wa = W + mp.w_off + (on ? 2 * pair * mp.ldz : 0), *wb = wa + mp.ldz;
     const int K = mp.kz_max;
     fft::line_fft<float, 1>(
-        az, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
+        use, threadIdx.x, nt, on, sm, sm2, tw, [&](int e) { return fft::row_at(az, e); },
         [&](int e, int side) {
             const bool up = side ? side > 0 : 2 * e > n;
             const int kz = up ? n - e : e;
