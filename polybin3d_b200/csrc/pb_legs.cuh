@@ -203,6 +203,8 @@ cudaError_t fl_launch(FlStage stage, const SlParams &p, const FlShells &sh, cons
         switch (n) { SL_GROUP_##K(FL_CASE) } \
         return false;                    \
     }
+cudaError_t fl_any_f64(FlStage stage, const SlParams &p, const FlShells &sh, const SlArgs &a, cudaStream_t s);
+cudaError_t fl_any_f32(FlStage stage, const SlParams &p, const FlShells &sh, const SlArgs &a, cudaStream_t s);
 bool fl_group_0(FL_ARGS);
 bool fl_group_1(FL_ARGS);
 bool fl_group_2(FL_ARGS);

@@ -697,7 +697,8 @@ static int sl_run(SlTypes ty, const SlParams &q, int n_maps, size_t csize, const
         cudaError_t e = cudaSuccess;
         if (!sl_group_0(len[i], ty, stage[i], q, a, s, &e) && !sl_group_1(len[i], ty, stage[i], q, a, s, &e) &&
             !sl_group_2(len[i], ty, stage[i], q, a, s, &e) && !sl_group_3(len[i], ty, stage[i], q, a, s, &e))
-            e = sl_dispatch<0>(ty, stage[i], q, a, s);
+            e = ty == SL_F64 ? sl_any_f64(stage[i], q, a, s)
+                : ty == SL_F32 || stage[i] != SL_X ? sl_any_f32(stage[i], q, a, s) : sl_any_f32_src64(stage[i], q, a, s);
         if (e != cudaSuccess) return cuda_check(e, where[i]);
     }
     return PB_OK;
@@ -897,7 +898,7 @@ extern "C" int pb_leg_gather(const pb_grid_t *g, const int32_t *out_n, int preci
         cudaError_t e = cudaSuccess;
         if (!fl_group_0(len[i], f64, stage[i], q, sh, a, s, &e) && !fl_group_1(len[i], f64, stage[i], q, sh, a, s, &e) &&
             !fl_group_2(len[i], f64, stage[i], q, sh, a, s, &e) && !fl_group_3(len[i], f64, stage[i], q, sh, a, s, &e))
-            e = f64 ? fl_launch<double, 0>(stage[i], q, sh, a, s) : fl_launch<float, 0>(stage[i], q, sh, a, s);
+            e = f64 ? fl_any_f64(stage[i], q, sh, a, s) : fl_any_f32(stage[i], q, sh, a, s);
         if (e != cudaSuccess) return cuda_check(e, "pb_leg_gather");
     }
     return PB_OK;

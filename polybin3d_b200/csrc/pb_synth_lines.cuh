@@ -379,6 +379,17 @@ template <typename K> static cudaError_t sl_allow(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+template <typename T, typename S, int N> cudaError_t sl_launch_x(const SlParams &p, const SlArgs &a, cudaStream_t s) {
+    using C = typename cplx<T>::type;
+    const int L = sl_lines<T>(p.ax), t = sl_threads<T>(p.ax), runs = p.kz_top / L + 1;
+    const size_t smem = sl_line_bytes<T>(p.ax, L);
+    const cudaError_t e = sl_allow(sl_x_kernel<T, S, N>, smem);
+    if (e != cudaSuccess) return e;
+    sl_x_kernel<T, S, N><<<dim3((unsigned)(p.m1 * runs), a.n_maps), dim3(L, t), smem, s>>>(
+        p, (const S *)a.src, (const T *)a.w, (C *)a.table, (C *)a.W);
+    return cudaGetLastError();
+}
+
 // one pass with the kernels of length N (0: the run-time plan)
 template <typename T, typename S, int N>
 cudaError_t sl_launch(SlStage stage, const SlParams &p, const SlArgs &a, cudaStream_t s) {
@@ -406,17 +417,11 @@ cudaError_t sl_launch(SlStage stage, const SlParams &p, const SlArgs &a, cudaStr
         }
         return cudaErrorInvalidValue;
     }
-    const fft::Axis &ax = stage == SL_X ? p.ax : p.ay;
-    const int L = sl_lines<T>(ax), t = sl_threads<T>(ax), runs = p.kz_top / L + 1;
-    const size_t smem = sl_line_bytes<T>(ax, L);
-    if (stage == SL_X) {
-        if ((e = sl_allow(sl_x_kernel<T, S, N>, smem)) != cudaSuccess) return e;
-        sl_x_kernel<T, S, N><<<dim3((unsigned)(p.m1 * runs), a.n_maps), dim3(L, t), smem, s>>>(
-            p, (const S *)a.src, (const T *)a.w, (C *)a.table, (C *)a.W);
-    } else {
-        if ((e = sl_allow(sl_y_kernel<T, N>, smem)) != cudaSuccess) return e;
-        sl_y_kernel<T, N><<<dim3((unsigned)(p.m0 * runs), a.n_maps), dim3(L, t), smem, s>>>(p, (const C *)a.table, (C *)a.W);
-    }
+    if (stage == SL_X) return sl_launch_x<T, S, N>(p, a, s);
+    const int L = sl_lines<T>(p.ay), t = sl_threads<T>(p.ay), runs = p.kz_top / L + 1;
+    const size_t smem = sl_line_bytes<T>(p.ay, L);
+    if ((e = sl_allow(sl_y_kernel<T, N>, smem)) != cudaSuccess) return e;
+    sl_y_kernel<T, N><<<dim3((unsigned)(p.m0 * runs), a.n_maps), dim3(L, t), smem, s>>>(p, (const C *)a.table, (C *)a.W);
     return cudaGetLastError();
 }
 
@@ -442,6 +447,11 @@ cudaError_t sl_dispatch(SlTypes ty, SlStage stage, const SlParams &p, const SlAr
         switch (n) { SL_GROUP_##K(SL_CASE) } \
         return false;                    \
     }
+// the run-time plan, any other length (a file per type: each takes the compiler a minute or two)
+#define SL_ANY_ARGS SlStage stage, const SlParams &p, const SlArgs &a, cudaStream_t s
+cudaError_t sl_any_f64(SL_ANY_ARGS);
+cudaError_t sl_any_f32(SL_ANY_ARGS);
+cudaError_t sl_any_f32_src64(SL_ANY_ARGS);
 bool sl_group_0(SL_ARGS);
 bool sl_group_1(SL_ARGS);
 bool sl_group_2(SL_ARGS);
