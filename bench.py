@@ -414,16 +414,11 @@ def run_ours(args, rank, world, local):
         print(json.dumps(line))
 
 
-def fisher_alg_bytes(kind, N, n_bins):
-    """Compulsory HBM bytes of one FP64 Monte Carlo realisation, each kernel reading its
-    inputs and writing its outputs once and each 3D FFT counted as one read + one write
-    (N^3 voxels of 8 B, N^3/2 half modes of 16 B).
-    Pk, per Fisher row: Q spectrum write (8 N^3), c2r (8 + 8), mask product (24), r2c (8 + 8),
-    CROSS reduction read (8): 72 N^3.
-    Bk, per bin: three accumulating leg passes (3 x 16 N^3), the S^-1 P mask filter of its
-    Q (c2r 16, mask 24, r2c 16) and its rows' read (8): 112 N^3."""
-    per = 72 if kind == "pk" else 112
-    return float(per) * N ** 3 * n_bins
+def fisher_alg_bytes(N, n_bins):
+    """Compulsory HBM bytes of one FP64 Monte Carlo realisation: the half spectrum of every row
+    (N^3/2 modes of 16 B) written once by its chain and read once by the sums, 16 N^3 a row.
+    (Filter, transforms and mask of a row are one chain; what its passes exchange is not counted.)"""
+    return 16.0 * N ** 3 * n_bins
 
 
 def fisher_cpu_baseline(cfg, kind):
@@ -549,7 +544,7 @@ def fisher_measure(name, steps, warmup, rank, world, local, with_cpu):
         except Exception:
             pass
         hbm = float(peaks.get("hbm_gbs", 6650.0))
-        alg = fisher_alg_bytes(kind, N, est.N_bins)
+        alg = fisher_alg_bytes(N, est.N_bins)
         achieved = alg / (ms / 1000.0 / (steps * B)) / 1e9
         fields = 1 if kind == "pk" else 2
         rec = {"metric": cfg["metric"], "value": value, "unit": "sims/s", "n_gpus": world, "steps": steps,
