@@ -89,6 +89,13 @@ static int mr_setup(const Grid &G, double k_out, MrParams *pp, MrShapes *sh) {
     sh->sz = zbytes(Lz);
     if (Tz * Lz > MR_THREADS || std::max(sh->sz, std::max(sh->sx, sh->sy)) > (size_t)MR_SMEM)
         return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: lines too long");
+    // every stage of a full chunk over all planes and rows can be launched
+    p.n_x = G.n0;
+    p.n_pairs = G.n0 * ((G.n1 + 1) / 2);
+    for (MrStage stage : {MR_X, MR_Y, MR_Z, MR_PRODUCT, MR_Y_BACK, MR_X_BACK}) {
+        const MrGrid n = mr_grid(stage, p, *sh, MR_MAX_MAPS);
+        if (n.x > 2147483647 || n.y > 65535) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: too many rows");
+    }
     return PB_OK;
 }
 
@@ -121,6 +128,10 @@ extern "C" int pb_masked_rows_table(const pb_grid_t *g, double *table, size_t *b
     if (!bytes) return fail(PB_ERR_INVALID, "pb_masked_rows_table: bytes is NULL");
     MrLayout L;
     st = mr_layout(G, &L);
+    if (st) return st;
+    MrParams p;
+    MrShapes sh;
+    st = mr_setup(G, G.kf2 * G.nh2, &p, &sh);  // what has a table is taken whatever the band
     if (st) return st;
     const size_t need = std::max<size_t>(16, (size_t)L.tw_len * 16);
     if (table) {
@@ -229,7 +240,6 @@ extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double
     const int chunk = (int)std::min<size_t>(MR_MAX_MAPS, workspace_bytes / per);
     if (!workspace || chunk < 1) return fail(PB_ERR_WORKSPACE, "pb_product_rows: workspace too small");
     cudaStream_t s = as_stream(stream);
-    p.n_x = G.n0;
     MrArgs a{};
     a.X = X;
     a.Y = Y ? Y : X;
@@ -237,7 +247,7 @@ extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double
     a.table = (const double2 *)table;
     a.W = (double2 *)workspace;
     for (int m0 = 0; m0 < n_pairs; m0 += chunk) {
-        a.maps = std::min(chunk, n_pairs - m0);
+        p.n_prod = a.maps = std::min(chunk, n_pairs - m0);
         for (int m = 0; m < a.maps; ++m) {
             a.products.i[m] = (int16_t)pairs[2 * (m0 + m)];
             a.products.j[m] = (int16_t)pairs[2 * (m0 + m) + 1];
