@@ -400,7 +400,7 @@ PB_API int pb_product_rows(const pb_grid_t *g, const double *X, const double *Y,
 /*   grad[dst[m]](k) += scale[m] Theta(lo[m] <= |k| < hi[m]) L_l[m](mu) rfftn(R[m])(k)                 */
 /* (spectra of grid g, dst NULL: 0, grad_stride apart; mu of grid g).  n_maps <= 64, precision PB_F32 or   */
 /* PB_F64, l = 0..4.  PB_ERR_UNSUPPORTED where a band reaches a grid's Nyquist frequency or a length of    */
-/* out_n has no line transform.                                                                          */
+/* out_n is odd or has no line transform.                                                                */
 PB_API int pb_leg_gather_workspace_size(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps,
                                         const double *hi, size_t *bytes);
 PB_API int pb_leg_gather(const pb_grid_t *g, const int32_t *out_n, int precision, const void *R, int n_maps,

@@ -816,6 +816,9 @@ extern "C" int pb_shell_synth_tiled(const pb_grid_t *g, const int32_t *out_n, in
 static int leg_setup(const pb_grid_t *g, const int32_t *out_n, int precision, int n_maps, const double *lo,
                      const double *hi, const int32_t *l, const double *scale, const int32_t *dst, SlParams *q,
                      size_t *bytes) {
+    // real maps of odd lengths come from whole transforms (the synthesis makes none): so do their legs
+    for (int i = 0; out_n && i < 3; ++i)
+        if (out_n[i] & 1) return fail(PB_ERR_UNSUPPORTED, "pb_leg_gather: output dims must be even");
     std::vector<double> zero(n_maps, 0.0), one(n_maps, 1.0);
     std::vector<int32_t> none(n_maps, 0);
     SynthLayout L;
