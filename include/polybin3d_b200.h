@@ -272,11 +272,10 @@ PB_API int pb_bilinear_maps(int precision, int64_t n_vox, const void *G, int n_g
                             int n_out, void *out, void *stream);
 /* The same maps with four consecutive outputs per pass over the terms (faster where             */
 /* neighbouring outputs share their (i, j) pairs).  Table: int32 offsets[ceil(n_out / 4) + 1]     */
-/* padded to 16 bytes, then 64-byte records: code (j | i << 8 | first of an i-group << 16),       */
-/* 12 bytes of padding, four FP32 and the four FP64 coefficients of the outputs.  slot            */
-/* (optional, [n_terms]): 4 record + output % 4 of every term, for a caller that refills the       */
-/* coefficients of a table it keeps; duplicates share a slot and add up.  A block uses a map for all */
-/* four of its outputs: a NaN or an infinity of that map reaches them all.                        */
+/* padded to 16 bytes, then 64-byte records: code (j | i << 8 | first of an i-group << 16 | outputs  */
+/* with this term << 17), 12 bytes of padding, four FP32 and the four FP64 coefficients of the outputs. */
+/* slot (optional, [n_terms]): 4 record + output % 4 of every term, for a caller that refills the     */
+/* coefficients of a table it keeps; duplicates share a slot and add up.                              */
 PB_API int pb_bilinear_block_plan(int n_g, int n_out, const int32_t *o, const int32_t *i, const int32_t *j,
                                   const double *c, int n_terms, void *table, size_t *table_bytes,
                                   int32_t *n_table, int32_t *slot);

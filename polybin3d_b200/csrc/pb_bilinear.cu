@@ -94,13 +94,16 @@ __global__ void __launch_bounds__(BL_THREADS, 4) bilinear_kernel(const T *G, int
 // other in (multipole, bin) order hold mostly the same pairs: 2752 terms of 16 bins, l = 0, 2 make 912
 // records, 75 % of their coefficients non-zero.  Records go through shared memory 32 at a time: with 200
 // KB of maps per SM there is little L1 left, and a record that misses it costs the warp an L2
-// round trip (2850 us).  Measured on a B200, those terms of 32 maps on 192^3: FP32 1980 us against
+// round trip (2850 us).  A zero coefficient stands for a term that is not there: harmless for finite values, so a tile
+// that holds a NaN or an infinity (one FMA per staged value finds it) takes its records one by one, each into the outputs
+// that its code names, and such a value reaches only the outputs that use its map.  Measured on a B200, those terms of 32 maps on 192^3: FP32 1980 us against
 // 3170 us one output at a time, FP64 3960 against 8500 us; ncu: 71 % of the shared-memory and
 // 65 % of the issue rate.  Packed FP32 pairs (fma.rn.f32x2) were slower, 2460 us.
 // ------------------------------------------------------------------------------------
 constexpr int BB_OUT = 4;
 
-// one (i, j) of a block of outputs: code as BlTerm's, the coefficients in FP32 and FP64 (0: no such term)
+// one (i, j) of a block of outputs: code as BlTerm's with the outputs that have the term in bits 17 - 20, the
+// coefficients in FP32 and FP64 (0: no such term)
 struct BbTerm {
     uint32_t code, pad[3];
     float cf[BB_OUT];
@@ -140,18 +143,31 @@ __global__ void __launch_bounds__(BL_THREADS, BB_OCC) bilinear_block_kernel(cons
         const bool whole = vec && v0 + tile <= n_vox;   // rows 16-byte aligned and inside the map
         __syncthreads();
         if (threadIdx.x == 0) next = nw;
+        T odd[N];   // 0, or NaN once a value is not finite
+#pragma unroll
+        for (int u = 0; u < N; ++u) odd[u] = (T)0;
         for (int m = warp; m < n_g; m += nw) {
             const T *src = G + (int64_t)m * n_vox + v0;
             T *dst = sg + m * tile;
             if (whole) {
 #pragma unroll 4
-                for (int e = lane * N; e < tile; e += 32 * N)
-                    *reinterpret_cast<Pack *>(dst + e) = *reinterpret_cast<const Pack *>(src + e);
+                for (int e = lane * N; e < tile; e += 32 * N) {
+                    const Pack g = *reinterpret_cast<const Pack *>(src + e);
+                    *reinterpret_cast<Pack *>(dst + e) = g;
+#pragma unroll
+                    for (int u = 0; u < N; ++u) odd[u] += (T)0 * g.v[u];
+                }
             } else {
-                for (int e = lane; e < tile; e += 32) dst[e] = v0 + e < n_vox ? src[e] : (T)0;
+                for (int e = lane; e < tile; e += 32) {
+                    const T g = v0 + e < n_vox ? src[e] : (T)0;
+                    dst[e] = g;
+                    odd[0] += (T)0 * g;
+                }
             }
         }
-        __syncthreads();
+#pragma unroll
+        for (int u = 1; u < N; ++u) odd[0] += odd[u];
+        const bool finite = !__syncthreads_or(odd[0] != (T)0);
         int unit = warp;
         while (unit < n_span * n_blk) {
             const int blk = n_blk - 1 - unit / n_span, at = (unit % n_span) * SPAN + lane * N;
@@ -171,6 +187,44 @@ __global__ void __launch_bounds__(BL_THREADS, BB_OCC) bilinear_block_kernel(cons
                         s[k][u] = (T)0;
                     }
             };
+            if (!finite) {
+                unsigned group = 0;   // outputs with a term of the current i
+                auto close_used = [&]() {
+#pragma unroll
+                    for (int k = 0; k < BB_OUT; ++k)
+                        if (group >> k & 1u) {
+#pragma unroll
+                            for (int u = 0; u < V; ++u) {
+                                acc[k][u] += gi[u] * s[k][u];
+                                s[k][u] = (T)0;
+                            }
+                        }
+                    group = 0;
+                };
+#pragma unroll 1
+                for (int q = offs[blk]; q < offs[blk + 1]; ++q) {
+                    const BbTerm &t = rec[q];
+                    const uint32_t now = t.code, used = now >> 17;
+                    if (now & (1u << 16)) {
+                        close_used();
+#pragma unroll
+                        for (int p = 0; p < BB_P; ++p)
+#pragma unroll
+                            for (int u = 0; u < N; ++u) gi[p * N + u] = sg[((now >> 8) & 0xFF) * tile + at + p * 32 * N + u];
+                    }
+                    group |= used;
+#pragma unroll
+                    for (int p = 0; p < BB_P; ++p)
+#pragma unroll
+                        for (int u = 0; u < N; ++u) {
+                            const T g = sg[(now & 0xFF) * tile + at + p * 32 * N + u];
+#pragma unroll
+                            for (int k = 0; k < BB_OUT; ++k)
+                                if (used >> k & 1u) s[k][p * N + u] += bb_coef<T>(t, k) * g;
+                        }
+                }
+                close_used();
+            } else {
             // 32 records at a time: lane i fetches record i of the next 32 while the warp works on these
             const int r1 = offs[blk + 1];
             int r = offs[blk];
@@ -215,6 +269,7 @@ __global__ void __launch_bounds__(BL_THREADS, BB_OCC) bilinear_block_kernel(cons
                 }
             }
             close();
+            }
 #pragma unroll
             for (int k = 0; k < BB_OUT; ++k) {
                 const int o = blk * BB_OUT + k;
@@ -390,6 +445,7 @@ extern "C" int pb_bilinear_block_plan(int n_g, int n_out, const int32_t *o, cons
             ++offs[(key >> 16) + 1];
         }
         const int q = o[t[k].second] % BB_OUT;
+        rec[r].code |= 1u << (17 + q);
         rec[r].c[q] += c[t[k].second];
         if (slot) slot[t[k].second] = BB_OUT * r + q;
     }
