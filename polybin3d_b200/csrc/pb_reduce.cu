@@ -570,11 +570,11 @@ __global__ void __launch_bounds__(256) binred_lanes_kernel(Grid g, const typenam
 //    sqrt(t_b) >= edge_b (sqrt is monotone and correctly rounded on both sides, so membership
 //    is bit for bit that of |k|), and s grows along a lane's walk over ky, so the search is
 //    one comparison with the next threshold;
-//  * the Legendre products are polynomials in mu^2 = kz^2 / s: a lane sums f mu^(2m) and the
-//    block turns its moments into the requested products.
+//  * the Legendre products are polynomials in mu^2 = kz^2 / s, evaluated by Horner's rule (sums of f mu^(2m), turned into
+//    the products once per block, made an infinite mode NaN: inf - inf, and inf mu^2 at kz = 0).
 // A unit is 32 consecutive kz of a kx plane (coalesced reads) times a run of ky that one warp
 // walks; each lane keeps the sums of its current bin in registers and adds them to its own slot
-// of the warp's shared-memory window [bin - first bin of the unit][moment][lane] when the bin
+// of the warp's shared-memory window [bin - first bin of the unit][product][lane] when the bin
 // changes; the window is summed over the lanes into the warp's totals after the unit.  No
 // atomics, a fixed order.  The window holds the bins that a unit can meet (a bound from the
 // bin widths), so that 16 warps fit on an SM; with all 40 bins' slots only 6 did (483 us).
@@ -582,6 +582,9 @@ __global__ void __launch_bounds__(256) binred_lanes_kernel(Grid g, const typenam
 // for the mode-tile kernel (256^3 FP32: 42 against 310 us; 128^3 FP64: below 20 against 50 us).
 // ------------------------------------------------------------------------------------
 constexpr int FOLD_MAX_M = 5;           // mu^0 .. mu^8
+// Kernels are compiled for NE products of degree DEG in mu^2; one that starts at l = 0, 2, 4, product e of degree e at
+// most, skips the zero coefficients above it
+__host__ __device__ constexpr int fold_degree(int ne, int deg, int e) { return ne == deg + 1 && e < deg ? e : deg; }
 constexpr int FOLD_SMEM = 100 * 1024;   // accumulators per block, two blocks per SM
 
 struct FoldParams {
@@ -607,16 +610,16 @@ __device__ __forceinline__ double fold_value(const typename cplx<T>::type *a, co
     return v * v;
 }
 
-template <typename T, int MODE, int NM>
+template <typename T, int MODE, int NE, int DEG>
 __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typename cplx<T>::type *a,
                                                             const typename cplx<T>::type *b, const T *w,
                                                             int64_t row_stride, const __grid_constant__ FoldParams p,
                                                             double *partials) {
     constexpr int U = sizeof(T) == 4 ? 4 : 2;  // ky steps whose values are in flight together
-    extern __shared__ __align__(16) double fold_smem[];  // [warp][window bin][moment][32], [warp][bin][moment]
+    extern __shared__ __align__(16) double fold_smem[];  // [warp][window bin][product][32], [warp][bin][product]
     __shared__ double t[PB_RED_MAX_BINS + 2];
     const int nk = p.nk, nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per = nk * NM, wper = p.wb * NM;
+    const int per = nk * NE, wper = p.wb * NE;
     double *const win = fold_smem + (size_t)warp * wper * 32;
     double *const totals = fold_smem + (size_t)nw * wper * 32;
     double *const tot = totals + (size_t)warp * per;
@@ -651,9 +654,9 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
             while (t[base + 1] <= sb) ++base;
         }
         int bin = base - 1;      // current bin (base - 1: none yet); t[bin + 1] is the next threshold
-        double next = t[base], acc[NM];
+        double next = t[base], acc[NE];
 #pragma unroll
-        for (int m = 0; m < NM; ++m) acc[m] = 0.0;
+        for (int e = 0; e < NE; ++e) acc[e] = 0.0;
         for (int j0 = jb; j0 < j1; j0 += U) {
             double s[U], f[U];
             bool any = false;
@@ -684,10 +687,10 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
                 if (s[q] >= next) {
                     if (bin >= base) {
 #pragma unroll
-                        for (int m = 0; m < NM; ++m) win[((bin - base) * NM + m) * 32 + lane] += acc[m];
+                        for (int e = 0; e < NE; ++e) win[((bin - base) * NE + e) * 32 + lane] += acc[e];
                     }
 #pragma unroll
-                    for (int m = 0; m < NM; ++m) acc[m] = 0.0;
+                    for (int e = 0; e < NE; ++e) acc[e] = 0.0;
                     do {
                         ++bin;
                         next = t[bin + 1];
@@ -698,32 +701,33 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
                         next = t[nk + 1];
                     }
                 }
-                double x = f[q] * deg;
-                acc[0] += x;
-                if (NM > 1) {
-                    const double mu2 = s[q] > 0.0 ? kz2 / s[q] : 0.0;
+                const double x = f[q] * deg, mu2 = DEG > 0 && s[q] > 0.0 ? kz2 / s[q] : 0.0;
 #pragma unroll
-                    for (int m = 1; m < NM; ++m) {
-                        x *= mu2;
-                        acc[m] += x;
-                    }
+                for (int e = 0; e < NE; ++e) {
+                    constexpr int top = DEG;
+                    const int d = fold_degree(NE, DEG, e);
+                    double w = p.coef[e][d];
+#pragma unroll
+                    for (int m = top - 1; m >= 0; --m)
+                        if (m < d) w = w * mu2 + p.coef[e][m];
+                    acc[e] += x * w;
                 }
             }
         }
         if (bin >= base) {
 #pragma unroll
-            for (int m = 0; m < NM; ++m) win[((bin - base) * NM + m) * 32 + lane] += acc[m];
+            for (int e = 0; e < NE; ++e) win[((bin - base) * NE + e) * 32 + lane] += acc[e];
         }
         __syncwarp();
-        // a lane sums one (bin, moment) over the 32 slots (rotated: no bank conflicts), clearing them
-        const int rows = min(p.wb, nk - base) * NM;
+        // a lane sums one (bin, product) over the 32 slots (rotated: no bank conflicts), clearing them
+        const int rows = min(p.wb, nk - base) * NE;
         for (int q = lane; q < rows; q += 32) {
             double x = 0.0;
 #pragma unroll 16
             for (int k = 0; k < 32; ++k) x += win[q * 32 + ((lane + k) & 31)];
 #pragma unroll 16
             for (int k = 0; k < 32; ++k) win[q * 32 + ((lane + k) & 31)] = 0.0;
-            tot[base * NM + q] += x;
+            tot[base * NE + q] += x;
         }
         __syncwarp();
     }
@@ -737,11 +741,7 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
     double *dst = partials + ((int64_t)row * gridDim.x + blockIdx.x) * (p.n_ell * nk);
     for (int i = threadIdx.x; i < p.n_ell * nk; i += blockDim.x) {
         const int e = i / nk, bn = i - e * nk;
-        double x = 0.0;
-#pragma unroll
-        for (int m = 0; m < NM; ++m)
-            if (p.coef[e][m] != 0.0) x += p.coef[e][m] * totals[bn * NM + m];
-        dst[i] = x;
+        dst[i] = totals[bn * NE + e];
     }
 }
 
@@ -758,25 +758,30 @@ static double sqrt_threshold(double e) {
 // sight (mu of the four mirrored modes agrees) and even Legendre products, or monopoles alone (no mu; one
 // FP64 row of 150 x 135 x 144 about another line of sight: 42 us by the mode-tile kernel, 12 us
 // folded); false otherwise.
-static bool fold_plan(const Grid &G, const RedParams &r, FoldParams *p, int *n_moments) {
+static bool fold_plan(const Grid &G, const RedParams &r, FoldParams *p) {
     for (int e = 0; e < r.n_ell; ++e)
         if (G.los && (r.la[e] | r.lb[e])) return false;
     static const double leg[5][3] = {{1.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {-0.5, 1.5, 0.0}, {0.0, 0.0, 0.0},
                                      {0.375, -3.75, 4.375}};
     memset(p, 0, sizeof(*p));
-    int top = 0;
     for (int e = 0; e < r.n_ell; ++e) {
         const int la = r.la[e], lb = r.lb[e];
         if ((la | lb) & 1) return false;
         for (int i = 0; i <= la / 2; ++i)
             for (int j = 0; j <= lb / 2; ++j) p->coef[e][i + j] += leg[la][i] * leg[lb][j];
-        top = std::max(top, (la + lb) / 2);
     }
     for (int i = 0; i <= r.nk; ++i) p->t[i] = sqrt_threshold(r.edges[i]);
     p->nk = r.nk;
     p->n_ell = r.n_ell;
-    *n_moments = top + 1;
     return true;
+}
+
+// whether the kernel of NE products of degree DEG holds the requested ones
+template <int NE, int DEG> static bool fold_holds(const FoldParams &p) {
+    for (int e = 0; e < p.n_ell; ++e)
+        for (int m = 0; m < FOLD_MAX_M; ++m)
+            if (p.coef[e][m] != 0.0 && (e >= NE || m > fold_degree(NE, DEG, e))) return false;
+    return p.n_ell <= NE;
 }
 
 struct LanesLaunch {
@@ -824,14 +829,14 @@ static void launch_binred_finalize(const double *partials, int n_blocks, int per
                                                                                           n_rows, scale, out, accumulate);
 }
 
-template <typename T, int MODE, int NM>
+template <typename T, int MODE, int NE, int DEG>
 static cudaError_t fold_launch(const Grid &G, const void *a, const void *b, int n_rows, int64_t row_stride,
                                const FoldParams &p, int nb, int nw, double *partials, cudaStream_t s) {
-    const size_t smem = (size_t)nw * (p.wb * 32 + p.nk) * NM * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(binred_fold_kernel<T, MODE, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const size_t smem = (size_t)nw * (p.wb * 32 + p.nk) * NE * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(binred_fold_kernel<T, MODE, NE, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    binred_fold_kernel<T, MODE, NM><<<dim3(nb, n_rows), 32 * nw, smem, s>>>(
+    binred_fold_kernel<T, MODE, NE, DEG><<<dim3(nb, n_rows), 32 * nw, smem, s>>>(
         G, (const typename cplx<T>::type *)a, (const typename cplx<T>::type *)b, (const T *)a, row_stride, p, partials);
     return cudaSuccess;
 }
@@ -849,8 +854,11 @@ static int bins_within(const double *edges, int nk, double D) {
 
 // one folded reduction on nb blocks per row; false when its accumulators do not fit
 static bool launch_fold(const Grid &G, int precision, int mode, const void *a, const void *b, int n_rows,
-                        int64_t row_stride, const double *edges, FoldParams p, int nm, int nb, double *partials,
+                        int64_t row_stride, const double *edges, FoldParams p, int nb, double *partials,
                         cudaStream_t s) {
+    if (n_rows > 65535) return false;   // rows lie in gridDim.y
+    // the products of one multipole each (l = 0; 0, 2; 0, 2, 4), of all pairs up to l = 2 and up to l = 4
+    const int variant = fold_holds<1, 0>(p) ? 1 : fold_holds<2, 1>(p) ? 2 : fold_holds<3, 2>(p) ? 3 : fold_holds<4, 2>(p) ? 4 : 9;
     const int m0 = G.n0 - G.n0 / 2, m1 = G.n1 - G.n1 / 2;
     p.n_lchunk = (G.nh2 + 31) / 32;
     // ky steps of a unit: 32, shorter while eight warps' windows do not fit or a warp gets fewer
@@ -859,19 +867,19 @@ static bool launch_fold(const Grid &G, int precision, int mode, const void *a, c
     for (p.jseg = 32;; p.jseg /= 2) {
         const double dy = (p.jseg + 1) * G.kf1, dz = 32 * G.kf2;
         p.wb = std::min(p.nk, 1 + bins_within(edges, p.nk, std::sqrt(dy * dy + dz * dz)));
-        nw = (int)std::min<size_t>(8, FOLD_SMEM / ((size_t)(p.wb * 32 + p.nk) * nm * sizeof(double)));
+        nw = (int)std::min<size_t>(8, FOLD_SMEM / ((size_t)(p.wb * 32 + p.nk) * variant * sizeof(double)));
         const int64_t units = (int64_t)(m0 + 1) * p.n_lchunk * ((m1 + p.jseg) / p.jseg);
         if (p.jseg == 8 || (nw == 8 && units >= (int64_t)8 * nb * nw)) break;
     }
     if (nw < 1) return false;
     p.n_jseg = (m1 + p.jseg) / p.jseg;  // m1 + 1 frequencies |f| = 0 .. m1
     cudaError_t e = cudaSuccess;
-#define PB_FOLD_M(T, MODE, M) \
-    case M: e = fold_launch<T, MODE, M>(G, a, b, n_rows, row_stride, p, nb, nw, partials, s); break;
+#define PB_FOLD_M(T, MODE, NE, DEG) \
+    case NE: e = fold_launch<T, MODE, NE, DEG>(G, a, b, n_rows, row_stride, p, nb, nw, partials, s); break;
 #define PB_FOLD(T, MODE)                                                                                          \
-    switch (nm) {                                                                                                 \
-        PB_FOLD_M(T, MODE, 1) PB_FOLD_M(T, MODE, 2) PB_FOLD_M(T, MODE, 3) PB_FOLD_M(T, MODE, 4)                    \
-        PB_FOLD_M(T, MODE, 5)                                                                                     \
+    switch (variant) {                                                                                            \
+        PB_FOLD_M(T, MODE, 1, 0) PB_FOLD_M(T, MODE, 2, 1) PB_FOLD_M(T, MODE, 3, 2) PB_FOLD_M(T, MODE, 4, 2)        \
+        PB_FOLD_M(T, MODE, 9, 4)                                                                                  \
     }
     if (precision == PB_F32) {
         if (mode == PB_RED_ABS2) PB_FOLD(float, PB_RED_ABS2)
@@ -1029,9 +1037,8 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
     // 37 / 71 / 141 us for 4 / 8 / 15 rows against 87 / 129 / 216 us for the mode-tile kernel (from
     // 16 rows the lane-per-row kernel above takes over)
     FoldParams fp;
-    int nm = 0;
-    if (tuning().red_method != 2 && fold_plan(G, p, &fp, &nm) &&
-        launch_fold(G, precision, mode, a, b, n_rows, row_stride, p.edges, fp, nm, nb, partials, s)) {
+    if (tuning().red_method != 2 && fold_plan(G, p, &fp) &&
+        launch_fold(G, precision, mode, a, b, n_rows, row_stride, p.edges, fp, nb, partials, s)) {
         PB_LAUNCH_CHECK("pb_bin_reduce(fold)");
         launch_binred_finalize(partials, nb, nk * n_ell, n_rows, scale, out, accumulate, s);
         PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");
