@@ -290,13 +290,15 @@ struct RtWalk {
         while (l >= l_end) {
             line += step;
             if (line >= n_lines) return 0;
-            // the run of the line that may hold binned modes, in units of kf2; FP32 with two modes of
-            // margin each side (the bins of the table decide)
+            // the run of the line that may hold binned modes, in units of kf2; FP32 with a margin for its rounding on
+            // the squares (lo^2 - r^2 may be small beside both where kf0 or kf1 is far above kf2) and two modes each
+            // side (the bins of the table decide)
             const int i = (int)((uint32_t)line / (uint32_t)g.n1), j = (int)line - i * g.n1;
             const float kx = freq_index(i, g.n0) * fx, ky = freq_index(j, g.n1) * fy;
             const float r2 = kx * kx + ky * ky, h2 = hi2 * (1.0f + 1e-5f) - r2;
             if (h2 < 0.0f) continue;
-            l = lo2 > r2 ? max(0, (int)sqrtf(lo2 - r2) - 2) : 0;
+            const float l2 = lo2 * (1.0f - 1e-5f) - r2;
+            l = l2 > 0.0f ? max(0, (int)sqrtf(l2) - 2) : 0;
             l_end = (int)fminf((float)g.nh2, sqrtf(h2) + 3.0f);
         }
         first = (int64_t)line * g.nh2 + l;
