@@ -43,7 +43,9 @@ def _settle():
     """Backward runs on autograd's device thread.  On B200 a cuFFT transform issued from that
     thread while the forward's kernels were still running returned CUFFT_EXEC_FAILED (seen at
     512^3, where the forward's contraction runs for tens of ms); waiting for the stream first
-    avoids it.  The wait costs nothing measurable next to a backward pass."""
+    avoids it.  The wait drains the queue in the middle of a call: nothing next to the backward of a large grid, but
+    small calls, whose time is host work for the most part (128^3 Pk gradient: 133 of 249 us are kernels), then queue
+    the backward's launches with the device idle."""
     torch.cuda.current_stream().synchronize()
 
 
@@ -254,7 +256,7 @@ class BkNumerator(torch.autograd.Function):
         grad_spec = torch.zeros((n_acc,) + b.nhalf_shape, dtype=cd, device=b.device)
         if np.any(coef):
             # one real-space map per leg (bin C, multipole lc): the coefficient-weighted sum of
-            # the products of the other two maps of every triplet ending on it (pb_bilinear_maps);
+            # the products of the other two maps of every triplet ending on it (pb_bilinear_block_maps);
             # then one forward transform per leg, filtered into the gradient in its last pass.
             # The terms depend on the binning alone: the table of all triplets is kept and only its
             # coefficients change (a cotangent with zeros gets a table of its own, without their legs)

@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(BL_THREADS, 4) bilinear_kernel(const T *G, int
 // round trip (2850 us).  A zero coefficient stands for a term that is not there: harmless for finite values, so a tile
 // that holds a NaN or an infinity (one FMA per staged value finds it) takes its records one by one, each into the outputs
 // that its code names, and such a value reaches only the outputs that use its map.  Measured on a B200, those terms of 32 maps on 192^3: FP32 1980 us against
-// 3170 us one output at a time, FP64 3960 against 8500 us; ncu: 71 % of the shared-memory and
-// 65 % of the issue rate.  Packed FP32 pairs (fma.rn.f32x2) were slower, 2460 us.
+// 3170 us one output at a time, FP64 3960 against 8500 us; 66 % of
+// the issue slots and 55 % of the shared-memory wavefronts (FP32).  Packed FP32 pairs (fma.rn.f32x2) were slower, 2460 us.
 // ------------------------------------------------------------------------------------
 constexpr int BB_OUT = 4;
 

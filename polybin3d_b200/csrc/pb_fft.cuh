@@ -5,8 +5,9 @@
 // passes: the first reads its operands through a functor (global memory, transformed on the way),
 // the last hands its results to a functor, and only the exchange between passes goes through
 // shared memory.  A butterfly of 8 - 16 points per thread in registers keeps that to one exchange
-// for most lengths up to 256, and that many independent loads in flight per thread.  The radices of an axis are
-// run-time values (one kernel serves every length; the branch on the radix is uniform).
+// for most lengths up to 256, and that many independent loads in flight per thread.  A kernel instantiated for a length
+// N > 0 has that length's radices, strides and counts in its code (AxisUse); its form for N = 0 takes the plan at run
+// time and serves every length (the branch on the radix is uniform).
 //   pass q (Ns = product of the earlier radices, nb = n / R): butterfly j < nb takes elements
 //   j + r nb, twiddled by e^{+-2 pi i r (j mod Ns) / (Ns R)}, to (j / Ns) Ns R + j mod Ns + r Ns.
 #pragma once

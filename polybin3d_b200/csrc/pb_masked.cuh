@@ -15,9 +15,10 @@
 // Three kinds of work are never done: columns (ky, kz) outside a map's own band on the way in,
 // columns outside k_out on the way out, and rows (x, y) where the mask is zero everywhere (Y
 // transforms only planes x that hold such a row, Z only those rows; the rest is exactly zero).
-// W holds kz <= k_out / kF only, rows padded to whole 128-byte lines.  Bound by instruction issue and load latency (20
-// warps per SM for the x and y passes, 16 for z) rather than by memory: chunks of 5 maps whose W stays in
-// L2 took longer than chunks of 32 (more blocks per launch, fewer tails).
+// W holds kz <= k_out / kF only, rows padded to whole 128-byte lines.  X, Y and Z wait for loads (20 warps per SM for the
+// x and y passes, 16 for z; 21 - 37 % of the copy rate); memory takes over in the last two passes, Y' 56 % and X' 62 % of
+// the copy rate for masked rows, 86 and 79 % for products (32 maps of 128^3).  Chunks of 5 maps whose W stays in L2 took
+// longer than chunks of 32 (more blocks per launch, fewer tails).
 // Measured on a B200, 60 rows of 128^3 (bins to 0.93 of the Nyquist frequency), against 2.95 ms for
 // filter, cuFFT and mask: 0.65 ms on a sector mask (17 % of the rows), 1.23 ms on a ball (71 %).
 #pragma once
@@ -456,8 +457,9 @@ cudaError_t mr_launch(MrStage stage, const MrParams &p, const MrShapes &sh, cons
     return cudaGetLastError();
 }
 
-// Lengths with kernels of their own (radices, strides and counts known to the compiler): the lengths with
-// factors 2, 3 and 5 that grids of 48 to 256 are usually given; the others run the run-time plan.
+// Lengths with kernels of their own (radices, strides and counts known to the compiler): twenty even lengths from 48 to
+// 256 with factors 2, 3 and 5, not all of them (each costs three families of kernels seconds of compilation).  Every
+// other length, 50, 54, 162, 250 and the odd ones among them, runs the run-time plan.
 // 60 rows of 128^3 on a ball mask: 1.23 ms against 1.59 ms with the run-time plan, 78 products 1.06
 // against 1.72 ms.  The groups only spread the compilation over files.
 #define MR_GROUP_0(X) X(48) X(60) X(64) X(72) X(80)

@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 3) triplet_simt_kernel(const flo
 // the warps that share pair tiles (KS of them, each on its voxels) add up in shared memory in order and
 // the block writes one partial per triplet.  The row stride of 8 mod 16 elements puts the rows of a read on
 // distinct banks.
-// The FP64 rate bounds it: 16 bins, l = 0, 2, on 192^3 take 2.52 ms, 26 TFLOP/s of matrix products.  The
+// The rate of the FP64 matrix instruction bounds it: the pipe is busy 70 % of the time (12 bins, l = 0, 2, on 120^3);
+// 16 bins, l = 0, 2, on 192^3 take 2.52 ms, 26 TFLOP/s of matrix products.  The
 // form before, 4 x 8 outputs per thread on CUDA cores, held its 32 FP64 sums, half of them empty, in
 // registers that left 8 warps per SM: 12 bins on 120^3 400 us, now 196 us (m8n8k4 and 8-byte reads: 214 us;
 // four pair tiles per warp: 241 us); 9 bins, l = 0, 2, on 90 x 120 x 100 260 us, now 119 us.
