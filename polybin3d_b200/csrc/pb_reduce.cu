@@ -1191,10 +1191,13 @@ __global__ void __launch_bounds__(SR_THREADS) shell_rows_kernel(Grid g, const ty
         }
 }
 
-// parts of the mode list: enough blocks for three per SM, at least eight steps each
+// parts of the mode list: enough blocks for three per SM, down to one step each.  A step is a chain of a load, two
+// barriers and the products, about 1.5 us: with eight steps at least, small shells ran on a few blocks, 12 - 16 us a
+// shell of 16^3 to 32^3 against 4 - 7 us (Bk Fisher of 32^3 295 -> 255 us, 48^3 529 -> 450, 64^3 685 -> 617 us; two
+// steps at least 263, 462 and 619 us; from 96^3 on all the same).
 static int shell_parts(int64_t n_modes, int n_cols, int64_t *per_block) {
     const int64_t steps = std::max<int64_t>(1, (n_modes + SR_M - 1) / SR_M), tiles = (n_cols + SR_CT - 1) / SR_CT;
-    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>((3LL * num_sms() + tiles - 1) / tiles, steps / 8));
+    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>((3LL * num_sms() + tiles - 1) / tiles, steps));
     *per_block = (steps + parts - 1) / parts * SR_M;
     return (int)std::max<int64_t>(1, (n_modes + *per_block - 1) / *per_block);
 }
