@@ -320,6 +320,13 @@ class PolyBin3D:
         p.exec(k, out, self.ws.get(p.ws_bytes, "fft"))
         return out
 
+    @property
+    def one_pass_axes(self):
+        """True on grids of at most 16 points an axis, whose Fisher rows take whole transforms: there one
+        thread of a band-limited chain does a line, 16 or 32 threads a block (Bk Fisher of 16^3: 291 us by
+        chains, 262 by whole transforms; of 20^3 228 and 248 us)."""
+        return int(max(self.gridsize)) <= 16
+
     def rows_table(self):
         """Device twiddle table of the band-limited FP64 chains on the data grid, or None when its
         lengths are not supported."""

@@ -922,11 +922,11 @@ class BSpec:
     def _key_fts(self, G1, G2, keys):
         """FT[g1_0,A g1_l,B - g2_0,A g2_l,B] for keys (A, B, l) as a batch of half spectra: the
         binned modes of each (what the legs and the shells read), or whole spectra where the
-        grid's lengths have no band-limited chain."""
+        grid's lengths have no band-limited chain or take one pass."""
         b = self.base
         nks = self.Nk_squeeze
         pairs = [(A, (l // 2) * nks + B) for (A, B, l) in keys]
-        table = b.rows_table()
+        table = None if b.one_pass_axes else b.rows_table()
         if table is not None:
             b.n_FFTs_forward += len(keys)
             out = torch.empty((len(keys),) + b.nhalf_shape, dtype=torch.complex128, device=b.device)

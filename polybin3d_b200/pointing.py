@@ -51,10 +51,10 @@ class Pointing:
 
     def rows(self):
         """The band-limited chain c2r, mask, r2c of half spectra (nat.MaskedRows), or None: an
-        integral constraint, or a grid whose lengths it does not transform."""
+        integral constraint, or a grid whose lengths it does not transform or that is too small for it."""
         if self._rows is False:
             self._rows = None
-            if self.kind == 'mask':
+            if self.kind == 'mask' and not self.base.one_pass_axes:
                 try:
                     self._rows = nat.MaskedRows(self.base.grid, self.mask)
                 except NotImplementedError:
