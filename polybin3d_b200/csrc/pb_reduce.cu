@@ -584,15 +584,16 @@ __global__ void __launch_bounds__(256) binred_lanes_kernel(Grid g, const typenam
 // for the mode-tile kernel (256^3 FP32: 42 against 310 us; 128^3 FP64: below 20 against 50 us).
 // ------------------------------------------------------------------------------------
 constexpr int FOLD_MAX_M = 5;           // mu^0 .. mu^8
-// Kernels are compiled for NE products of degree DEG in mu^2; one that starts at l = 0, 2, 4, product e of degree e at
-// most, skips the zero coefficients above it
-__host__ __device__ constexpr int fold_degree(int ne, int deg, int e) { return ne == deg + 1 && e < deg ? e : deg; }
+// Kernels are compiled for slots of one degree in mu^2 each: l = 0; 0, 2; 0, 2, 4; and the six different products of two
+// of 0, 2, 4 (those of 0, 2 fit the three slots).  Equal products share a slot.
+__host__ __device__ constexpr int fold_degree(int ne, int e) { return ne <= 3 || e < 3 ? e : e - 1; }
 constexpr int FOLD_SMEM = 100 * 1024;   // accumulators per block, two blocks per SM
 
 struct FoldParams {
     double t[PB_RED_MAX_BINS + 1];                  // thresholds on |k|^2
-    double coef[PB_RED_MAX_ELLS][FOLD_MAX_M];       // L_la L_lb as a polynomial in mu^2
+    double coef[PB_RED_MAX_ELLS][FOLD_MAX_M];       // the slots' products as polynomials in mu^2
     int32_t nk, n_ell;
+    int8_t slot[PB_RED_MAX_ELLS];                   // of each requested product
     int32_t jseg, n_jseg, n_lchunk;                 // ky steps per unit, units per (kx, kz chunk)
     int32_t wb;                                     // bins of a unit's window
 };
@@ -612,7 +613,7 @@ __device__ __forceinline__ double fold_value(const typename cplx<T>::type *a, co
     return v * v;
 }
 
-template <typename T, int MODE, int NE, int DEG>
+template <typename T, int MODE, int NE>
 __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typename cplx<T>::type *a,
                                                             const typename cplx<T>::type *b, const T *w,
                                                             int64_t row_stride, const __grid_constant__ FoldParams p,
@@ -703,14 +704,13 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
                         next = t[nk + 1];
                     }
                 }
-                const double x = f[q] * deg, mu2 = DEG > 0 && s[q] > 0.0 ? kz2 / s[q] : 0.0;
+                const double x = f[q] * deg, mu2 = NE > 1 && s[q] > 0.0 ? kz2 / s[q] : 0.0;
 #pragma unroll
                 for (int e = 0; e < NE; ++e) {
-                    constexpr int top = DEG;
-                    const int d = fold_degree(NE, DEG, e);
+                    const int d = fold_degree(NE, e);
                     double w = p.coef[e][d];
 #pragma unroll
-                    for (int m = top - 1; m >= 0; --m)
+                    for (int m = FOLD_MAX_M - 2; m >= 0; --m)
                         if (m < d) w = w * mu2 + p.coef[e][m];
                     acc[e] += x * w;
                 }
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256, 2) binred_fold_kernel(Grid g, const typen
     double *dst = partials + ((int64_t)row * gridDim.x + blockIdx.x) * (p.n_ell * nk);
     for (int i = threadIdx.x; i < p.n_ell * nk; i += blockDim.x) {
         const int e = i / nk, bn = i - e * nk;
-        dst[i] = totals[bn * NE + e];
+        dst[i] = totals[bn * NE + p.slot[e]];
     }
 }
 
@@ -760,30 +760,39 @@ static double sqrt_threshold(double e) {
 // sight (mu of the four mirrored modes agrees) and even Legendre products, or monopoles alone (no mu; one
 // FP64 row of 150 x 135 x 144 about another line of sight: 42 us by the mode-tile kernel, 12 us
 // folded); false otherwise.
-static bool fold_plan(const Grid &G, const RedParams &r, FoldParams *p) {
+static bool fold_plan(const Grid &G, const RedParams &r, FoldParams *p, int *slots) {
     for (int e = 0; e < r.n_ell; ++e)
         if (G.los && (r.la[e] | r.lb[e])) return false;
     static const double leg[5][3] = {{1.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {-0.5, 1.5, 0.0}, {0.0, 0.0, 0.0},
                                      {0.375, -3.75, 4.375}};
     memset(p, 0, sizeof(*p));
-    for (int e = 0; e < r.n_ell; ++e) {
-        const int la = r.la[e], lb = r.lb[e];
-        if ((la | lb) & 1) return false;
-        for (int i = 0; i <= la / 2; ++i)
-            for (int j = 0; j <= lb / 2; ++j) p->coef[e][i + j] += leg[la][i] * leg[lb][j];
+    // the different products, each in the first free slot that holds its degree, in the smallest kernel with such slots
+    for (int n : {1, 2, 3, 6}) {
+        int used = 0, e = 0;
+        memset(p->coef, 0, sizeof(p->coef));
+        for (; e < r.n_ell; ++e) {
+            const int la = std::min(r.la[e], r.lb[e]), lb = std::max(r.la[e], r.lb[e]), top = (la + lb) / 2;
+            if ((la | lb) & 1) return false;
+            int s = 0;
+            while (s < e && !(std::min(r.la[s], r.lb[s]) == la && std::max(r.la[s], r.lb[s]) == lb)) ++s;
+            if (s < e) {
+                p->slot[e] = p->slot[s];
+                continue;
+            }
+            for (s = 0; s < n && ((used >> s & 1) || fold_degree(n, s) < top);) ++s;
+            if (s == n) break;
+            used |= 1 << s;
+            p->slot[e] = (int8_t)s;
+            for (int i = 0; i <= la / 2; ++i)
+                for (int j = 0; j <= lb / 2; ++j) p->coef[s][i + j] += leg[la][i] * leg[lb][j];
+        }
+        *slots = n;
+        if (e == r.n_ell) break;
     }
     for (int i = 0; i <= r.nk; ++i) p->t[i] = sqrt_threshold(r.edges[i]);
     p->nk = r.nk;
     p->n_ell = r.n_ell;
     return true;
-}
-
-// whether the kernel of NE products of degree DEG holds the requested ones
-template <int NE, int DEG> static bool fold_holds(const FoldParams &p) {
-    for (int e = 0; e < p.n_ell; ++e)
-        for (int m = 0; m < FOLD_MAX_M; ++m)
-            if (p.coef[e][m] != 0.0 && (e >= NE || m > fold_degree(NE, DEG, e))) return false;
-    return p.n_ell <= NE;
 }
 
 struct LanesLaunch {
@@ -831,14 +840,14 @@ static void launch_binred_finalize(const double *partials, int n_blocks, int per
                                                                                           n_rows, scale, out, accumulate);
 }
 
-template <typename T, int MODE, int NE, int DEG>
+template <typename T, int MODE, int NE>
 static cudaError_t fold_launch(const Grid &G, const void *a, const void *b, int n_rows, int64_t row_stride,
                                const FoldParams &p, int nb, int nw, double *partials, cudaStream_t s) {
     const size_t smem = (size_t)nw * (p.wb * 32 + p.nk) * NE * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(binred_fold_kernel<T, MODE, NE, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(binred_fold_kernel<T, MODE, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    binred_fold_kernel<T, MODE, NE, DEG><<<dim3(nb, n_rows), 32 * nw, smem, s>>>(
+    binred_fold_kernel<T, MODE, NE><<<dim3(nb, n_rows), 32 * nw, smem, s>>>(
         G, (const typename cplx<T>::type *)a, (const typename cplx<T>::type *)b, (const T *)a, row_stride, p, partials);
     return cudaSuccess;
 }
@@ -856,11 +865,9 @@ static int bins_within(const double *edges, int nk, double D) {
 
 // one folded reduction on nb blocks per row; false when its accumulators do not fit
 static bool launch_fold(const Grid &G, int precision, int mode, const void *a, const void *b, int n_rows,
-                        int64_t row_stride, const double *edges, FoldParams p, int nb, double *partials,
-                        cudaStream_t s) {
+                        int64_t row_stride, const double *edges, FoldParams p, int slots, int nb,
+                        double *partials, cudaStream_t s) {
     if (n_rows > 65535) return false;   // rows lie in gridDim.y
-    // the products of one multipole each (l = 0; 0, 2; 0, 2, 4), of all pairs up to l = 2 and up to l = 4
-    const int variant = fold_holds<1, 0>(p) ? 1 : fold_holds<2, 1>(p) ? 2 : fold_holds<3, 2>(p) ? 3 : fold_holds<4, 2>(p) ? 4 : 9;
     const int m0 = G.n0 - G.n0 / 2, m1 = G.n1 - G.n1 / 2;
     p.n_lchunk = (G.nh2 + 31) / 32;
     // ky steps of a unit: 32, shorter while eight warps' windows do not fit or a warp gets fewer
@@ -869,19 +876,21 @@ static bool launch_fold(const Grid &G, int precision, int mode, const void *a, c
     for (p.jseg = 32;; p.jseg /= 2) {
         const double dy = (p.jseg + 1) * G.kf1, dz = 32 * G.kf2;
         p.wb = std::min(p.nk, 1 + bins_within(edges, p.nk, std::sqrt(dy * dy + dz * dz)));
-        nw = (int)std::min<size_t>(8, FOLD_SMEM / ((size_t)(p.wb * 32 + p.nk) * variant * sizeof(double)));
+        nw = (int)std::min<size_t>(8, FOLD_SMEM / ((size_t)(p.wb * 32 + p.nk) * slots * sizeof(double)));
         const int64_t units = (int64_t)(m0 + 1) * p.n_lchunk * ((m1 + p.jseg) / p.jseg);
         if (p.jseg == 8 || (nw == 8 && units >= (int64_t)8 * nb * nw)) break;
     }
-    if (nw < 1) return false;
+    // where a block holds one window only, its one warp is slower than the mode-tile kernel: all products up to l = 4 in 60
+    // bins, FP64 weights of 64^3 (95 KB a window) 43 against 29 us, of 128^3 (58 KB) 94 against 64 us; with two warps, of
+    // 200^3 (41 KB), 71 against 199 us
+    if (nw < 2) return false;
     p.n_jseg = (m1 + p.jseg) / p.jseg;  // m1 + 1 frequencies |f| = 0 .. m1
     cudaError_t e = cudaSuccess;
-#define PB_FOLD_M(T, MODE, NE, DEG) \
-    case NE: e = fold_launch<T, MODE, NE, DEG>(G, a, b, n_rows, row_stride, p, nb, nw, partials, s); break;
+#define PB_FOLD_M(T, MODE, NE) \
+    case NE: e = fold_launch<T, MODE, NE>(G, a, b, n_rows, row_stride, p, nb, nw, partials, s); break;
 #define PB_FOLD(T, MODE)                                                                                          \
-    switch (variant) {                                                                                            \
-        PB_FOLD_M(T, MODE, 1, 0) PB_FOLD_M(T, MODE, 2, 1) PB_FOLD_M(T, MODE, 3, 2) PB_FOLD_M(T, MODE, 4, 2)        \
-        PB_FOLD_M(T, MODE, 9, 4)                                                                                  \
+    switch (slots) {                                                                                              \
+        PB_FOLD_M(T, MODE, 1) PB_FOLD_M(T, MODE, 2) PB_FOLD_M(T, MODE, 3) PB_FOLD_M(T, MODE, 6)                    \
     }
     if (precision == PB_F32) {
         if (mode == PB_RED_ABS2) PB_FOLD(float, PB_RED_ABS2)
@@ -1039,8 +1048,9 @@ extern "C" int pb_bin_reduce(const pb_grid_t *g, int precision, int mode, const 
     // 37 / 71 / 141 us for 4 / 8 / 15 rows against 87 / 129 / 216 us for the mode-tile kernel (from
     // 16 rows the lane-per-row kernel above takes over)
     FoldParams fp;
-    if (tuning().red_method != 2 && fold_plan(G, p, &fp) &&
-        launch_fold(G, precision, mode, a, b, n_rows, row_stride, p.edges, fp, nb, partials, s)) {
+    int slots = 0;
+    if (tuning().red_method != 2 && fold_plan(G, p, &fp, &slots) &&
+        launch_fold(G, precision, mode, a, b, n_rows, row_stride, p.edges, fp, slots, nb, partials, s)) {
         PB_LAUNCH_CHECK("pb_bin_reduce(fold)");
         launch_binred_finalize(partials, nb, nk * n_ell, n_rows, scale, out, accumulate, s);
         PB_LAUNCH_CHECK("pb_bin_reduce(finalize)");

@@ -50,3 +50,26 @@ def test_infinite_modes(ells, mode, dtype):
                 assert abs(out[e, i] - want) <= tol, (e, i)
             else:
                 assert np.array_equal([out[e, i]], [want], equal_nan=True), (e, i, out[e, i], want)
+
+
+@pytest.mark.parametrize("ells", [[(4, 4), (2, 0), (0, 2), (4, 0)], [(2, 2), (4, 0), (0, 0)], [(4, 2), (2, 4)], [(4, 0)]])
+def test_products_in_any_order(ells):
+    """Orders and repeats of the products that share slots, on finite values."""
+    n, edges = (10, 9, 12), [0.5, 2.5, 4.0]
+    rng = np.random.default_rng(8)
+    x = torch.from_numpy(rng.standard_normal((n[0], n[1], n[2] // 2 + 1, 2))).cuda()
+    g = nat.PBGrid()
+    for i in range(3):
+        g.n[i], g.kf[i] = n[i], 1.0
+    out = torch.empty(len(ells), 2, dtype=torch.float64, device="cuda")
+    nat.bin_reduce(g, nat.PB_F64, nat.PB_RED_ABS2, x, None, 1, edges, ells, 1.0, out, nat.Workspace(torch.device("cuda")))
+    ka = [np.fft.fftshift(np.arange(-n[i] // 2, n[i] // 2)) for i in range(2)]
+    kx, ky, kz = np.meshgrid(ka[0], ka[1], np.arange(n[2] // 2 + 1), indexing="ij")
+    k = np.sqrt(kx ** 2.0 + ky ** 2 + kz ** 2)
+    mu = np.divide(kz, k, out=np.zeros_like(k), where=k > 0)
+    f = (1.0 + (kz > 0)) * (x.cpu().numpy() ** 2).sum(-1)
+    for e, (la, lb) in enumerate(ells):
+        for i in range(2):
+            sel = (edges[i] <= k) & (k < edges[i + 1])
+            t = f[sel] * LEG[la](mu[sel]) * LEG[lb](mu[sel])
+            assert abs(float(out[e, i]) - t.sum()) <= 64 * t.size * np.finfo(np.float64).eps * np.sum(f[sel])
