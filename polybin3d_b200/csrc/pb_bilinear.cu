@@ -304,7 +304,9 @@ static int launch_blocks(const void *G, int n_g, int64_t n_vox, const int32_t *o
     const int vec = (n_vox * (int64_t)sizeof(T)) % 16 == 0 && (((uintptr_t)G | (uintptr_t)out) & 15) == 0;
     // BB_OCC blocks per SM (227 KB, 1 KB of it taken per block); one span of 128 maps is 128 KB, one block
     int n_span = std::min(8, ((227 * 1024 / BB_OCC - 2048) - fixed) / row);
-    n_span = std::max(1, n_span);
+    // and no more than leave every SM its blocks (13,824 voxels, 16 bins, l = 0, 2: 42 us with tiles as large as fit, now
+    // 20 us; 4 bins 10 and 4.5 us)
+    n_span = std::max(1, (int)std::min<int64_t>(n_span, (n_vox + span - 1) / span / ((int64_t)num_sms() * BB_OCC)));
     const int tile = span * n_span;
     const size_t smem = (size_t)row * n_span;
     const int blocks = (int)std::min<int64_t>((n_vox + tile - 1) / tile, (int64_t)num_sms() * BB_OCC * 16);
