@@ -49,6 +49,9 @@ template <typename T> __host__ __device__ constexpr size_t sl_line_bytes(const f
 template <typename T> __host__ __device__ constexpr int sl_lines(const fft::Axis &ax) {
     int L = SlShape<T>::LINES;
     while (L > 2 && sl_line_bytes<T>(ax, L) > (size_t)SL_SMEM) L /= 2;
+    // three passes (two exchange buffers): four blocks per SM, down to runs of 64 bytes (16 FP32 maps of 320^3 2.54 ms with
+    // the larger blocks, 2.33 so; runs of 32 bytes at 480 points 8.0 against 7.4 ms)
+    while (ax.np == 3 && L * 2 * sizeof(T) > 64 && sl_line_bytes<T>(ax, L) > (size_t)54 * 1024) L /= 2;
     return L;
 }
 // threads per line: equal rounds of butterflies in the first pass
@@ -57,10 +60,12 @@ template <typename T> __host__ __device__ constexpr int sl_threads(const fft::Ax
     return (ax.nb[0] + rounds - 1) / rounds;
 }
 // threads per line of the z pass: eight for two passes (16 for 192 took 386 against 348 us for 32 FP32 maps: a
-// quarter of them idle in the first pass), the count up to 32 with the fewest idle butterfly slots for three
+// quarter of them idle in the first pass), the count from 16 to 32 with the fewest idle butterfly slots for three (eight,
+// with no idle slot, left 384 points four blocks of 64 threads per SM: 16 FP64 maps of 384^3 10.2 ms, with 32 threads a
+// line 6.3 ms)
 __host__ __device__ constexpr int sl_z_threads(const fft::Axis &ax) {
     int best = 1, cost = 1 << 30;
-    for (int t = ax.np == 1 ? 1 : 8; t <= (ax.np == 3 ? 32 : 8); ++t) {
+    for (int t = ax.np == 1 ? 1 : ax.np == 2 ? 8 : 16; t <= (ax.np == 3 ? 32 : 8); ++t) {
         int c = 0;
         for (int q = 0; q < ax.np; ++q) c += (ax.nb[q] + t - 1) / t * t * ax.R[q];
         if (c <= cost) {
