@@ -94,7 +94,7 @@ static int mr_setup(const Grid &G, double k_out, MrParams *pp, MrShapes *sh) {
     p.n_pairs = G.n0 * ((G.n1 + 1) / 2);
     for (MrStage stage : {MR_X, MR_Y, MR_Z, MR_PRODUCT, MR_Y_BACK, MR_X_BACK}) {
         const MrGrid n = mr_grid(stage, p, *sh, MR_MAX_MAPS);
-        if (n.x > 2147483647 || n.y > 65535) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: too many rows");
+        if (n.x > 2147483647 || n.y > 65535 || n.z > 65535) return fail(PB_ERR_UNSUPPORTED, "pb_masked_rows: too many rows");
     }
     return PB_OK;
 }
@@ -247,7 +247,7 @@ extern "C" int pb_product_rows(const pb_grid_t *g, const double *X, const double
     a.table = (const double2 *)table;
     a.W = (double2 *)workspace;
     for (int m0 = 0; m0 < n_pairs; m0 += chunk) {
-        p.n_prod = a.maps = std::min(chunk, n_pairs - m0);
+        a.maps = std::min(chunk, n_pairs - m0);
         for (int m = 0; m < a.maps; ++m) {
             a.products.i[m] = (int16_t)pairs[2 * (m0 + m)];
             a.products.j[m] = (int16_t)pairs[2 * (m0 + m) + 1];

@@ -48,7 +48,7 @@ struct MrParams {
     int n_legs, ldz, kz_out;
     double out2;                   // square of k_out (with a margin)
     int64_t src_stride, w_map;     // elements per map of src and W
-    int n_x, n_pairs, n_prod;      // planes, row pairs and products of a launch
+    int n_x, n_pairs;
     Axis ax, ay, azi, azf;
     int tw_x, tw_y, tw_zi, tw_zf;  // table offsets (complex elements)
     MrMap maps[MR_MAX_MAPS];
@@ -311,9 +311,10 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_z_kernel(const __grid_consta
 }
 
 // ---- products: forward transform along z of X_i Y_j - Z_i Z_j, two rows per complex line ----------
-// block (threads per line, L pairs of rows); grid (row pairs / L x products, products fastest): the products of a
-// few rows follow each other, so the maps' rows come from L2 after the first (all in x: the row blocks of 512 x 512
-// x 500 and of 640^3 are more than y takes)
+// block (threads per line, L pairs of rows); grid (products, row pairs / L): the products of a few rows follow each
+// other, so the maps' rows come from L2 after the first.  The row blocks lie in y and z: those of 512 x 512 x 500 and of
+// 640^3 are more than y takes (in x with the products, taken apart by a division, 5 products of 150 x 135 x 144 took 104
+// against 101 us)
 struct MrPairs {
     int16_t i[MR_MAX_MAPS], j[MR_MAX_MAPS];
 };
@@ -329,16 +330,15 @@ __global__ void __launch_bounds__(MR_THREADS, 2) mr_product_kernel(const __grid_
     const int L = blockDim.y, n = ax.n, ld = fft::row_len(ax);
     double2 *tw = mr_smem, *sm = tw + ax.tw_len + threadIdx.y * ld, *sm2 = sm + L * ld;
     load_table(tw, table + p.tw_zf, ax.tw_len);
-    const int rb = blockIdx.x / p.n_prod, pm = blockIdx.x - rb * p.n_prod;
-    const int half = (g.n1 + 1) / 2, q = rb * L + threadIdx.y;
+    const int half = (g.n1 + 1) / 2, q = (blockIdx.z * gridDim.y + blockIdx.y) * L + threadIdx.y;
     const bool on = q < g.n0 * half;
     const int x = on ? q / half : 0, y = on ? 2 * (q - x * half) : 0;
     const bool two = y + 1 < g.n1;
     const double h = two ? 0.5 : 1.0;
-    const int64_t ra = (int64_t)x * g.n1 + y, oi = pr.i[pm] * g.nreal, oj = pr.j[pm] * g.nreal;
+    const int64_t ra = (int64_t)x * g.n1 + y, oi = pr.i[blockIdx.x] * g.nreal, oj = pr.j[blockIdx.x] * g.nreal;
     const double *xi = X + oi + ra * n, *xj = Y + oj + ra * n;
     const double *zi = Z ? Z + oi + ra * n : nullptr, *zj = Z ? Z + oj + ra * n : nullptr;
-    double2 *wa = W + pm * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
+    double2 *wa = W + blockIdx.x * p.w_map + ra * p.ldz, *wb = wa + p.ldz;
     fft::line_fft<double, -1>(
         use, threadIdx.x, N ? ax.nb[0] : (int)blockDim.x, on, sm, sm2, tw, [&](int e) { return fft::row_at(ax, e); },
         [&](int e, int) {
@@ -405,16 +405,19 @@ enum MrStage { MR_X, MR_Y, MR_Z, MR_PRODUCT, MR_Y_BACK, MR_X_BACK };
 
 // blocks of a stage for nm maps
 struct MrGrid {
-    int64_t x, y;
+    int64_t x, y, z;
 };
 static inline MrGrid mr_grid(MrStage stage, const MrParams &p, const MrShapes &sh, int nm) {
     switch (stage) {
         case MR_X:
-        case MR_X_BACK: return {(int64_t)p.g.n1 * (p.kz_out / sh.Lx + 1), nm};
+        case MR_X_BACK: return {(int64_t)p.g.n1 * (p.kz_out / sh.Lx + 1), nm, 1};
         case MR_Y:
-        case MR_Y_BACK: return {(int64_t)p.n_x * (p.kz_out / sh.Ly + 1), nm};
-        case MR_Z: return {((int64_t)p.n_pairs + sh.Lz - 1) / sh.Lz, nm};
-        default: return {((int64_t)p.g.n0 * ((p.g.n1 + 1) / 2) + sh.Lz - 1) / sh.Lz * nm, 1};
+        case MR_Y_BACK: return {(int64_t)p.n_x * (p.kz_out / sh.Ly + 1), nm, 1};
+        case MR_Z: return {((int64_t)p.n_pairs + sh.Lz - 1) / sh.Lz, nm, 1};
+        default: {
+            const int64_t rows = ((int64_t)p.g.n0 * ((p.g.n1 + 1) / 2) + sh.Lz - 1) / sh.Lz, z = (rows + 65534) / 65535;
+            return {nm, (rows + z - 1) / z, z};
+        }
     }
 }
 
@@ -426,7 +429,7 @@ template <typename K> static cudaError_t mr_allow(K kernel, size_t bytes) {
 template <int N>
 cudaError_t mr_launch(MrStage stage, const MrParams &p, const MrShapes &sh, const MrArgs &a, cudaStream_t s) {
     const MrGrid n = mr_grid(stage, p, sh, a.maps);
-    const dim3 grid((unsigned)n.x, (unsigned)n.y);
+    const dim3 grid((unsigned)n.x, (unsigned)n.y, (unsigned)n.z);
     cudaError_t e = cudaSuccess;
     switch (stage) {
         case MR_X:
